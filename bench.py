@@ -740,7 +740,8 @@ def run_ours(args, rank, world, local):
                               if info.vort2flux_order == L.IB_V2F_LEVELS else "level by level (the reference's order)"),
                 "parallelism": "replicas",
                 "transforms": {0: "Stockham FFT passes", 1: "warp-per-line FFT passes",
-                               2: "BF16x3 tensor-core sine GEMMs"}.get(int(info.transform_form)),
+                               2: "BF16x3 tensor-core sine GEMMs",
+                               3: "64-bit block fixed-point FFT passes"}.get(int(info.transform_form)),
                 "autotune": arm["solver"].autotune(),
                 "device_bytes": int(info.device_bytes),
                 "setup_s": info.setup_ms / 1e3, "host_wall_ms_per_step": arm["host_s"] / K * 1e3},
@@ -778,7 +779,7 @@ def run_ours(args, rank, world, local):
     fp64, fp32 = C.c_double(), C.c_double()
     lib.ib_measure_fp_peaks(local, C.byref(fp64), C.byref(fp32))
     achieved = bytes_per_launch / per_launch_s / 1e9
-    form = {0: "stockham", 1: "warp", 2: "tensor"}.get(int(info.transform_form), "stockham")
+    form = {0: "stockham", 1: "warp", 2: "tensor", 3: "fixed"}.get(int(info.transform_form), "stockham")
     v2f = "levels" if info.vort2flux_order == L.IB_V2F_LEVELS else "sequential"
     meas = measured_traffic(args.workload, prec, f"{form}/{v2f}", dom)
     traffic = meas[0] if meas else None
@@ -789,6 +790,8 @@ def run_ours(args, rank, world, local):
                             "y": "k_wy (y-direction sine passes + spectral op, one warp per column)"},
                    "stockham": {"x": "k_xpass (x-direction sine pass)",
                                 "y": "k_ypass (y-direction sine pass + spectral op)"},
+                   "fixed": {"x": "k_fx_fwd/k_fx_inv (x-direction block fixed-point sine passes)",
+                             "y": "k_fx_y (y-direction block fixed-point sine passes + spectral op)"},
                    "tensor": {"x": "k_gpro + k_sgemm (x-direction BF16x3 sine GEMMs)",
                               "y": "k_sgemm (y-direction BF16x3 sine GEMMs)"}}[form][dom],
         "bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,

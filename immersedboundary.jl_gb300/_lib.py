@@ -28,7 +28,7 @@ IB_PREC_FP64 = 0
 IB_PREC_MIXED = 1
 IB_PREC_MIXED_TC = 2
 PRECISIONS = {"fp64": IB_PREC_FP64, "mixed": IB_PREC_MIXED, "mixed_tc": IB_PREC_MIXED_TC}
-IB_FORM_STOCKHAM, IB_FORM_WARP, IB_FORM_TENSOR = 0, 1, 2
+IB_FORM_STOCKHAM, IB_FORM_WARP, IB_FORM_TENSOR, IB_FORM_FIXED = 0, 1, 2, 3
 IB_SCHEME_CNAB, IB_SCHEME_RKC = 0, 1
 IB_MOTION_STATIC = 0
 IB_MOTION_PRESCRIBED = 1

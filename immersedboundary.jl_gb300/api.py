@@ -411,7 +411,8 @@ def initstate(prob: Problem, t: float = 0.0) -> State:
 class Solver:
     """``CNAB.Solver`` (cnab/timestepping.jl:173-249) backed by a libibgb300 handle.
 
-    ``precision``: ``"fp64"`` (every sine transform in FP64, the reference's arithmetic),
+    ``precision``: ``"fp64"`` (the reference's arithmetic; the sine transforms in 64-bit block
+    fixed point, whose rounding error is below FP64's),
     ``"mixed"`` (FP32 sine transforms refined with float-float residuals, ``refine_sweeps`` sweeps per
     Poisson solve: 1 or 2 everywhere, or 0 = the library default of 2 with 1 for the Vort2Flux
     solves of the third and coarser levels; state, stencils and the nonlinear term in float-float

@@ -1,4 +1,5 @@
-// Batched 2-D DST-I passes: the Poisson / Crank-Nicolson solves of the IBPM step.
+// Batched 2-D DST-I passes of the mixed-precision solves (FP32 lines) for axes without warp-per-line
+// passes, and the tables of the FP32 transforms.  The FP64 solves use dstfx.cu.
 //
 // Replaces the FFTW RODFT00 plan + `LaplacianInv` call of the reference
 // (src/streamfcn/fluid-ops.jl:19-56) and the CN multipliers of `A_Ainv_linearmaps`
@@ -250,9 +251,6 @@ k_xpass(Geometry g, DstAxis<T> ax, XArgs a) {
       Tout* dst = out + off;
       if (EPI == kEpiStore) {
         for (int I = t; I < ncol; I += kGroup) dst[I] = (Tout)s[I + 1];
-      } else if (EPI == kEpiSub) {
-        const A* sf = static_cast<const A*>(a.sub_from) + off;
-        for (int I = t; I < ncol; I += kGroup) dst[I] = (Tout)(sf[I] - A(s[I + 1]));
       } else {
         const float* bs = a.base + off;
         const float* bs2 = a.base2 ? a.base2 + off : nullptr;
@@ -275,7 +273,7 @@ k_xpass(Geometry g, DstAxis<T> ax, XArgs a) {
 // (index I*(ny-1) + J) so a column reads them contiguously.
 // Shared memory per column: the line and the FFT scratch.
 // ------------------------------------------------------------------------------------------
-template <typename T, SpecOp OP>
+template <typename T>
 __global__ void __launch_bounds__(512)
 k_ypass(Geometry g, DstAxis<T> ax, YPassArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -299,13 +297,9 @@ k_ypass(Geometry g, DstAxis<T> ax, YPassArgs<T> a) {
     const int I = I0 + grp;
     dst1_line<T>(p, sc, D, ax, t);
     const int64_t mo = (int64_t)b * a.mstride + (int64_t)min(I, ncol - 1) * nrow;
-    if (OP == SpecOp::kScale) {
-      for (int J = t; J < nrow; J += kGroup) p[J + 1] *= __ldg(&a.m1[mo + J]);
-    } else {
-      for (int J = t; J < nrow; J += kGroup) p[J + 1] *= a.scal;
-    }
+    for (int J = t; J < nrow; J += kGroup) p[J + 1] *= __ldg(&a.m1[mo + J]);
     __syncthreads();
-    if (OP != SpecOp::kFwd) dst1_line<T>(p, sc, D, ax, t);
+    dst1_line<T>(p, sc, D, ax, t);
     for (int idx = threadIdx.x; idx < nrow * W; idx += blockDim.x) {
       const int J = idx / W, w = idx - J * W, Ic = I0 + w;
       if (Ic < ncol) a.out[off + (int64_t)J * ncol + Ic] = P[w * lv + J + 1];
@@ -330,25 +324,6 @@ cudaError_t ensure_smem(const void* fn, size_t bytes) {
   return e;
 }
 
-// Radix plan of an M-point FFT: powers of two first (8s, then a 4/4, 4 or 2 remainder), then 3s,
-// then 5s, so the leading stages have power-of-two strides (k = j & (Ns-1)).
-int plan_radices(int M, int* radix) {
-  int m = M, ns = 0, p2 = 0, n3 = 0, n5 = 0;
-  while (m % 5 == 0) { ++n5; m /= 5; }
-  while (m % 3 == 0) { ++n3; m /= 3; }
-  while (m % 2 == 0) { ++p2; m /= 2; }
-  if (m != 1) return -1;
-  int a = p2 / 3, rem = p2 % 3;
-  if (rem == 1 && a >= 1) { a -= 1; radix[ns++] = 4; radix[ns++] = 4; }
-  else if (rem == 1) { radix[ns++] = 2; }
-  else if (rem == 2) { radix[ns++] = 4; }
-  for (int i = 0; i < a; ++i) radix[ns++] = 8;
-  for (int i = 0; i < n3; ++i) radix[ns++] = 3;
-  for (int i = 0; i < n5; ++i) radix[ns++] = 5;
-  if (ns > kMaxStages) return -1;
-  return ns;
-}
-
 template <typename T, typename Tin, typename Tout, int PRO, int EPI, bool kBC>
 cudaError_t launch_x1(const Geometry& g, const DstAxis<T>& ax, const XArgs& a, cudaStream_t s) {
   const int total = a.batch * (g.ny - 1);
@@ -368,9 +343,6 @@ cudaError_t launch_x_epi(const Geometry& g, const DstAxis<T>& ax, const XArgs& a
     case kEpiStore:
       return bc ? launch_x1<T, Tin, Tout, PRO, kEpiStore, true>(g, ax, a, s)
                 : launch_x1<T, Tin, Tout, PRO, kEpiStore, false>(g, ax, a, s);
-    case kEpiSub:
-      if (bc) return cudaErrorInvalidValue;
-      return launch_x1<T, Tin, Tout, PRO, kEpiSub, false>(g, ax, a, s);
     case kEpiAddBase:
       if (bc) return cudaErrorInvalidValue;
       return launch_x1<T, Tin, Tout, PRO, kEpiAddBase, false>(g, ax, a, s);
@@ -393,19 +365,32 @@ cudaError_t launch_y(const Geometry& g, const DstAxis<T>& ax, const YPassArgs<T>
   const int nstrips = (g.nx - 1 + W - 1) / W;
   const int blocks = a.batch * nstrips;
   cudaError_t e;
-  if (a.op == SpecOp::kFwd) {
-    auto k = k_ypass<T, SpecOp::kFwd>;
-    if ((e = ensure_smem((const void*)k, smem)) != cudaSuccess) return e;
-    k<<<blocks, W * kGroup, smem, s>>>(g, ax, a);
-  } else {
-    auto k = k_ypass<T, SpecOp::kScale>;
-    if ((e = ensure_smem((const void*)k, smem)) != cudaSuccess) return e;
-    k<<<blocks, W * kGroup, smem, s>>>(g, ax, a);
-  }
+  auto k = k_ypass<T>;
+  if ((e = ensure_smem((const void*)k, smem)) != cudaSuccess) return e;
+  k<<<blocks, W * kGroup, smem, s>>>(g, ax, a);
   return cudaGetLastError();
 }
 
 }  // namespace
+
+// Radix plan of an M-point FFT: powers of two first (8s, then a 4/4, 4 or 2 remainder), then 3s,
+// then 5s, so the leading stages have power-of-two strides (k = j & (Ns-1)).
+int plan_radices(int M, int* radix) {
+  int m = M, ns = 0, p2 = 0, n3 = 0, n5 = 0;
+  while (m % 5 == 0) { ++n5; m /= 5; }
+  while (m % 3 == 0) { ++n3; m /= 3; }
+  while (m % 2 == 0) { ++p2; m /= 2; }
+  if (m != 1) return -1;
+  int a = p2 / 3, rem = p2 % 3;
+  if (rem == 1 && a >= 1) { a -= 1; radix[ns++] = 4; radix[ns++] = 4; }
+  else if (rem == 1) { radix[ns++] = 2; }
+  else if (rem == 2) { radix[ns++] = 4; }
+  for (int i = 0; i < a; ++i) radix[ns++] = 8;
+  for (int i = 0; i < n3; ++i) radix[ns++] = 3;
+  for (int i = 0; i < n5; ++i) radix[ns++] = 5;
+  if (ns > kMaxStages) return -1;
+  return ns;
+}
 
 cudaError_t set_smem_limit(const void* fn, size_t bytes) { return ensure_smem(fn, bytes); }
 
@@ -543,15 +528,11 @@ cudaError_t ypass(const Geometry& g, const DstAxis<T>& ax, const YPassArgs<T>& a
   return launch_y<T>(g, ax, a, s);
 }
 
-template struct AxisTables<double>;
 template struct AxisTables<float>;
-// FP64 path: double in, double out.  Mixed path: FP32 transforms fed from float-float inputs,
-// FP32 intermediates, float-float results.
-template cudaError_t xpass<double, double, double>(const Geometry&, const DstAxis<double>&, const XArgs&, cudaStream_t);
+// FP32 transforms fed from float-float inputs, FP32 intermediates, float-float results
 template cudaError_t xpass<float, df64, float>(const Geometry&, const DstAxis<float>&, const XArgs&, cudaStream_t);
 template cudaError_t xpass<float, float, float>(const Geometry&, const DstAxis<float>&, const XArgs&, cudaStream_t);
 template cudaError_t xpass<float, float, df64>(const Geometry&, const DstAxis<float>&, const XArgs&, cudaStream_t);
-template cudaError_t ypass<double>(const Geometry&, const DstAxis<double>&, const YPassArgs<double>&, cudaStream_t);
 template cudaError_t ypass<float>(const Geometry&, const DstAxis<float>&, const YPassArgs<float>&, cudaStream_t);
 
 

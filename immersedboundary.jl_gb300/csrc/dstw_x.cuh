@@ -252,10 +252,6 @@ k_wxi(Geometry g, DstAxis<T> ax, XArgs a) {
       if (EPI == kEpiStore) {
 #pragma unroll 8
         for (int I = lane; I < ncol; I += NL) dst[I] = (Tout)U[I + 1];
-      } else if (EPI == kEpiSub) {
-        const A* sf = static_cast<const A*>(a.sub_from) + off;
-#pragma unroll 4
-        for (int I = lane; I < ncol; I += NL) dst[I] = (Tout)(sf[I] - A(U[I + 1]));
       } else if constexpr (is_df64<Tout>::value) {
         // x = x0 [+ x1] + d: the FP32 parts summed error-free, the (small) correction added
         // to the low part
@@ -354,16 +350,12 @@ cudaError_t launch_inv(const Geometry& g, const DstAxis<T>& ax, const XArgs& a, 
   return launch_k(k, dim3((total + kLines - 1) / kLines), dim3(kLines * NL), smem, s, g, ax, a);
 }
 
-// epilogues per output type: FP64 path store / subtract; mixed path FP32 store of the iterate
-// and float-float sums with the base iterate
+// epilogues per output type: FP32 store of the iterate, float-float sums with the base iterate
 template <typename T, typename Tout, int P, int NL>
 cudaError_t inv_p(const Geometry& g, const DstAxis<T>& ax, const XArgs& a, cudaStream_t s) {
   if (a.bc) return cudaErrorInvalidValue;
   if constexpr (std::is_same<Tout, T>::value) {
     if (a.epi == kEpiStore) return launch_inv<T, Tout, P, NL, kEpiStore>(g, ax, a, s);
-    if constexpr (std::is_same<T, double>::value) {
-      if (a.epi == kEpiSub) return launch_inv<T, Tout, P, NL, kEpiSub>(g, ax, a, s);
-    }
     return cudaErrorInvalidValue;
   } else {
     // a float-float result needs no base (a transform-only solve); a double one does

@@ -18,7 +18,6 @@ cudaError_t wx_fwd(const Geometry& g, const DstAxis<T>& ax, const XArgs& a, cuda
 }
 
 // FP64 path: double in.  Mixed path: float-float input, FP32 transforms.
-template cudaError_t wx_fwd<double, double>(const Geometry&, const DstAxis<double>&, const XArgs&, cudaStream_t);
 template cudaError_t wx_fwd<float, df64>(const Geometry&, const DstAxis<float>&, const XArgs&, cudaStream_t);
 
 }  // namespace ib

@@ -18,7 +18,6 @@ cudaError_t wx_inv(const Geometry& g, const DstAxis<T>& ax, const XArgs& a, cuda
 }
 
 // FP64 path: double out.  Mixed path: FP32 iterates and float-float results.
-template cudaError_t wx_inv<double, double>(const Geometry&, const DstAxis<double>&, const XArgs&, cudaStream_t);
 template cudaError_t wx_inv<float, float>(const Geometry&, const DstAxis<float>&, const XArgs&, cudaStream_t);
 template cudaError_t wx_inv<float, df64>(const Geometry&, const DstAxis<float>&, const XArgs&, cudaStream_t);
 

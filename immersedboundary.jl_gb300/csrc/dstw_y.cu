@@ -20,11 +20,8 @@ cudaError_t wypass(const Geometry& g, const DstAxis<T>& ax, const YPassArgs<T>& 
   return wypass_minb<T, IB_WDST_YMINB>(g, ax, a, s);
 }
 
-template cudaError_t wypass_minb<double, IB_WDST_YMINB>(const Geometry&, const DstAxis<double>&,
-                                                       const YPassArgs<double>&, cudaStream_t);
 template cudaError_t wypass_minb<float, IB_WDST_YMINB>(const Geometry&, const DstAxis<float>&, const YPassArgs<float>&,
                                                       cudaStream_t);
-template cudaError_t wypass<double>(const Geometry&, const DstAxis<double>&, const YPassArgs<double>&, cudaStream_t);
 template cudaError_t wypass<float>(const Geometry&, const DstAxis<float>&, const YPassArgs<float>&, cudaStream_t);
 
 }  // namespace ib

@@ -16,7 +16,7 @@ using wdst::Shape;
 using wdst::line_dst;
 using wdst::line_sync;
 
-template <typename T, int P, int NL, SpecOp OP, int MINB>
+template <typename T, int P, int NL, int MINB>
 __global__ void __launch_bounds__(kLines * NL, MINB)
 k_wy(Geometry g, DstAxis<T> ax, YPassArgs<T> a) {
   pdl_begin();
@@ -43,23 +43,17 @@ k_wy(Geometry g, DstAxis<T> ax, YPassArgs<T> a) {
     }
     line_sync<NL>(w + 1);
     line_dst<T, P, NL>(U, D, ax, lane, w + 1);
-    if (OP == SpecOp::kScale) {
-      const T* m = a.m1 + (int64_t)b * a.mstride + (int64_t)I * nrow;
-      for (int J0 = lane; J0 < nrow; J0 += LB * NL) {
-        T v[LB];
+    const T* m = a.m1 + (int64_t)b * a.mstride + (int64_t)I * nrow;
+    for (int J0 = lane; J0 < nrow; J0 += LB * NL) {
+      T v[LB];
 #pragma unroll
-        for (int u = 0; u < LB; ++u) v[u] = (J0 + NL * u < nrow) ? __ldg(&m[J0 + NL * u]) : T(0);
+      for (int u = 0; u < LB; ++u) v[u] = (J0 + NL * u < nrow) ? __ldg(&m[J0 + NL * u]) : T(0);
 #pragma unroll
-        for (int u = 0; u < LB; ++u)
-          if (J0 + NL * u < nrow) U[J0 + NL * u + 1] *= v[u];
-      }
-      line_sync<NL>(w + 1);
-      line_dst<T, P, NL>(U, D, ax, lane, w + 1);
-    } else {
-#pragma unroll 8
-      for (int J = lane; J < nrow; J += NL) U[J + 1] *= a.scal;
-      line_sync<NL>(w + 1);
+      for (int u = 0; u < LB; ++u)
+        if (J0 + NL * u < nrow) U[J0 + NL * u + 1] *= v[u];
     }
+    line_sync<NL>(w + 1);
+    line_dst<T, P, NL>(U, D, ax, lane, w + 1);
     T* dst = a.out + off;
 #pragma unroll 8
     for (int J = lane; J < nrow; J += NL) dst[J] = U[J + 1];
@@ -73,15 +67,9 @@ cudaError_t launch(const Geometry& g, const DstAxis<T>& ax, const YPassArgs<T>& 
   const int total = a.batch * (g.nx - 1);
   const int blocks = (total + kLines - 1) / kLines;
   cudaError_t e;
-  if (a.op == SpecOp::kFwd) {
-    auto k = k_wy<T, P, NL, SpecOp::kFwd, MINB>;
-    if ((e = set_smem_limit((const void*)k, smem)) != cudaSuccess) return e;
-    if ((e = launch_k(k, dim3(blocks), dim3(kLines * NL), smem, s, g, ax, a)) != cudaSuccess) return e;
-  } else {
-    auto k = k_wy<T, P, NL, SpecOp::kScale, MINB>;
-    if ((e = set_smem_limit((const void*)k, smem)) != cudaSuccess) return e;
-    if ((e = launch_k(k, dim3(blocks), dim3(kLines * NL), smem, s, g, ax, a)) != cudaSuccess) return e;
-  }
+  auto k = k_wy<T, P, NL, MINB>;
+  if ((e = set_smem_limit((const void*)k, smem)) != cudaSuccess) return e;
+  if ((e = launch_k(k, dim3(blocks), dim3(kLines * NL), smem, s, g, ax, a)) != cudaSuccess) return e;
   return cudaGetLastError();
 }
 

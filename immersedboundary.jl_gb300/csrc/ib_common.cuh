@@ -103,7 +103,28 @@ template <typename T> struct AxisTables {
   void release();
 };
 
+// Tables of one axis for the FP64 passes (dstfx.cu), factors in the fixed-point form of fx.cuh.
+namespace fx { struct cwgt; struct wgt; }
+struct FxAxis {
+  int n, M, nstages;
+  int radix[kMaxStages];
+  int ns[kMaxStages];          // product of the radices before the stage
+  unsigned magic[kMaxStages];  // ceil(2^32 / ns): j / ns = umulhi(j, magic)
+  int twoff[kMaxStages];       // stage's twiddles in tw: [r - 1][k], r < radix, k < ns
+  const fx::cwgt* tw;          // e^{-2 pi i r k / (ns radix)}
+  const fx::cwgt* post;        // [M/2+1] e^{-2 pi i k / n}
+  const fx::wgt* sin2;         // [M] 2 sin(pi j / n)
+};
+struct FxTables {
+  FxAxis d{};
+  void* mem = nullptr;
+  cudaError_t build(int n);
+  void release();
+};
+
 bool dst_axis_supported(int n);
+// radix plan of an M-point FFT (number of stages, or -1): 4s and 8s, then 3s, then 5s
+int plan_radices(int M, int* radix);
 // both axes have warp-per-line tables: the solves use the dstw passes (transposed intermediate)
 bool wdst_axis_supported(int n);
 
@@ -115,11 +136,6 @@ cudaError_t set_smem_limit(const void* fn, size_t bytes);
 // ----------------------------------------------------------------------------------------------
 // Every pass takes arrays of (nx-1)*(ny-1) values; `batch` arrays live at stride nG.
 // Spectral multipliers are stored per array slot with stride `mstride` (0 = shared).
-enum class SpecOp : int {
-  kScale = 0,      // out = S_y(m1 * S_y(in1))
-  kFwd = 2,        // out = scal * S_y(in1)   (one transform only)
-};
-
 // x pass: a 1-D sine transform along x of every row of `batch` arrays (compute type T).
 // prologue (how a row is formed before the transform):
 //   kProLoad   row = in                                  (in: Tin)
@@ -129,12 +145,11 @@ enum class SpecOp : int {
 // either optionally plus fac * apply_bc(bc) on the edges (bc != nullptr)
 // epilogue (what is stored):
 //   kEpiStore       out = row                              (out: Tout)
-//   kEpiSub         out = sub_from - row
 //   kEpiAddBase     out = base [+ base2] + row             (FP64 sum)
 //   kEpiSubAddBase  out = sub_from - (base [+ base2] + row)
 //   kEpiAddTo       out = sub_from + (base [+ base2] + row)  (float-float output; out may be sub_from)
 enum XPro : int { kProLoad = 0, kProResid = 1, kProResidD = 2 };
-enum XEpi : int { kEpiStore = 0, kEpiSub = 1, kEpiAddBase = 2, kEpiSubAddBase = 3, kEpiAddTo = 4 };
+enum XEpi : int { kEpiStore = 0, kEpiAddBase = 2, kEpiSubAddBase = 3, kEpiAddTo = 4 };
 
 struct XArgs {
   const void* in;           // Tin
@@ -143,7 +158,7 @@ struct XArgs {
   int64_t stride;           // elements between batch slots (in, out, base, sub_from)
   const void* bc;           // apply_bc ring per slot (stride nbc) or nullptr; element type is the
   double bcfac;             //   pass's exact type (double, or df64 in the mixed path)
-  const void* sub_from;     // kEpiSub / kEpiSubAddBase (same element type as bc)
+  const void* sub_from;     // kEpiSubAddBase / kEpiAddTo (same element type as bc)
   const float* base;        // x0 of the refinement (kProResid, kEpiAddBase)
   const float* base2;       // optional second FP32 part of x0 (second refinement sweep)
   const df64* based;        // float-float x0 (kProResidD)
@@ -162,12 +177,22 @@ template <typename T>
 struct YPassArgs {
   const T* in1; T* out; int batch; int64_t stride;
   const T* m1; int64_t mstride;                // multipliers (per slot stride)
-  SpecOp op;
-  T scal;                                      // kFwd scale
 };
 
 template <typename T>
 cudaError_t ypass(const Geometry& g, const DstAxis<T>& ax, const YPassArgs<T>& a, cudaStream_t s);
+
+// The FP64 passes (dstfx.cu), arrays of nG doubles.  The intermediate of a solve is stored transposed,
+// column by column: element (I, J) of slot b at b*nG + I*(ny-1) + J.
+//   fx_fwd:   in [+ bcfac * apply_bc(bc) on the edges] -> x transform -> transposed store
+//   fx_ypass: per column S_y, times mult (per slot stride mstride), S_y; mult == nullptr: scal * S_y
+//   fx_inv:   transposed load -> x transform -> out, or out = sub_from - (.) (out may be sub_from)
+cudaError_t fx_fwd(const Geometry& g, const FxAxis& ax, const double* in, double* out, int batch, const double* bc,
+                   double bcfac, cudaStream_t s);
+cudaError_t fx_ypass(const Geometry& g, const FxAxis& ay, const double* in, double* out, int batch, const double* mult,
+                     int64_t mstride, double scal, cudaStream_t s);
+cudaError_t fx_inv(const Geometry& g, const FxAxis& ax, const double* in, double* out, int batch,
+                   const double* sub_from, cudaStream_t s);
 
 // Warp-per-line passes (dstw_*.cu), for axes with wdst_axis_supported.  The intermediate of a
 // solve is stored transposed, column by column: element (I, J) of slot b at b*stride + I*(ny-1) + J.
@@ -446,11 +471,10 @@ struct ProfScope {
 // ----------------------------------------------------------------------------------------------
 struct LapView {
   Geometry g;
-  DstAxis<double> ax, ay;
+  FxAxis ax, ay;
   const double* mlap;
   cudaStream_t stream;
   int device;
-  bool wdst;  // both axes use the warp-per-line passes (wx_fwd / wypass / wx_inv)
 };
 
 // Makes `dev` the current device for the lifetime of the guard and restores the caller's

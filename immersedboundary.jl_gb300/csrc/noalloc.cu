@@ -6,7 +6,7 @@
 // allocation's implicit synchronisation of the whole device.  ib_op_laplacian_inv allocates its
 // work buffer on every call; this variant keeps that work buffer in a fixed array compiled into
 // the library instead, and runs the same transform kernels as ib_op_laplacian_inv on the same
-// handle (warp-per-line passes where the handle uses them, Stockham passes otherwise).
+// handle.
 //
 // The array is a file-scope __device__ variable of kNoAllocMaxValues FP64 values (32 MiB).
 // Every GPU that loads the library holds it until the process exits.  In host code its name
@@ -45,35 +45,9 @@ extern "C" int ib_op_laplacian_inv_noalloc(ib_handle* h, int32_t batch, const do
   if (e != cudaSuccess) return ib_handle_fail(h, IB_ERR_CUDA, cudaGetErrorString(e));
   double* w = static_cast<double*>(wp);
   // x = F2D(mlap .* F2D(b)): x pass into the fixed work array, y pass in place, x pass out
-  ib::XArgs xa{};
-  xa.in = b;
-  xa.out = w;
-  xa.batch = batch;
-  xa.stride = v.g.nG;
-  xa.bcfac = 1.0;
-  xa.pro = ib::kProLoad;
-  xa.epi = ib::kEpiStore;
-  ib::YPassArgs<double> ya{};
-  ya.in1 = w;
-  ya.out = w;
-  ya.batch = batch;
-  ya.stride = v.g.nG;
-  ya.m1 = v.mlap;
-  ya.mstride = 0;
-  ya.op = ib::SpecOp::kScale;
-  ib::XArgs xb = xa;
-  xb.in = w;
-  xb.out = x;
-  if (v.wdst) {
-    // warp-per-line passes; the work array holds the transposed intermediate
-    e = ib::wx_fwd<double, double>(v.g, v.ax, xa, v.stream);
-    if (e == cudaSuccess) e = ib::wypass<double>(v.g, v.ay, ya, v.stream);
-    if (e == cudaSuccess) e = ib::wx_inv<double, double>(v.g, v.ax, xb, v.stream);
-  } else {
-    e = ib::xpass<double, double, double>(v.g, v.ax, xa, v.stream);
-    if (e == cudaSuccess) e = ib::ypass<double>(v.g, v.ay, ya, v.stream);
-    if (e == cudaSuccess) e = ib::xpass<double, double, double>(v.g, v.ax, xb, v.stream);
-  }
+  e = ib::fx_fwd(v.g, v.ax, b, w, batch, nullptr, 1.0, v.stream);
+  if (e == cudaSuccess) e = ib::fx_ypass(v.g, v.ay, w, w, batch, v.mlap, 0, 1.0, v.stream);
+  if (e == cudaSuccess) e = ib::fx_inv(v.g, v.ax, w, x, batch, nullptr, v.stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(v.stream);
   if (e != cudaSuccess) return ib_handle_fail(h, IB_ERR_CUDA, cudaGetErrorString(e));
   return IB_OK;

@@ -440,7 +440,7 @@ cudaError_t gy_pass(const Geometry& g, const SineGemm& ay, const YPassArgs<float
                     cudaStream_t s) {
   if (a.batch <= 0) return cudaSuccess;
   // a.out may be a.in1: the first product has read all of it before the second one writes
-  if (a.stride != g.nG || ay.n != g.ny || a.op != SpecOp::kScale || a.out == work) return cudaErrorInvalidValue;
+  if (a.stride != g.nG || ay.n != g.ny || a.out == work) return cudaErrorInvalidValue;
   ProfScope prof(kClassYPass, s);
   const int ncol = g.nx - 1, nrow = g.ny - 1;
   SgIn in{a.in1, nrow, a.batch * ncol, nrow};

@@ -59,7 +59,7 @@ struct ib_handle {
   double dt = 0, re = 0, beta0 = 1.5, beta1 = -0.5;
   int nbodies = 0, nb = 0, nf = 0;
   int precision = IB_PREC_FP64;
-  AxisTables<double> axx, axy;
+  FxTables axx, axy;               // FP64 passes
   AxisTables<float> axx32, axy32;  // mixed precision: FP32 transform tables
   // state
   double* G[2] = {nullptr, nullptr};
@@ -229,52 +229,13 @@ SolveOp op_cn_all(const ib_handle* h) { return {h->mCN1, h->mCN1_32, h->g.nG, h-
 SolveOp op_cn1(const ib_handle* h) { return {h->mCN1, h->mCN1_32, 0, h->d_one, h->d_alpha, 0}; }
 
 // FP64 solve of `batch` arrays: out = F2D(m .* F2D(in [+ apply_bc(bc, 1)])), optional
-// subtract epilogue out = sub_from - (...).  w: FP64 work of batch arrays.
+// subtract epilogue out = sub_from - (...).  w: FP64 work of batch arrays (the transposed
+// intermediate).
 cudaError_t poisson64(ib_handle* h, const double* in, double* out, int batch, const double* bc, const SolveOp& op,
                       const double* sub_from, double* w) {
-  if (h->wdst) {
-    // warp-per-line passes; w holds the transposed intermediate
-    XArgs xa{};
-    xa.in = in; xa.out = w; xa.batch = batch; xa.stride = h->g.nG; xa.bc = bc; xa.bcfac = 1.0;
-    xa.pro = kProLoad; xa.epi = kEpiStore;
-    CE((wx_fwd<double, double>(h->g, h->axx.d, xa, h->stream)));
-    YPassArgs<double> ya{};
-    ya.in1 = w; ya.out = w; ya.batch = batch; ya.stride = h->g.nG; ya.m1 = op.m64; ya.mstride = op.mstride;
-    ya.op = SpecOp::kScale;
-    CE(wypass<double>(h->g, h->axy.d, ya, h->stream));
-    XArgs xb{};
-    xb.in = w; xb.out = out; xb.batch = batch; xb.stride = h->g.nG; xb.sub_from = sub_from;
-    xb.pro = kProLoad; xb.epi = sub_from ? kEpiSub : kEpiStore;
-    return wx_inv<double, double>(h->g, h->axx.d, xb, h->stream);
-  }
-  XArgs xa{};
-  xa.in = in;
-  xa.out = w;
-  xa.batch = batch;
-  xa.stride = h->g.nG;
-  xa.bc = bc;
-  xa.bcfac = 1.0;
-  xa.pro = kProLoad;
-  xa.epi = kEpiStore;
-  CE((xpass<double, double, double>(h->g, h->axx.d, xa, h->stream)));
-  YPassArgs<double> ya{};
-  ya.in1 = w;
-  ya.out = w;
-  ya.batch = batch;
-  ya.stride = h->g.nG;
-  ya.m1 = op.m64;
-  ya.mstride = op.mstride;
-  ya.op = SpecOp::kScale;
-  CE(ypass<double>(h->g, h->axy.d, ya, h->stream));
-  XArgs xb{};
-  xb.in = w;
-  xb.out = out;
-  xb.batch = batch;
-  xb.stride = h->g.nG;
-  xb.sub_from = sub_from;
-  xb.pro = kProLoad;
-  xb.epi = sub_from ? kEpiSub : kEpiStore;
-  return xpass<double, double, double>(h->g, h->axx.d, xb, h->stream);
+  CE(fx_fwd(h->g, h->axx.d, in, w, batch, bc, 1.0, h->stream));
+  CE(fx_ypass(h->g, h->axy.d, w, w, batch, op.m64, op.mstride, 1.0, h->stream));
+  return fx_inv(h->g, h->axx.d, w, out, batch, sub_from, h->stream);
 }
 
 // Mixed-precision solve: FP32 sine transforms refined with float-float residuals.
@@ -297,7 +258,6 @@ cudaError_t poisson_mixed(ib_handle* h, const df64* in, df64* out, int batch, co
   ya.stride = g.nG;
   ya.m1 = op.m32;
   ya.mstride = op.mstride;
-  ya.op = SpecOp::kScale;
   XArgs a{};
   a.batch = batch;
   a.stride = g.nG;
@@ -496,7 +456,6 @@ cudaError_t vort2flux_levels(ib_handle* h, df64* gam, df64* psi, df64* q, df64* 
   CE((wx_fwd<float, df64>(g, ax, a, s)));
   YPassArgs<float> ya{};
   ya.in1 = h->w32; ya.out = h->w32; ya.batch = L; ya.stride = nG; ya.m1 = op.m32; ya.mstride = op.mstride;
-  ya.op = SpecOp::kScale;
   CE(wypass<float>(g, ay, ya, s));
   a = XArgs{};
   a.batch = L; a.stride = nG; a.bcfac = 1.0;
@@ -1689,7 +1648,6 @@ bool ib_handle_lap_view(const ib_handle* h, ib::LapView* v) {
   v->mlap = h->mLap;
   v->stream = h->stream;
   v->device = h->device;
-  v->wdst = h->wdst;
   return true;
 }
 
@@ -1822,14 +1780,10 @@ int ib_create(const ib_problem* p, ib_handle** out) {
   h->cn_pred = h->refine >= 2;
   if (const char* env = std::getenv("IBGB300_CN_PREDICTOR")) h->cn_pred = h->cn_pred && env[0] != '0';
   if (const char* env = std::getenv("IBGB300_PC_ASSEMBLY")) h->asm_fp64 = std::strcmp(env, "fp64") == 0;
-  // transform kernels, by measurement on GB300: FP32 (mixed) transforms run faster one warp
-  // per line where both axes allow it; FP64 transforms are FP64-pipe bound and the shared-memory
-  // Stockham passes, with fewer twiddle multiplies and no transposing copies, are faster up to
-  // 1024-cell axes (3.85 vs 4.35 ms per 1024^2 4-level step), the warp passes at 2048 cells
-  // (19.3 vs 21.4 ms per 2048^2 5-level step).
-  // IBGB300_DST=warp|stockham overrides the choice for both precisions.
+  // FP32 (mixed) transforms run faster one warp per line where both axes allow it
+  // (IBGB300_DST=warp|stockham overrides the choice); FP64 ones have one form (dstfx.cu)
   const bool wsup = wdst_axis_supported(p->nx) && wdst_axis_supported(p->ny);
-  h->wdst = wsup && (p->precision == IB_PREC_MIXED || std::max(p->nx, p->ny) >= 2048);
+  h->wdst = wsup && p->precision != IB_PREC_FP64;
   h->gdst = want_tc;
   bool pin_form = want_tc, pin_v2f = false;
   if (const char* env = std::getenv("IBGB300_DST")) {
@@ -2420,7 +2374,8 @@ int ib_get_info(ib_handle* h, ib_info* info) {
   info->device_bytes = h->device_bytes;
   info->setup_ms = h->setup_ms;
   info->vort2flux_order = h->v2f_levels ? IB_V2F_LEVELS : IB_V2F_SEQUENTIAL;
-  info->transform_form = h->gdst ? IB_FORM_TENSOR : (h->wdst ? IB_FORM_WARP : IB_FORM_STOCKHAM);
+  info->transform_form = h->precision == IB_PREC_FP64 ? IB_FORM_FIXED
+                         : h->gdst ? IB_FORM_TENSOR : (h->wdst ? IB_FORM_WARP : IB_FORM_STOCKHAM);
   info->scheme = h->scheme;
   info->rkc_stages = h->rkc_s;
   int sms = 0;
@@ -2511,23 +2466,12 @@ int ib_op_dst2(ib_handle* h, int32_t batch, const double* in, double* out) {
   if (batch < 1) return IB_ERR_INVALID;
   double* w;
   CK(cudaMalloc(&w, sizeof(double) * batch * g.nG));
-  // RODFT00 in both dimensions = 4 F_y F_x (F: the half-scaled transform of dst.cu)
-  XArgs xa{};
-  xa.in = in; xa.out = w; xa.batch = batch; xa.stride = g.nG; xa.pro = kProLoad; xa.epi = kEpiStore;
-  YPassArgs<double> ya{};
-  ya.in1 = w; ya.out = out; ya.batch = batch; ya.stride = g.nG; ya.op = SpecOp::kFwd; ya.scal = 4.0;
-  cudaError_t e;
-  if (h->wdst) {
-    // warp-per-line passes leave the result transposed ([I][J] per slot): transpose it back
-    e = wx_fwd<double, double>(g, h->axx.d, xa, s);
-    ya.out = w;
-    if (e == cudaSuccess) e = wypass<double>(g, h->axy.d, ya, s);
-    for (int b = 0; b < batch && e == cudaSuccess; ++b)
-      e = transpose(w + (int64_t)b * g.nG, out + (int64_t)b * g.nG, g.nx - 1, g.ny - 1, s);
-  } else {
-    e = xpass<double, double, double>(g, h->axx.d, xa, s);
-    if (e == cudaSuccess) e = ypass<double>(g, h->axy.d, ya, s);
-  }
+  // RODFT00 in both dimensions = 4 F_y F_x (F: the half-scaled transform of dstfx.cu); the passes
+  // leave the result transposed ([I][J] per slot): transpose it back
+  cudaError_t e = fx_fwd(g, h->axx.d, in, w, batch, nullptr, 1.0, s);
+  if (e == cudaSuccess) e = fx_ypass(g, h->axy.d, w, w, batch, nullptr, 0, 4.0, s);
+  for (int b = 0; b < batch && e == cudaSuccess; ++b)
+    e = transpose(w + (int64_t)b * g.nG, out + (int64_t)b * g.nG, g.nx - 1, g.ny - 1, s);
   cudaStreamSynchronize(s);
   cudaFree(w);
   CK(e);

@@ -43,7 +43,8 @@ extern "C" {
 
 /* arithmetic of the fluid solve (state, nonlinear term, Schur solve and forces are FP64 in
  * every mode) */
-#define IB_PREC_FP64 0   /* every sine transform in FP64 (the reference's arithmetic) */
+#define IB_PREC_FP64 0   /* FP64 throughout (the reference's arithmetic); the sine transforms run in 64-bit
+                            block fixed point, with less rounding error than in FP64 */
 #define IB_PREC_MIXED 1  /* FP32 sine transforms refined with float-float residuals (refine_sweeps);
                             state and stencils in float-float (two-float) arithmetic */
 #define IB_PREC_MIXED_TC 2  /* as IB_PREC_MIXED, with every sine transform a BF16x3 split-precision

@@ -30,6 +30,7 @@ typedef struct ib_info {
 #define IB_FORM_STOCKHAM 0   /* shared-memory Stockham FFT passes, 64 threads per line */
 #define IB_FORM_WARP 1       /* warp-per-line FFT passes with a transposed intermediate */
 #define IB_FORM_TENSOR 2     /* BF16x3 sine-matrix GEMMs on the tensor cores (tcgen05) */
+#define IB_FORM_FIXED 3      /* FP64 handles: passes in 64-bit block fixed point */
 
 int ib_get_info(ib_handle* h, ib_info* info);
 
