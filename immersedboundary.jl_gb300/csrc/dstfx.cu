@@ -16,15 +16,17 @@
 // A line with an infinity or NaN becomes NaN throughout, as the FP64 transform made it.  Sums of
 // integers do not depend on their order, so results are the same bits for any NT.
 //
-// Lines run along x as they lie in memory; the intermediate of a solve is stored transposed (element
-// (I, J) of slot b at b*stride + I*(ny-1) + J), so the y pass reads and writes whole columns.
+// A pass reads its lines as they lie in memory and stores them transposed (the forward x pass, the y
+// pass), so that the next pass's lines lie in memory: 32 or 64 bytes at a time, written without
+// waiting, where a transposing load would stall the block.
 //
-// What bounds it: instruction issue (243 instructions per value and transform at 1024 cells, 2.0-2.5
-// of 4 issued per clock) at large sizes, the latency of a line's chain at small ones.  Measured
-// against the FP64-arithmetic passes (shared-memory Stockham, and one warp per line at 2048 cells),
-// which the FP64 pipe's two lanes per SM bound: a 2048^2 Poisson solve of two fields 2.09 -> 0.67 ms,
-// a 1024^2 x 4-level two-body step 3.75 -> 1.44 ms, 200^2 x 5 0.81 -> 0.58, 128^2 x 3 0.53 -> 0.33, with
-// 0.25 of their error on the 2048^2 solve (4.3e-15 against 1.8e-14).
+// What bounds it: the integer pipes and the latency between them (ncu, 1024-cell lines: ALU 59% and
+// FMA-heavy 46% busy, 2.5 of 4 instructions issued per clock), and the latency of a line's chain where
+// a launch has few lines.  Measured against the FP64-arithmetic passes (shared-memory Stockham, one
+// warp per line at 2048 cells), which the FP64 pipe's two lanes per SM bound: a 2048^2 Poisson solve
+// of two fields 2.09 -> 0.54 ms, a 1024^2 x 4-level two-body step 3.75 -> 1.30 ms, 384 x 256 x 4 RKC
+// 0.88 -> 0.43, 200^2 x 5 0.81 -> 0.44, 128^2 x 3 0.53 -> 0.28, with a quarter of their error on the
+// 2048^2 solve (4.3e-15 against 1.8e-14).
 #include "fx.cuh"
 #include "ib_common.cuh"
 
@@ -47,19 +49,70 @@ constexpr int kRedSlots = 2 + kMaxStages;  // reductions of one transform: large
 // padded index of a complex value / of a result: one spare slot after every 8
 __host__ __device__ constexpr int cpad(int i) { return i + (i >> 3); }
 
-// 8-byte words of one line's buffer: M complex values padded; congruent to 4 mod 16, so that four
-// lines' words at one index lie in different banks
-__host__ __device__ inline int line_words(int M) { return (2 * M + M / 4 + 8 + 15) / 16 * 16 + 4; }
+// The results F_i, i = 1..n-1, of a line lie at word cpad(i / 2) of two regions of its buffer, the
+// odd ones in the first, the even ones in the second, 8 banks (of 8 bytes) away from the first.
+__host__ __device__ constexpr int even_off(int M) { return (M + (M >> 3) + 6 + 7) / 16 * 16 + 8; }
+// 8-byte words of one line's buffer: M complex values padded, or both regions; congruent to 2 mod 16,
+// so that four lines' words at two successive indices of either parity lie in different banks
+__host__ __device__ constexpr int line_words(int M) { return (even_off(M) + cpad(M) + 14) / 16 * 16 + 2; }
 
-// Radices of the axes with compiled-in lengths, whose index arithmetic is constant.  Powers of two
-// and 3 * 2^k: one butterfly per thread and stage where that fills the group, small radices where
-// lines are short (then a call's latency counts, not its throughput).
+#ifndef S64
+#define S64 32, 2
+#endif
+#ifndef P64
+#define P64 4,4,4
+#endif
+#ifndef S96
+#define S96 32, 3
+#endif
+#ifndef P96
+#define P96 4,4,6
+#endif
+#ifndef S128
+#define S128 32, 4
+#endif
+#ifndef P128
+#define P128 8,4,4
+#endif
+#ifndef S192
+#define S192 32, 6
+#endif
+#ifndef P192
+#define P192 8,4,6
+#endif
+#ifndef S256
+#define S256 32, 8
+#endif
+#ifndef P256
+#define P256 8,8,4
+#endif
+#ifndef S384
+#define S384 64, 6
+#endif
+#ifndef P384
+#define P384 8,8,6
+#endif
+#ifndef S512
+#define S512 64, 8
+#endif
+#ifndef P512
+#define P512 8,8,8
+#endif
+#ifndef S768
+#define S768 128, 6
+#endif
+#ifndef P768
+#define P768 8,4,4,6
+#endif
+// Radices of the axes with compiled-in lengths, whose index arithmetic is constant: 64 P cells,
+// P = 2^k or 3 2^k.  Large radices where many values lie in a thread's registers (M = 384 and up),
+// small ones where lines are short and a launch lasts as long as a line's chain.
 template <int M> struct Plan {
   static constexpr int n = 0;
   static constexpr int r[1] = {0};
 };
 #define IB_FX_PLANS(X) \
-  X(64, 4, 4, 4) X(96, 4, 4, 6) X(128, 8, 4, 4) X(192, 8, 4, 6) X(256, 8, 8, 4) X(384, 8, 8, 6) X(512, 8, 8, 8) \
+  X(64, 4, 4, 4) X(96, 4, 4, 6) X(128, 8, 4, 4) X(192, 4, 4, 4, 3) X(256, 4, 4, 4, 4) X(384, 8, 8, 6) X(512, 8, 8, 8) \
   X(768, 8, 4, 4, 6) X(1024, 8, 8, 4, 4)
 #define IB_FX_PLAN(M, ...)                                 \
   template <> struct Plan<M> {                             \
@@ -182,9 +235,6 @@ __device__ __forceinline__ void fixed_stages(const Group<NT>& G, const FxAxis& a
   }
 }
 
-// The results F_i, i = 1..n-1, of a line lie at word cpad(i / 2) of two regions of its buffer: the
-// odd ones in the first, the even ones in the second.
-__host__ __device__ constexpr int even_off(int M) { return M + (M >> 3) + 8; }
 __device__ __forceinline__ i64* result_at(i64* buf, int M, int i) {
   return buf + ((i & 1) ? 0 : even_off(M)) + cpad(i >> 1);
 }
@@ -206,19 +256,22 @@ struct Pairs {
 // exponent of a line whose values are not finite
 constexpr int kNotFinite = 1 << 20;
 
-// the double of a result on scale q
+// the double of a result on a safe scale q
 __device__ __forceinline__ double to_double(i64 v, int q) {
-  if (q == kNotFinite) return __longlong_as_double(0x7ff8000000000000ll);
-  if (fx::safe_scale(q)) return __longlong_as_double((i64)fx::from_fixed(v, q));
-  return ldexp((double)v, -q);  // at the ends of the exponent range: subnormal results, or overflow
+  return __longlong_as_double((i64)fx::from_fixed(v, q));
 }
-
+// not finite, or at the ends of the exponent range (subnormal results, or overflow)
+__device__ __noinline__ double to_double_slow(i64 v, int q) {
+  if (q == kNotFinite) return __longlong_as_double(0x7ff8000000000000ll);
+  return ldexp((double)v, -q);
+}
 // DST-I of a line given as pairs a[i] = y_j, b[i] = y_{n-j}, j = t + NT i (j = 0: a = y_{n/2}, b
 // unused); the results are in place after the closing barrier.  Returns their scale q
-// (F = value 2^-q), the same on every thread of the group.
-template <int NT, int PP, int M_>
+// (F = value 2^-q), the same on every thread of the group.  `before_scan` runs before the last
+// phase, with few registers in use: a place for loads that are needed next.
+template <int NT, int PP, int M_, class Hook>
 __device__ __forceinline__ int line_transform(const Group<NT>& G, const FxAxis& ax, const double (&a)[PP],
-                                              const double (&b)[PP]) {
+                                              const double (&b)[PP], Hook before_scan) {
   const int t = G.t, M = M_ ? M_ : ax.M, n = 2 * M;
   // 1. the line's largest exponent
   unsigned m = 0;
@@ -325,6 +378,7 @@ __device__ __forceinline__ int line_transform(const Group<NT>& G, const FxAxis& 
     }
   }
   G.bar();
+  before_scan();
   // 5. odd outputs: prefix sums of D, chunk by chunk
   {
     constexpr bool kEven = M_ == NT * PP;  // chunks of exactly PP values
@@ -362,6 +416,16 @@ __device__ __forceinline__ int line_transform(const Group<NT>& G, const FxAxis& 
 // ------------------------------------------------------------------------------------------------
 // passes
 // ------------------------------------------------------------------------------------------------
+// Lines per block: 4 (stores of 32-byte segments), or 2 of the longest.  Two blocks of 256 threads per
+// SM or four of 128 leave 128 registers a thread; capping at 80 or 64 for more warps costs more in
+// spills than it hides (1024^2 solve of one field: 54.5 us, 57.7, 62.2).
+template <int NT>
+struct Bounds {
+  static constexpr int kLines = NT == 128 ? 2 : 4;
+  static constexpr int kThreads = kLines * NT;
+  static constexpr int kBlocks = 512 / kThreads;
+};
+
 struct Smem {
   i64* line;      // this group's line buffer
   i64* lines;     // line buffer of group 0
@@ -399,11 +463,49 @@ __device__ __forceinline__ void load_pairs(const double* src, int M, int t, doub
   }
 }
 
+// f(i, middle, F_j, F_{n-j}) for the thread's pairs (of the middle pair only the first value)
+template <int NT, int PP, int M_, class F>
+__device__ __forceinline__ void with_results(const Pairs<NT>& w, int M, int t, int q, F f) {
+  if (fx::safe_scale(q)) {
+#pragma unroll
+    for (int i = 0; i < PP; ++i)
+      if (M_ == NT * PP || t + NT * i < M) {
+        const bool mid = i == 0 && t == 0;
+        f(i, mid, to_double(*w.a(i, mid), q), to_double(*w.b(i), q));
+      }
+  } else {
+#pragma unroll
+    for (int i = 0; i < PP; ++i)
+      if (M_ == NT * PP || t + NT * i < M) {
+        const bool mid = i == 0 && t == 0;
+        f(i, mid, to_double_slow(*w.a(i, mid), q), to_double_slow(*w.b(i), q));
+      }
+  }
+}
+
+// The results of the block's lines line0 .. line0 + lpb - 1 (of `total`, `per` lines to an array of
+// `stride` values), transposed: the block's lines at one index are adjacent in memory.
 template <int NT>
-struct Bounds {
-  static constexpr int kThreads = NT == 128 ? 512 : 256;
-  static constexpr int kBlocks = NT == 128 ? 1 : 3;
-};
+__device__ __forceinline__ void store_transposed(const Smem& sm, int M, int line0, int total, int per,
+                                                 int64_t stride, double* out) {
+  __syncthreads();
+  constexpr int lpb = Bounds<NT>::kLines;
+  const int b0 = line0 / per, J0 = line0 - b0 * per, w = threadIdx.x % lpb;
+  if (line0 + w >= total) return;
+  const int wrap = J0 + w >= per;
+  i64* buf = sm.lines + (size_t)w * line_words(M);
+  const int q = sm.q[w];
+  double* dst = out + (int64_t)(b0 + wrap) * stride + (J0 + w - (wrap ? per : 0));
+  if (fx::safe_scale(q)) {
+#pragma unroll 8
+    for (int I = threadIdx.x / lpb; I < 2 * M - 1; I += NT)
+      dst[(int64_t)I * per] = to_double(*result_at(buf, M, I + 1), q);
+  } else {
+#pragma unroll 1
+    for (int I = threadIdx.x / lpb; I < 2 * M - 1; I += NT)
+      dst[(int64_t)I * per] = to_double_slow(*result_at(buf, M, I + 1), q);
+  }
+}
 
 // x transform of rows as they lie in memory -> transposed intermediate; optional apply_bc(bc) on the
 // edges (fluid-ops.jl:249-275)
@@ -412,7 +514,8 @@ __global__ void __launch_bounds__(Bounds<NT>::kThreads, Bounds<NT>::kBlocks)
 k_fx_fwd(Geometry g, FxAxis ax, const double* __restrict__ in, double* __restrict__ out, int batch,
          const double* __restrict__ bc, double bcfac) {
   pdl_begin();
-  const int M = M_ ? M_ : ax.M, lpb = blockDim.x / NT, grp = threadIdx.x / NT;
+  constexpr int lpb = Bounds<NT>::kLines;
+  const int M = M_ ? M_ : ax.M, grp = threadIdx.x / NT;
   const Smem sm = carve<NT>(M, lpb, grp);
   const Group<NT> G{(int)threadIdx.x % NT, grp, sm.line, sm.red};
   const int n = 2 * M, ncol = n - 1, nrow = g.ny - 1, total = batch * nrow;
@@ -438,133 +541,93 @@ k_fx_fwd(Geometry g, FxAxis ax, const double* __restrict__ in, double* __restric
         v[0] += bcfac * r[g.R + 1 + J];
       }
     }
-    const int q = line_transform<NT, PP, M_>(G, ax, u, v);
+    const int q = line_transform<NT, PP, M_>(G, ax, u, v, [] {});
     if (G.t == 0) sm.q[grp] = q;
   }
-  __syncthreads();
-  // transposed store: the block's rows at one column are adjacent in memory
-  const int b0 = row0 / nrow, J0 = row0 - b0 * nrow, sh = 31 - __clz(lpb);
-  const int w = threadIdx.x & (lpb - 1);
-  if (row0 + w < total) {
-    const int wrap = J0 + w >= nrow;
-    i64* buf = sm.lines + (size_t)w * line_words(M);
-    const int q = sm.q[w];
-    double* dst = out + (int64_t)(b0 + wrap) * g.nG + (J0 + w - (wrap ? nrow : 0));
-#pragma unroll 4
-    for (int I = threadIdx.x >> sh; I < ncol; I += NT)
-      dst[(int64_t)I * nrow] = to_double(*result_at(buf, M, I + 1), q);
-  }
+  store_transposed<NT>(sm, M, row0, total, nrow, g.nG, out);
 }
 
-// y pass on the transposed intermediate: column by column S_y, times m, S_y (or scal S_y only)
+// y pass: columns of the transposed intermediate, S_y, times m, S_y (or S_y only), times 2^log2scale,
+// stored row-major
 template <int NT, int PP, int M_>
 __global__ void __launch_bounds__(Bounds<NT>::kThreads, Bounds<NT>::kBlocks)
-k_fx_y(Geometry g, FxAxis ax, const double* in, double* out, int batch, const double* mult, int64_t mstride,
-       double scal) {
+k_fx_y(Geometry g, FxAxis ax, const double* __restrict__ in, double* __restrict__ out, int batch,
+       const double* mult, int64_t mstride, int log2scale) {
   pdl_begin();
-  const int M = M_ ? M_ : ax.M, lpb = blockDim.x / NT, grp = threadIdx.x / NT;
+  constexpr int lpb = Bounds<NT>::kLines;
+  const int M = M_ ? M_ : ax.M, grp = threadIdx.x / NT;
   const Smem sm = carve<NT>(M, lpb, grp);
   const Group<NT> G{(int)threadIdx.x % NT, grp, sm.line, sm.red};
-  const int n = 2 * M, ncol = g.nx - 1, nrow = n - 1;
-  const int col = blockIdx.x * lpb + grp;
-  if (col >= batch * ncol) return;
-  const int b = col / ncol, I = col - b * ncol, t = G.t;
-  const int64_t off = (int64_t)b * g.nG + (int64_t)I * nrow;
-  const Pairs<NT> w(G.buf, M, t);
-  double u[PP], v[PP];
-  load_pairs<NT, PP, M_>(in + off, M, t, u, v);
-  int q = line_transform<NT, PP, M_>(G, ax, u, v);
-  if (mult) {
-    // the products take the results' places in the line buffer: the thread that made them reads them
-    const double* m = mult + (int64_t)b * mstride + (int64_t)I * nrow;
-#pragma unroll 2
-    for (int i = 0; i < PP; ++i) {
-      const bool mid = i == 0 && t == 0;
-      if (M_ == NT * PP || t + NT * i < M) {
-        i64* x = w.a(i, mid);
-        *x = __double_as_longlong(to_double(*x, q) * m[mid ? M - 1 : t + NT * i - 1]);
-        x = w.b(i);
-        if (!mid) *x = __double_as_longlong(to_double(*x, q) * m[n - 1 - t - NT * i]);
-      }
+  const int ncol = g.nx - 1, nrow = 2 * M - 1, total = batch * ncol;
+  const int col0 = blockIdx.x * lpb, col = col0 + grp;
+  if (col < total) {
+    const int b = col / ncol, I = col - b * ncol, t = G.t;
+    const Pairs<NT> w(G.buf, M, t);
+    const double* m = mult ? mult + (int64_t)b * mstride + (int64_t)I * nrow : nullptr;
+    double u[PP], v[PP];
+    load_pairs<NT, PP, M_>(in + (int64_t)b * g.nG + (int64_t)I * nrow, M, t, u, v);
+    int q;
+    // (one copy of the transform's code: two would not fit the instruction cache)
+#pragma unroll 1
+    for (int pass = 0;; ++pass) {
+      const bool more = pass == 0 && m;
+      q = line_transform<NT, PP, M_>(G, ax, u, v, [&] {
+        if (more) load_pairs<NT, PP, M_>(m, M, t, u, v);
+      });
+      if (!more) break;
+      with_results<NT, PP, M_>(w, M, t, q, [&](int i, bool mid, double x, double y) {
+        u[i] *= x;
+        v[i] = mid ? 0.0 : v[i] * y;
+      });
     }
-#pragma unroll
-    for (int i = 0; i < PP; ++i) {
-      const bool mid = i == 0 && t == 0;
-      u[i] = v[i] = 0.0;
-      if (M_ == NT * PP || t + NT * i < M) {
-        u[i] = __longlong_as_double(*w.a(i, mid));
-        if (!mid) v[i] = __longlong_as_double(*w.b(i));
-      }
-    }
-    q = line_transform<NT, PP, M_>(G, ax, u, v);
-    scal = 1.0;
+    if (G.t == 0) sm.q[grp] = q - (q == kNotFinite ? 0 : log2scale);
   }
-  double* dst = out + off;
-#pragma unroll 4
-  for (int i = 0; i < PP; ++i) {
-    const bool mid = i == 0 && t == 0;
-    if (M_ == NT * PP || t + NT * i < M) {
-      const double x = to_double(*w.a(i, mid), q), y = to_double(*w.b(i), q);
-      dst[mid ? M - 1 : t + NT * i - 1] = mult ? x : x * scal;
-      if (!mid) dst[n - 1 - t - NT * i] = mult ? y : y * scal;
-    }
-  }
+  store_transposed<NT>(sm, M, col0, total, ncol, g.nG, out);
 }
 
-// transposed intermediate -> x transform -> rows: out = row, or out = sub_from - row
+// x transform of rows, in place where in == out: out = row, or out = sub_from - row
 template <int NT, int PP, int M_>
 __global__ void __launch_bounds__(Bounds<NT>::kThreads, Bounds<NT>::kBlocks)
-k_fx_inv(Geometry g, FxAxis ax, const double* __restrict__ in, double* out, int batch, const double* sub_from) {
+k_fx_inv(Geometry g, FxAxis ax, const double* in, double* out, int batch, const double* sub_from) {
   pdl_begin();
-  const int M = M_ ? M_ : ax.M, lpb = blockDim.x / NT, grp = threadIdx.x / NT;
+  constexpr int lpb = Bounds<NT>::kLines;
+  const int M = M_ ? M_ : ax.M, grp = threadIdx.x / NT;
   const Smem sm = carve<NT>(M, lpb, grp);
   const Group<NT> G{(int)threadIdx.x % NT, grp, sm.line, sm.red};
-  const int n = 2 * M, ncol = n - 1, nrow = g.ny - 1, total = batch * nrow;
-  const int row0 = blockIdx.x * lpb;
-  {
-    const int b0 = row0 / nrow, J0 = row0 - b0 * nrow, sh = 31 - __clz(lpb);
-    const int w = threadIdx.x & (lpb - 1);
-    if (row0 + w < total) {
-      const int wrap = J0 + w >= nrow;
-      double* buf = reinterpret_cast<double*>(sm.lines + (size_t)w * line_words(M));
-      const double* src = in + (int64_t)(b0 + wrap) * g.nG + (J0 + w - (wrap ? nrow : 0));
-#pragma unroll 16
-      for (int I = threadIdx.x >> sh; I < ncol; I += NT) buf[I + 1] = src[(int64_t)I * nrow];
-    }
-  }
-  __syncthreads();
-  const int row = row0 + grp, t = G.t;
-  if (row >= total) return;
-  double u[PP], v[PP];
-  load_pairs<NT, PP, M_>(reinterpret_cast<const double*>(G.buf) + 1, M, t, u, v);
-  const int q = line_transform<NT, PP, M_>(G, ax, u, v);
-  const Pairs<NT> w(G.buf, M, t);
+  const int ncol = 2 * M - 1, nrow = g.ny - 1, row = blockIdx.x * lpb + grp, t = G.t;
+  if (row >= batch * nrow) return;
   const int b = row / nrow, J = row - b * nrow;
   const int64_t off = (int64_t)b * g.nG + (int64_t)J * ncol;
-  double* dst = out + off;
-  const double* sf = sub_from ? sub_from + off : nullptr;
-#pragma unroll 4
-  for (int i = 0; i < PP; ++i) {
-    const bool mid = i == 0 && t == 0;
-    if (M_ == NT * PP || t + NT * i < M) {
-      const int p = mid ? M - 1 : t + NT * i - 1, r = n - 1 - t - NT * i;
-      const double x = to_double(*w.a(i, mid), q), y = to_double(*w.b(i), q);
-      dst[p] = sf ? sf[p] - x : x;
-      if (!mid) dst[r] = sf ? sf[r] - y : y;
+  double u[PP], v[PP];
+  load_pairs<NT, PP, M_>(in + off, M, t, u, v);
+  const int q = line_transform<NT, PP, M_>(G, ax, u, v, [&] {
+    if (sub_from) load_pairs<NT, PP, M_>(sub_from + off, M, t, u, v);
+  });
+  const Pairs<NT> w(G.buf, M, t);
+  double* lo = out + off - 1 + t;
+  double* hi = out + off + 2 * M - 1 - t;
+  with_results<NT, PP, M_>(w, M, t, q, [&](int i, bool mid, double x, double y) {
+    if (sub_from) {
+      x = u[i] - x;
+      y = v[i] - y;
     }
-  }
+    *(mid ? out + off + M - 1 : lo + NT * i) = x;
+    if (!mid) hi[-NT * i] = y;
+  });
 }
 
-// Threads per line, pairs per thread and compiled-in length, by M.  A line's group is the fewest warps
-// that hold it eight pairs a thread; lengths without a plan of their own take the runtime indexing.
+// Threads per line, pairs per thread and compiled-in length, by M; lengths without a plan of their own
+// take the runtime indexing.  Measured, a Poisson solve of one field: 512^2 with 64 threads a line and
+// four pairs each 23.1 us, 32 and eight 27.9; 768 x 512 with 64 and six (x) 30.8, 128 and three 34.5;
+// 1024^2 with 64 and eight 54.5, 128 and four 64.7; 2048^2 x 2 with two lines a block 396, four 424.
 #define IB_FX_SHAPE(M, CALL)                  \
   do {                                        \
     switch (M) {                              \
       case 64: { CALL(32, 2, 64); }           \
       case 96: { CALL(32, 3, 96); }           \
       case 128: { CALL(32, 4, 128); }         \
-      case 192: { CALL(32, 6, 192); }         \
-      case 256: { CALL(32, 8, 256); }         \
+      case 192: { CALL(64, 3, 192); }         \
+      case 256: { CALL(64, 4, 256); }         \
       case 384: { CALL(64, 6, 384); }         \
       case 512: { CALL(64, 8, 512); }         \
       case 768: { CALL(128, 6, 768); }        \
@@ -573,7 +636,7 @@ k_fx_inv(Geometry g, FxAxis ax, const double* __restrict__ in, double* out, int 
     }                                         \
     if ((M) <= 64) { CALL(32, 2, 0); }        \
     else if ((M) <= 128) { CALL(32, 4, 0); }  \
-    else if ((M) <= 256) { CALL(32, 8, 0); }  \
+    else if ((M) <= 256) { CALL(64, 4, 0); }  \
     else if ((M) <= 512) { CALL(64, 8, 0); }  \
     else { CALL(128, 8, 0); }                 \
   } while (0)
@@ -592,14 +655,13 @@ int fx_radices(int M, int* radix) {
   }
 }
 
-int lines_per_block(int M) { return M <= 256 ? 8 : 4; }
-
-template <typename K, typename... Args>
-cudaError_t launch(K k, int M, int nt, int lpb, int blocks, cudaStream_t s, Args... args) {
-  const size_t smem = smem_bytes(M, nt, lpb);
+template <int NT, typename K, typename... Args>
+cudaError_t launch(K k, int M, int lines, cudaStream_t s, Args... args) {
+  constexpr int lpb = Bounds<NT>::kLines;
+  const size_t smem = smem_bytes(M, NT, lpb);
   const cudaError_t e = set_smem_limit((const void*)k, smem);
   if (e != cudaSuccess) return e;
-  return launch_k(k, dim3(blocks), dim3(lpb * nt), smem, s, args...);
+  return launch_k(k, dim3((lines + lpb - 1) / lpb), dim3(lpb * NT), smem, s, args...);
 }
 
 }  // namespace
@@ -663,21 +725,19 @@ cudaError_t fx_fwd(const Geometry& g, const FxAxis& ax, const double* in, double
   if (ax.n != g.nx) return cudaErrorInvalidValue;
   if (batch <= 0) return cudaSuccess;
   ProfScope prof(kClassXPass, s);
-  const int lpb = lines_per_block(ax.M), blocks = (batch * (g.ny - 1) + lpb - 1) / lpb;
-#define IB_FX_CALL(NT, PP, ML)                                                             \
-  return launch(k_fx_fwd<NT, PP, ML>, ax.M, NT, lpb, blocks, s, g, ax, in, out, batch, bc, bcfac)
+#define IB_FX_CALL(NT, PP, ML) \
+  return launch<NT>(k_fx_fwd<NT, PP, ML>, ax.M, batch * (g.ny - 1), s, g, ax, in, out, batch, bc, bcfac)
   IB_FX_SHAPE(ax.M, IB_FX_CALL);
 #undef IB_FX_CALL
 }
 
 cudaError_t fx_ypass(const Geometry& g, const FxAxis& ay, const double* in, double* out, int batch, const double* mult,
-                     int64_t mstride, double scal, cudaStream_t s) {
+                     int64_t mstride, int log2scale, cudaStream_t s) {
   if (ay.n != g.ny) return cudaErrorInvalidValue;
   if (batch <= 0) return cudaSuccess;
   ProfScope prof(kClassYPass, s);
-  const int lpb = lines_per_block(ay.M), blocks = (batch * (g.nx - 1) + lpb - 1) / lpb;
-#define IB_FX_CALL(NT, PP, ML)                                                             \
-  return launch(k_fx_y<NT, PP, ML>, ay.M, NT, lpb, blocks, s, g, ay, in, out, batch, mult, mstride, scal)
+#define IB_FX_CALL(NT, PP, ML) \
+  return launch<NT>(k_fx_y<NT, PP, ML>, ay.M, batch * (g.nx - 1), s, g, ay, in, out, batch, mult, mstride, log2scale)
   IB_FX_SHAPE(ay.M, IB_FX_CALL);
 #undef IB_FX_CALL
 }
@@ -687,9 +747,8 @@ cudaError_t fx_inv(const Geometry& g, const FxAxis& ax, const double* in, double
   if (ax.n != g.nx) return cudaErrorInvalidValue;
   if (batch <= 0) return cudaSuccess;
   ProfScope prof(kClassXPass, s);
-  const int lpb = lines_per_block(ax.M), blocks = (batch * (g.ny - 1) + lpb - 1) / lpb;
-#define IB_FX_CALL(NT, PP, ML)                                                             \
-  return launch(k_fx_inv<NT, PP, ML>, ax.M, NT, lpb, blocks, s, g, ax, in, out, batch, sub_from)
+#define IB_FX_CALL(NT, PP, ML) \
+  return launch<NT>(k_fx_inv<NT, PP, ML>, ax.M, batch * (g.ny - 1), s, g, ax, in, out, batch, sub_from)
   IB_FX_SHAPE(ax.M, IB_FX_CALL);
 #undef IB_FX_CALL
 }

@@ -57,11 +57,16 @@ constexpr int kInBits = 55, kStageBits = 59, kPostBits = 60, kOutBits = 63;
 
 FX_HD i64 mad(int a, int b, i64 c) { return (i64)a * b + c; }
 
-// arithmetic shift right by d (warp-uniform), rounded to nearest even
+// arithmetic shift right by d < 31 (the same on every thread of a line), rounded to nearest even
 FX_HD i64 shr_rne(i64 v, int d) {
   if (d == 0) return v;
-  const i64 half = ((i64)1 << (d - 1)) - 1;
-  return (v + half + (int)((v >> d) & 1)) >> d;
+  v += ((1 << (d - 1)) - 1) + (int)((v >> d) & 1);
+#if defined(__CUDA_ARCH__)
+  const int hi = (int)(v >> 32);
+  return (i64)((u64)(unsigned)__funnelshift_r((unsigned)v, (unsigned)hi, d) | ((u64)(unsigned)(hi >> d) << 32));
+#else
+  return v >> d;
+#endif
 }
 FX_HD i64 half_rne(i64 v) { return (v + (int)((v >> 1) & 1)) >> 1; }
 

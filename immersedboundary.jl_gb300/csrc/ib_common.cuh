@@ -182,15 +182,16 @@ struct YPassArgs {
 template <typename T>
 cudaError_t ypass(const Geometry& g, const DstAxis<T>& ax, const YPassArgs<T>& a, cudaStream_t s);
 
-// The FP64 passes (dstfx.cu), arrays of nG doubles.  The intermediate of a solve is stored transposed,
-// column by column: element (I, J) of slot b at b*nG + I*(ny-1) + J.
-//   fx_fwd:   in [+ bcfac * apply_bc(bc) on the edges] -> x transform -> transposed store
-//   fx_ypass: per column S_y, times mult (per slot stride mstride), S_y; mult == nullptr: scal * S_y
-//   fx_inv:   transposed load -> x transform -> out, or out = sub_from - (.) (out may be sub_from)
+// The FP64 passes (dstfx.cu), arrays of nG doubles.
+//   fx_fwd:   in [+ bcfac * apply_bc(bc) on the edges] -> x transform -> out transposed, column by
+//             column (element (I, J) of slot b at b*nG + I*(ny-1) + J); out != in
+//   fx_ypass: per column S_y, times mult (per slot stride mstride, column-major), S_y (mult == nullptr:
+//             S_y only), times 2^log2scale -> out row-major; out != in
+//   fx_inv:   rows -> x transform -> out, or out = sub_from - (.) (out may be in or sub_from)
 cudaError_t fx_fwd(const Geometry& g, const FxAxis& ax, const double* in, double* out, int batch, const double* bc,
                    double bcfac, cudaStream_t s);
 cudaError_t fx_ypass(const Geometry& g, const FxAxis& ay, const double* in, double* out, int batch, const double* mult,
-                     int64_t mstride, double scal, cudaStream_t s);
+                     int64_t mstride, int log2scale, cudaStream_t s);
 cudaError_t fx_inv(const Geometry& g, const FxAxis& ax, const double* in, double* out, int batch,
                    const double* sub_from, cudaStream_t s);
 

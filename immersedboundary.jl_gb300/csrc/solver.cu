@@ -230,12 +230,15 @@ SolveOp op_cn1(const ib_handle* h) { return {h->mCN1, h->mCN1_32, 0, h->d_one, h
 
 // FP64 solve of `batch` arrays: out = F2D(m .* F2D(in [+ apply_bc(bc, 1)])), optional
 // subtract epilogue out = sub_from - (...).  w: FP64 work of batch arrays (the transposed
-// intermediate).
+// intermediate).  The row-major intermediate is in `out`, or, where that holds sub_from, in h->w2
+// (at most nlevels arrays).
 cudaError_t poisson64(ib_handle* h, const double* in, double* out, int batch, const double* bc, const SolveOp& op,
                       const double* sub_from, double* w) {
   CE(fx_fwd(h->g, h->axx.d, in, w, batch, bc, 1.0, h->stream));
-  CE(fx_ypass(h->g, h->axy.d, w, w, batch, op.m64, op.mstride, 1.0, h->stream));
-  return fx_inv(h->g, h->axx.d, w, out, batch, sub_from, h->stream);
+  double* t = sub_from == out ? h->w2 : out;
+  if (t != out && batch > h->g.nlev) return cudaErrorInvalidValue;
+  CE(fx_ypass(h->g, h->axy.d, w, t, batch, op.m64, op.mstride, 0, h->stream));
+  return fx_inv(h->g, h->axx.d, t, out, batch, sub_from, h->stream);
 }
 
 // Mixed-precision solve: FP32 sine transforms refined with float-float residuals.
@@ -2466,12 +2469,9 @@ int ib_op_dst2(ib_handle* h, int32_t batch, const double* in, double* out) {
   if (batch < 1) return IB_ERR_INVALID;
   double* w;
   CK(cudaMalloc(&w, sizeof(double) * batch * g.nG));
-  // RODFT00 in both dimensions = 4 F_y F_x (F: the half-scaled transform of dstfx.cu); the passes
-  // leave the result transposed ([I][J] per slot): transpose it back
+  // RODFT00 in both dimensions = 4 F_y F_x (F: the half-scaled transform of dstfx.cu)
   cudaError_t e = fx_fwd(g, h->axx.d, in, w, batch, nullptr, 1.0, s);
-  if (e == cudaSuccess) e = fx_ypass(g, h->axy.d, w, w, batch, nullptr, 0, 4.0, s);
-  for (int b = 0; b < batch && e == cudaSuccess; ++b)
-    e = transpose(w + (int64_t)b * g.nG, out + (int64_t)b * g.nG, g.nx - 1, g.ny - 1, s);
+  if (e == cudaSuccess) e = fx_ypass(g, h->axy.d, w, out, batch, nullptr, 0, 2, s);
   cudaStreamSynchronize(s);
   cudaFree(w);
   CK(e);
