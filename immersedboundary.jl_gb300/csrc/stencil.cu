@@ -175,128 +175,81 @@ __global__ void k_rot(Geometry g, const T* __restrict__ q, T* __restrict__ gam, 
 
 // ---- nonlinear term + explicit right-hand side (cnab/ops.jl:151-167, fluid-ops.jl:277-401,
 //      cnab/timestepping.jl:54-67) ----------------------------------------------------------
-template <typename T>
-struct LevelView {
-  const T* qx; const T* qy; const T* G; const T* bc;
-  T q0x, q0y;
-  int nx, ny, ncol;
-  // avg_flux!: Qx at (Jq in 1..ny-1, Iq in 0..nx), Qy at (Jq in 0..ny, Iq in 1..nx-1)
-  __device__ __forceinline__ T Qx(int Jq, int Iq) const {
-    return xscale((((qx[Jq * (nx + 1) + Iq] + qx[(Jq - 1) * (nx + 1) + Iq]) + q0x) + q0x), 0.5f);
-  }
-  __device__ __forceinline__ T Qy(int Jq, int Iq) const {
-    return xscale((((qy[Jq * nx + Iq] + qy[Jq * nx + Iq - 1]) + q0y) + q0y), 0.5f);
-  }
-  __device__ __forceinline__ T Gm(int J, int I) const { return G[J * ncol + I]; }
-};
-
-// fqx at (Jf, If), If in 1..nx-1 (direct_product_loops!, fluid-ops.jl:329-362)
-template <typename T>
-__device__ __forceinline__ T fqx_at(const Geometry& g, const LevelView<T>& v, int Jf, int If, T qyHi, T qyLo) {
-  if (Jf == 0) return xscale(qyHi * v.Gm(0, If - 1) + qyLo * v.bc[g.B + If], 0.5f);
-  if (Jf == v.ny - 1) return xscale(qyLo * v.Gm(v.ny - 2, If - 1) + qyHi * v.bc[g.T + If], 0.5f);
-  return xscale(qyHi * v.Gm(Jf, If - 1) + qyLo * v.Gm(Jf - 1, If - 1), 0.5f);
-}
-// fqy at (Jf, If), Jf in 1..ny-1 (fluid-ops.jl:365-398); qxHi = Qx(Jf, If+1), qxLo = Qx(Jf, If)
-template <typename T>
-__device__ __forceinline__ T fqy_at(const Geometry& g, const LevelView<T>& v, int Jf, int If, T qxHi, T qxLo) {
-  if (If == 0) return xscale(qxHi * v.Gm(Jf - 1, 0) + qxLo * v.bc[g.L + Jf], -0.5f);
-  if (If == v.nx - 1) return xscale(qxLo * v.Gm(Jf - 1, v.nx - 2) + qxHi * v.bc[g.R + Jf], -0.5f);
-  return xscale(qxHi * v.Gm(Jf - 1, If) + qxLo * v.Gm(Jf - 1, If - 1), -0.5f);
-}
-
 // Nonlinear term and CN right-hand side of every level (Nonlinear/RhsForce, timestepping.jl:
-// 31-66; avg_flux! fluid-ops.jl:276-301, direct_product! :303-398, rot!): one block per tile of
-// kNTY x kNTX cells.  The averaged fluxes (Qx, Qy) and the flux products (fqx, fqy) the tile's
-// cells share are formed once into shared memory, then each cell combines its four products;
-// every value is the same expression as a per-cell evaluation would form.
+// 31-66; avg_flux! fluid-ops.jl:276-301, direct_product! :303-398, rot!).  With Qx, Qy the fluxes
+// averaged to the nodes and G the circulation at the nodes (the ring on the boundary), the face
+// products are fqx(j) = (Qy G)(j+1) + (Qy G)(j) and -fqy(i) = (Qx G)(i+1) + (Qx G)(i), up to exact
+// factors; in rot the node's own products drop out, so that
+//   N(j, i) = ((Qy G)(j-1) - (Qy G)(j+1) + (Qx G)(i-1) - (Qx G)(i+1)) / (4 hc^2).
+// One block per tile of kNTY x kNTX cells: the products its cells share are formed once into shared
+// memory, then each cell combines its four.
+//
+// FP64 is bound by its pipe (18 operations a cell; one takes 6.9 us at 1024^2 x 4 levels), float-float
+// by instruction issue.  Measured there: FP64 325 us (averages, face products and combination, 30
+// operations a cell) -> 191 us, float-float 111 -> 94 us; 200^2 x 5 in
+// FP64 21.8 -> 14.4.  (4 rows a tile: 203 and 106; 16 rows: 189 and 100.)  A warp walking up its columns
+// with the products in registers has fewer operations but waits for each row's loads: 207 and 105.
 constexpr int kNTX = 32, kNTY = 8;
 template <typename T>
 __global__ void __launch_bounds__(kNTX * kNTY) k_nonlin_rhs(Geometry g, NonlinArgs<T> a) {
   pdl_begin();
-  __shared__ T sQy[kNTY + 2][kNTX];   // Qy(J0 + r, I0 + 1 + c)
-  __shared__ T sQx[kNTY][kNTX + 2];   // Qx(J0 + 1 + r, I0 + c)
-  __shared__ T sFx[kNTY + 1][kNTX];   // fqx(J0 + r, I0 + 1 + c)
-  __shared__ T sFy[kNTY][kNTX + 1];   // fqy(J0 + 1 + r, I0 + c)
-  __shared__ T sK[6];                 // the tile level's q0x, q0y, 1/hc^2, alpha; dt beta0, dt beta1
-  const int nx = g.nx, ny = g.ny, ncol = nx - 1, nrow = ny - 1;
-  const int ne = 2 * ncol + 2 * nrow;
-  const int tx = (ncol + kNTX - 1) / kNTX, ty = (nrow + kNTY - 1) / kNTY;
-  const int ntiles = g.nlev * tx * ty;
-  const int tid = threadIdx.x, cr = tid / kNTX, cc = tid % kNTX;
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int l = tile / (tx * ty), rem = tile - l * tx * ty;
-    const int J0 = (rem / tx) * kNTY, I0 = (rem % tx) * kNTX;
-    LevelView<T> v;
-    v.qx = a.q + (int64_t)l * g.nq;
-    v.qy = v.qx + g.nu;
-    v.G = a.gamma + (int64_t)l * g.nG;
-    v.bc = a.bcn + (int64_t)l * g.nbc;
-    // the level's constants, converted once per tile (a double-to-float-float conversion costs
-    // FP64 operations, which GB300 runs at 1/64 of its FP32 rate)
-    if (tid < 6) {
-      const double kv = tid == 0 ? a.q0[2 * l]
-                      : tid == 1 ? a.q0[2 * l + 1]
-                      : tid == 2 ? a.inv_hc2[l]
-                      : tid == 3 ? (a.alpha ? a.alpha[l] : 0.0)
-                      : tid == 4 ? a.dtb0 : a.dtb1;
-      sK[tid] = (T)kv;
-    }
-    __syncthreads();
-    v.q0x = sK[0];
-    v.q0y = sK[1];
-    v.nx = nx; v.ny = ny; v.ncol = ncol;
-    // averaged fluxes: Qy rows 0..ny, columns 1..nx-1; Qx rows 1..ny-1, columns 0..nx
-    for (int i = tid; i < (kNTY + 2) * kNTX; i += kNTX * kNTY) {
-      const int r = i / kNTX, c = i % kNTX, Jq = J0 + r, Iq = I0 + 1 + c;
-      if (Jq <= ny && Iq <= nx - 1) sQy[r][c] = v.Qy(Jq, Iq);
-    }
-    for (int i = tid; i < kNTY * (kNTX + 2); i += kNTX * kNTY) {
-      const int r = i / (kNTX + 2), c = i % (kNTX + 2), Jq = J0 + 1 + r, Iq = I0 + c;
-      if (Jq <= ny - 1 && Iq <= nx) sQx[r][c] = v.Qx(Jq, Iq);
-    }
-    __syncthreads();
-    // flux products: fqx rows 0..ny-1, columns 1..nx-1; fqy rows 1..ny-1, columns 0..nx-1
-    for (int i = tid; i < (kNTY + 1) * kNTX; i += kNTX * kNTY) {
-      const int r = i / kNTX, c = i % kNTX, Jf = J0 + r, If = I0 + 1 + c;
-      if (Jf <= ny - 1 && If <= nx - 1) sFx[r][c] = fqx_at(g, v, Jf, If, sQy[r + 1][c], sQy[r][c]);
-    }
-    for (int i = tid; i < kNTY * (kNTX + 1); i += kNTX * kNTY) {
-      const int r = i / (kNTX + 1), c = i % (kNTX + 1), Jf = J0 + 1 + r, If = I0 + c;
-      if (Jf <= ny - 1 && If <= nx - 1) sFy[r][c] = fqy_at(g, v, Jf, If, sQx[r][c + 1], sQx[r][c]);
-    }
-    __syncthreads();
-    const int J = J0 + cr, I = I0 + cc;
-    if (J < nrow && I < ncol) {
-      const int64_t t = (int64_t)l * g.nG + (int64_t)J * ncol + I;
-      const T fx_lo = sFx[cr][cc];       // fqx[J,   I+1]
-      const T fx_hi = sFx[cr + 1][cc];   // fqx[J+1, I+1]
-      const T fy_r = sFy[cr][cc + 1];    // fqy[J+1, I+1]
-      const T fy_l = sFy[cr][cc];        // fqy[J+1, I]
-      const T nl = ((fx_lo - fx_hi) + (fy_r - fy_l)) * sK[2];
-      a.nl_new[t] = nl;
-      T r = sK[4] * nl;
-      r = r + sK[5] * a.nl_old[t];
-      if (a.alpha) {
-        // A_l gamma = gamma - alpha_l (4 gamma - neighbours), zero outside the array
-        const T gc = v.Gm(J, I);
-        T lap = xscale(gc, 4.0f);
-        if (I > 0) lap -= v.Gm(J, I - 1);
-        if (I < ncol - 1) lap -= v.Gm(J, I + 1);
-        if (J > 0) lap -= v.Gm(J - 1, I);
-        if (J < nrow - 1) lap -= v.Gm(J + 1, I);
-        r = (gc - sK[3] * lap) + r;
-      }
-      const T* ed = a.edges + (int64_t)l * ne;
-      T edge = T(0);
-      if (J == 0) edge += ed[I];
-      if (J == nrow - 1) edge += ed[ncol + I];
-      if (I == 0) edge += ed[2 * ncol + J];
-      if (I == ncol - 1) edge += ed[2 * ncol + nrow + J];
-      a.rhs[t] = r + edge;
-    }
-    __syncthreads();
+  __shared__ T sM[kNTY + 2][kNTX];  // 2 Qy G at nodes (J0 + r, I0 + 1 + c)
+  __shared__ T sN[kNTY][kNTX + 2];  // 2 Qx G at nodes (J0 + 1 + r, I0 + c)
+  __shared__ T sK[6];               // the level's 2 q0x, 2 q0y, 1/(4 hc^2), alpha; dt beta0, dt beta1
+  const int nx = g.nx, ny = g.ny, ncol = nx - 1, nrow = ny - 1, l = blockIdx.z;
+  const int J0 = blockIdx.y * kNTY, I0 = blockIdx.x * kNTX, tid = threadIdx.x;
+  const T* __restrict__ qx = a.q + (int64_t)l * g.nq;
+  const T* __restrict__ qy = qx + g.nu;
+  const T* __restrict__ G = a.gamma + (int64_t)l * g.nG;
+  const T* __restrict__ bc = a.bcn + (int64_t)l * g.nbc;
+  // the level's constants, converted once per block (a double-to-float-float conversion costs
+  // FP64 operations, which GB300 runs at 1/64 of its FP32 rate)
+  if (tid < 6) {
+    sK[tid] = (T)(tid == 0 ? 2.0 * a.q0[2 * l]
+                : tid == 1 ? 2.0 * a.q0[2 * l + 1]
+                : tid == 2 ? 0.25 * a.inv_hc2[l]
+                : tid == 3 ? (a.alpha ? a.alpha[l] : 0.0)
+                : tid == 4 ? a.dtb0 : a.dtb1);
   }
+  __syncthreads();
+  // circulation at node (j, i) next to the interior, the ring on the boundary
+  auto node = [&](int j, int i) -> T {
+    if (j == 0) return bc[g.B + i];
+    if (j == ny) return bc[g.T + i];
+    if (i == 0) return bc[g.L + j];
+    if (i == nx) return bc[g.R + j];
+    return G[(j - 1) * ncol + i - 1];
+  };
+  for (int k = tid; k < (kNTY + 2) * kNTX; k += kNTX * kNTY) {
+    const int r = k / kNTX, c = k % kNTX, j = J0 + r, i = I0 + 1 + c;
+    if (j <= ny && i <= nx - 1) sM[r][c] = ((qy[j * nx + i] + qy[j * nx + i - 1]) + sK[1]) * node(j, i);
+  }
+  for (int k = tid; k < kNTY * (kNTX + 2); k += kNTX * kNTY) {
+    const int r = k / (kNTX + 2), c = k % (kNTX + 2), j = J0 + 1 + r, i = I0 + c;
+    if (j <= ny - 1 && i <= nx) sN[r][c] = ((qx[j * (nx + 1) + i] + qx[(j - 1) * (nx + 1) + i]) + sK[0]) * node(j, i);
+  }
+  __syncthreads();
+  const int cr = tid / kNTX, cc = tid % kNTX, J = J0 + cr, I = I0 + cc;
+  if (J >= nrow || I >= ncol) return;
+  const int64_t t = (int64_t)l * g.nG + (int64_t)J * ncol + I;
+  const T nl = ((sM[cr][cc] - sM[cr + 2][cc]) + (sN[cr][cc] - sN[cr][cc + 2])) * sK[2];
+  a.nl_new[t] = nl;
+  T r = sK[4] * nl + sK[5] * a.nl_old[t];
+  if (a.alpha) {
+    // A_l gamma = gamma - alpha_l (4 gamma - neighbours), zero outside the array
+    const T* p = G + J * ncol + I;
+    const T gc = *p;
+    const T gl = I > 0 ? p[-1] : T(0), gr = I < ncol - 1 ? p[1] : T(0);
+    const T gd = J > 0 ? p[-ncol] : T(0), gu = J < nrow - 1 ? p[ncol] : T(0);
+    const T lap = xscale(gc, 4.0f) - ((gl + gr) + (gd + gu));
+    r = (gc - sK[3] * lap) + r;
+  }
+  const T* ed = a.edges + (int64_t)l * (2 * ncol + 2 * nrow);
+  if (J == 0) r += ed[I];
+  if (J == nrow - 1) r += ed[ncol + I];
+  if (I == 0) r += ed[2 * ncol + J];
+  if (I == ncol - 1) r += ed[2 * ncol + nrow + J];
+  a.rhs[t] = r;
 }
 
 // Rings of the trial step (cnab/timestepping.jl:42-57): bcn[l] = 0.25 * get_bc(gamma[l+1]) for
@@ -401,8 +354,8 @@ cudaError_t rot(const Geometry& g, const T* q, T* gam, int batch, cudaStream_t s
 template <typename T>
 cudaError_t nonlin_rhs(const Geometry& g, const NonlinArgs<T>& a, cudaStream_t s) {
   ProfScope prof(kClassNonlin, s);
-  const int tiles = g.nlev * ((g.nx - 1 + kNTX - 1) / kNTX) * ((g.ny - 1 + kNTY - 1) / kNTY);
-  return launch_k(k_nonlin_rhs<T>, dim3(tiles < 65535 * 8 ? tiles : 65535 * 8), dim3(kNTX * kNTY), 0, s, g, a);
+  const dim3 grid((g.nx - 1 + kNTX - 1) / kNTX, (g.ny - 1 + kNTY - 1) / kNTY, g.nlev);
+  return launch_k(k_nonlin_rhs<T>, grid, dim3(kNTX * kNTY), 0, s, g, a);
 }
 template <typename T>
 cudaError_t trial_rings(const Geometry& g, const T* gamma, T* bcn, T* edges, const double* fac, cudaStream_t s,
