@@ -324,6 +324,25 @@ cudaError_t ensure_smem(const void* fn, size_t bytes) {
   return e;
 }
 
+// Radix plan of an M-point FFT: powers of two first (8s, then a 4/4, 4 or 2 remainder), then 3s,
+// then 5s, so the leading stages have power-of-two strides (k = j & (Ns-1)).
+int plan_radices(int M, int* radix) {
+  int m = M, ns = 0, p2 = 0, n3 = 0, n5 = 0;
+  while (m % 5 == 0) { ++n5; m /= 5; }
+  while (m % 3 == 0) { ++n3; m /= 3; }
+  while (m % 2 == 0) { ++p2; m /= 2; }
+  if (m != 1) return -1;
+  int a = p2 / 3, rem = p2 % 3;
+  if (rem == 1 && a >= 1) { a -= 1; radix[ns++] = 4; radix[ns++] = 4; }
+  else if (rem == 1) { radix[ns++] = 2; }
+  else if (rem == 2) { radix[ns++] = 4; }
+  for (int i = 0; i < a; ++i) radix[ns++] = 8;
+  for (int i = 0; i < n3; ++i) radix[ns++] = 3;
+  for (int i = 0; i < n5; ++i) radix[ns++] = 5;
+  if (ns > kMaxStages) return -1;
+  return ns;
+}
+
 template <typename T, typename Tin, typename Tout, int PRO, int EPI, bool kBC>
 cudaError_t launch_x1(const Geometry& g, const DstAxis<T>& ax, const XArgs& a, cudaStream_t s) {
   const int total = a.batch * (g.ny - 1);
@@ -372,25 +391,6 @@ cudaError_t launch_y(const Geometry& g, const DstAxis<T>& ax, const YPassArgs<T>
 }
 
 }  // namespace
-
-// Radix plan of an M-point FFT: powers of two first (8s, then a 4/4, 4 or 2 remainder), then 3s,
-// then 5s, so the leading stages have power-of-two strides (k = j & (Ns-1)).
-int plan_radices(int M, int* radix) {
-  int m = M, ns = 0, p2 = 0, n3 = 0, n5 = 0;
-  while (m % 5 == 0) { ++n5; m /= 5; }
-  while (m % 3 == 0) { ++n3; m /= 3; }
-  while (m % 2 == 0) { ++p2; m /= 2; }
-  if (m != 1) return -1;
-  int a = p2 / 3, rem = p2 % 3;
-  if (rem == 1 && a >= 1) { a -= 1; radix[ns++] = 4; radix[ns++] = 4; }
-  else if (rem == 1) { radix[ns++] = 2; }
-  else if (rem == 2) { radix[ns++] = 4; }
-  for (int i = 0; i < a; ++i) radix[ns++] = 8;
-  for (int i = 0; i < n3; ++i) radix[ns++] = 3;
-  for (int i = 0; i < n5; ++i) radix[ns++] = 5;
-  if (ns > kMaxStages) return -1;
-  return ns;
-}
 
 cudaError_t set_smem_limit(const void* fn, size_t bytes) { return ensure_smem(fn, bytes); }
 

@@ -1,0 +1,643 @@
+// The kernels of the FP64 sine-transform passes (launched by dstfx.cu): every line is transformed in 64-bit block fixed point (fx.cuh).
+//
+// Replaces, like dst.cu, the FFTW RODFT00 plan + `LaplacianInv` call of the reference
+// (src/streamfcn/fluid-ops.jl:19-56) and the CN multipliers of `A_Ainv_linearmaps`
+// (src/streamfcn/cnab/ops.jl:14-42).  The algorithm of a line is dst.cu's (fold, half-length complex
+// FFT, split of the real transform, prefix sum of the differences); its values are integers.
+//
+// A group of NT threads (32, 64 or 128, by the axis length: M = n/2 <= PP NT) owns a line:
+//   1. each thread loads the pairs (y_j, y_{n-j}) of j = t + NT i straight into registers, the group
+//      finds the line's largest exponent and turns the pairs into folded integers in shared memory
+//   2. Stockham stages of radix 8, 4, 2, 3, 5: read, group barrier, shift + twiddle + DFT in
+//      registers, write in place; the bits the results occupy (one OR per value) give the next
+//      stage's shift.  Complex values are padded one slot in eight
+//   3. split into even outputs and differences D_k; the odd outputs are D's exact prefix sums
+//   4. doubles leave by their bits (leading-zero count, round, pack)
+// A line with an infinity or NaN becomes NaN throughout, as the FP64 transform made it.  Sums of
+// integers do not depend on their order, so results are the same bits for any NT.
+//
+// A pass reads its lines as they lie in memory and stores them transposed (the forward x pass, the y
+// pass), so that the next pass's lines lie in memory: 32 or 64 bytes at a time, written without
+// waiting, where a transposing load would stall the block.
+//
+// What bounds it: the integer pipes and the latency between them (ncu, 1024-cell lines: ALU 59% and
+// FMA-heavy 46% busy, 2.5 of 4 instructions issued per clock), and the latency of a line's chain where
+// a launch has few lines.  Measured against the FP64-arithmetic passes (shared-memory Stockham, one
+// warp per line at 2048 cells), which the FP64 pipe's two lanes per SM bound: a 2048^2 Poisson solve
+// of two fields 2.09 -> 0.53 ms, a 1024^2 x 4-level two-body step 3.75 -> 1.16 ms, 384 x 256 x 4 RKC
+// 0.88 -> 0.40, 200^2 x 5 0.81 -> 0.39, 128^2 x 3 0.53 -> 0.28, with a quarter of their error on the
+// 2048^2 solve (4.3e-15 against 1.8e-14).
+#pragma once
+
+#include "fx.cuh"
+#include "ib_common.cuh"
+
+namespace ib {
+
+namespace fxp {
+
+using fx::cpx;
+using fx::cwgt;
+using fx::i64;
+using fx::u64;
+using fx::wgt;
+
+constexpr unsigned kAll = 0xffffffffu;
+constexpr int kRedSlots = 2 + kMaxStages;  // reductions of one transform: largest, sum, one per stage
+
+// padded index of a complex value / of a result: one spare slot after every 8
+__host__ __device__ constexpr int cpad(int i) { return i + (i >> 3); }
+
+// The results F_i, i = 1..n-1, of a line lie at word cpad(i / 2) of two regions of its buffer, the
+// odd ones in the first, the even ones in the second, 8 banks (of 8 bytes) away from the first.
+__host__ __device__ constexpr int even_off(int M) { return (M + (M >> 3) + 6 + 7) / 16 * 16 + 8; }
+// 8-byte words of one line's buffer: M complex values padded, or both regions; congruent to 2 mod 16,
+// so that four lines' words at two successive indices of either parity lie in different banks
+__host__ __device__ constexpr int line_words(int M) { return (even_off(M) + cpad(M) + 14) / 16 * 16 + 2; }
+
+// Every accepted length is compiled in (M = n / 2: even, with factors 2, 3 and 5, at most 1024), so
+// that index arithmetic is constant: a 200^2 solve 22.8 -> 19.6 us, 600 x 400 38.4 -> 29.1.
+//
+// Threads of a line's group: the fewest warps that hold it eight pairs a thread at most, and two from
+// M = 129 on, where a launch still lasts as long as a line's chain.  Measured, a Poisson solve of one
+// field: 512^2 with 64 threads a line and four pairs each 23.1 us, 32 and eight 27.9; 768 x 512 with 64
+// and six (x) 30.8, 128 and three 34.5; 1024^2 with 64 and eight 54.5, 128 and four 64.7.
+constexpr int group_threads(int M) { return M <= 128 ? 32 : M <= 512 ? 64 : 128; }
+constexpr int pairs(int M) { return (M + group_threads(M) - 1) / group_threads(M); }
+
+// Radices of the FFT of M points: eights where many values lie in a thread's registers (M >= 384), fours
+// where lines are short; a left-over 2 makes a six with a 3, or an eight.
+struct Radices {
+  int n, r[kMaxStages];
+};
+constexpr Radices radices(int M) {
+  Radices p{};
+  int twos = 0, threes = 0, fives = 0, eights = 0, fours = 0, sixes = 0;
+  const bool large = M >= 384;
+  for (; M % 2 == 0; M /= 2) ++twos;
+  for (; M % 3 == 0; M /= 3) ++threes;
+  for (; M % 5 == 0; M /= 5) ++fives;
+  const int over = large ? twos % 3 : twos % 2;  // large: twos left over by eights; else by fours
+  if (over == 1 && threes > 0) {
+    sixes = 1;
+    --twos;
+    --threes;
+  }
+  if (large) {
+    while (twos % 3 != 0 && twos >= 2) {
+      ++fours;
+      twos -= 2;
+    }
+  } else if (twos % 2 != 0 && twos >= 3) {
+    eights = 1;
+    twos -= 3;
+  }
+  if (large) {
+    eights = twos / 3;
+    twos %= 3;
+  } else {
+    fours = twos / 2;
+    twos %= 2;
+  }
+  for (int i = 0; i < eights; ++i) p.r[p.n++] = 8;
+  for (int i = 0; i < fours; ++i) p.r[p.n++] = 4;
+  for (int i = 0; i < sixes; ++i) p.r[p.n++] = 6;
+  for (int i = 0; i < twos; ++i) p.r[p.n++] = 2;
+  for (int i = 0; i < threes; ++i) p.r[p.n++] = 3;
+  for (int i = 0; i < fives; ++i) p.r[p.n++] = 5;
+  return p;
+}
+
+// barrier of a line's group of threads
+template <int NT>
+__device__ __forceinline__ void group_bar(int id) {
+  if (NT == 32) __syncwarp();
+  else asm volatile("bar.sync %0, %1;" ::"r"(id + 1), "r"(NT) : "memory");
+}
+
+template <int NT>
+struct Group {
+  int t;          // thread in the group
+  int id;         // group in the block (barrier id + 1)
+  i64* buf;       // the line's buffer
+  unsigned* red;  // [kRedSlots][NT / 32]
+
+  __device__ __forceinline__ void bar() const { group_bar<NT>(id); }
+  __device__ __forceinline__ void put(int slot, unsigned v) const {  // v: warp-reduced already
+    if (NT > 32 && (t & 31) == 0) red[slot * (NT / 32) + (t >> 5)] = v;
+  }
+  template <class Op>
+  __device__ __forceinline__ unsigned get(int slot, unsigned v, Op op) const {
+    if (NT == 32) return v;
+    unsigned m = red[slot * (NT / 32)];
+#pragma unroll
+    for (int w = 1; w < NT / 32; ++w) m = op(m, red[slot * (NT / 32) + w]);
+    return m;
+  }
+};
+
+__device__ __forceinline__ unsigned occupied(i64 v) {
+  const int h = (int)(v >> 32);
+  return (unsigned)(h ^ (h >> 31));
+}
+
+// One Stockham stage of radix R, in place, by the threads of a group; NS: product of the radices before.
+// The first stage (NS = 1) reads the folded line in its natural layout.  Returns the OR of the bits
+// this thread's results occupy.
+template <int M, int R, int NS>
+__device__ __forceinline__ unsigned stage(const Group<group_threads(M)>& G, const FxAxis& ax, int st, int d) {
+  constexpr int NT = group_threads(M), nb = M / R, NB = (nb + NT - 1) / NT;  // butterflies in all, per thread
+  constexpr bool kFull = nb % NT == 0;
+  const int t = G.t;
+  cpx* z = reinterpret_cast<cpx*>(G.buf);
+  cpx v[NB][R];
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    const int j = t + NT * b;
+    if (!kFull) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[b][r] = {0, 0};  // (a predicated load alone would keep the old value live)
+    }
+    if (kFull || j < nb) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        if (NS == 1) v[b][r] = z[j + r * nb];
+        else if (nb % 8 == 0) v[b][r] = z[cpad(t) + b * (NT + NT / 8) + r * (nb + nb / 8)];
+        else v[b][r] = z[cpad(j + r * nb)];
+      }
+    }
+  }
+  G.bar();
+  unsigned o = 0;
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    const int j = t + NT * b;
+    if (kFull || j < nb) {
+      const int k = j % NS;
+      if (NS > 1) {
+        if (d > 0) {
+#pragma unroll
+          for (int r = 0; r < R; ++r) v[b][r] = {fx::shr_rne(v[b][r].x, d), fx::shr_rne(v[b][r].y, d)};
+        }
+        const cwgt* tw = ax.tw + ax.twoff[st] + k;
+#pragma unroll
+        for (int r = 1; r < R; ++r) {
+          const int4 w = __ldg(reinterpret_cast<const int4*>(tw + (r - 1) * NS));
+          v[b][r] = fx::cmul(v[b][r], {w.x, w.y, w.z, w.w});
+        }
+      }
+      fx::Dft<R>::run(v[b]);
+      const int base = (j - k) * R + k;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        o |= occupied(v[b][r].x) | occupied(v[b][r].y);
+        if (NS % 8 == 0 || (NS == 1 && R == 8)) z[cpad(base) + (NS == 1 ? r : r * (NS + NS / 8))] = v[b][r];
+        else z[cpad(base + r * NS)] = v[b][r];
+      }
+    }
+  }
+  return o;
+}
+
+// Shift the values now need (bits from the OR of occupied()) to fit `limit` bits.
+__device__ __forceinline__ int excess(unsigned o, int limit) { return max(0, 64 - __clz((int)o) - limit); }
+
+// The stages ST.. of the transform; T: the shifts so far, o: the bits the values occupy.
+template <int M, int ST, int NS>
+__device__ __forceinline__ void stages(const Group<group_threads(M)>& G, const FxAxis& ax, int& T, unsigned& o) {
+  constexpr Radices p = radices(M);
+  if constexpr (ST < p.n) {
+    constexpr int R = p.r[ST];
+    const int d = ST > 0 ? excess(o, fx::kStageBits) : 0;
+    T += d;
+    o = __reduce_or_sync(kAll, stage<M, R, NS>(G, ax, ST, d));
+    G.put(2 + ST, o);
+    G.bar();
+    o = G.get(2 + ST, o, [](unsigned a, unsigned b) { return a | b; });
+    stages<M, ST + 1, NS * R>(G, ax, T, o);
+  }
+}
+
+__device__ __forceinline__ i64* result_at(i64* buf, int M, int i) {
+  return buf + ((i & 1) ? 0 : even_off(M)) + cpad(i >> 1);
+}
+// The words of a thread's pairs (j, n - j), j = t + NT i: at lo + i kStride and hi - i kStride (the
+// pair j = 0 stands for the middle value, j = n / 2, alone).
+template <int M>
+struct Pairs {
+  static constexpr int NT = group_threads(M), kStride = NT / 2 + NT / 16;
+  i64 *lo, *hi, *mid;
+  __device__ __forceinline__ Pairs(i64* buf, int t) {
+    lo = buf + ((t & 1) ? 0 : even_off(M)) + cpad(t >> 1);
+    hi = buf + ((t & 1) ? 0 : even_off(M)) + cpad(M - ((t + 1) >> 1));
+    mid = result_at(buf, M, M);
+  }
+  __device__ __forceinline__ i64* a(int i, bool middle) const { return middle ? mid : lo + i * kStride; }
+  __device__ __forceinline__ i64* b(int i) const { return hi - i * kStride; }
+};
+
+// exponent of a line whose values are not finite
+constexpr int kNotFinite = 1 << 20;
+
+// the double of a result on a safe scale q
+__device__ __forceinline__ double to_double(i64 v, int q) {
+  return __longlong_as_double((i64)fx::from_fixed(v, q));
+}
+// not finite, or at the ends of the exponent range (subnormal results, or overflow)
+static __device__ __noinline__ double to_double_slow(i64 v, int q) {
+  if (q == kNotFinite) return __longlong_as_double(0x7ff8000000000000ll);
+  return ldexp((double)v, -q);
+}
+// DST-I of a line given as pairs a[i] = y_j, b[i] = y_{n-j}, j = t + NT i (j = 0: a = y_{n/2}, b
+// unused); the results are in place after the closing barrier.  Returns their scale q
+// (F = value 2^-q), the same on every thread of the group.  `before_scan` runs before the last
+// phase, with few registers in use: a place for loads that are needed next.
+template <int M, class Hook>
+__device__ __forceinline__ int line_transform(const Group<group_threads(M)>& G, const FxAxis& ax,
+                                              const double (&a)[pairs(M)], const double (&b)[pairs(M)],
+                                              Hook before_scan) {
+  constexpr int NT = group_threads(M), PP = pairs(M), n = 2 * M;
+  constexpr bool kEven = M == NT * PP;  // every thread has PP pairs
+  const int t = G.t;
+  // 1. the line's largest exponent
+  unsigned m = 0;
+#pragma unroll
+  for (int i = 0; i < PP; ++i) {
+    m = max(m, fx::mag_hi((u64)__double_as_longlong(a[i])));
+    m = max(m, fx::mag_hi((u64)__double_as_longlong(b[i])));
+  }
+  m = __reduce_max_sync(kAll, m);
+  G.put(0, m);
+  G.bar();
+  m = G.get(0, m, [](unsigned x, unsigned y) { return max(x, y); });
+  if (m >= 0x7ff00000u) {
+    G.bar();
+    return kNotFinite;
+  }
+  const int ex = max(1, (int)(m >> 20));
+  // 2. integers, folded
+  unsigned asum = 0;
+#pragma unroll
+  for (int i = 0; i < PP; ++i) {
+    const int j = t + NT * i;
+    if (kEven || j < M) {
+      const i64 va = fx::to_fixed((u64)__double_as_longlong(a[i]), ex);
+      const i64 vb = fx::to_fixed((u64)__double_as_longlong(b[i]), ex);
+      // upper bound of |va| + |vb| in units of 2^35
+      asum += ((unsigned)((int)(va >> 32) ^ (int)(va >> 63)) >> 3) + ((unsigned)((int)(vb >> 32) ^ (int)(vb >> 63)) >> 3) + 2u;
+      const int2 w = __ldg(reinterpret_cast<const int2*>(ax.sin2 + j));
+      const i64 p = fx::mul(va + vb, {w.x, w.y}), df = va - vb;
+      if (i == 0 && t == 0) {
+        G.buf[0] = 0;
+        G.buf[M] = 4 * va;
+      } else {
+        G.buf[j] = p + df;
+        G.buf[n - j] = p - df;
+      }
+    }
+  }
+  asum = __reduce_add_sync(kAll, asum);
+  G.put(1, asum);
+  G.bar();
+  asum = G.get(1, asum, [](unsigned x, unsigned y) { return x + y; });
+  // 3. FFT of length M
+  int T = 0;
+  unsigned o = 0;
+  stages<M, 0, 1>(G, ax, T, o);
+  // 4. split: even outputs and differences, at four times their value
+  const int abits = 37 + 32 - __clz((int)(asum - 1u));  // 4 sum |y| <= 2^abits
+  const int d = max(excess(o, fx::kPostBits), abits - fx::kOutBits - T);
+  T += d;
+  {
+    constexpr int hM = M / 2, PQ = (hM + NT - 1) / NT;
+    constexpr bool kAllK = hM == NT * PQ;  // exactly PQ values of k per thread
+    const cpx* z = reinterpret_cast<const cpx*>(G.buf);
+    cpx zk[PQ], zm[PQ];
+#pragma unroll
+    for (int i = 0; i < PQ; ++i) {
+      const int k = t + NT * i;
+      if (!kAllK) zk[i] = zm[i] = {0, 0};
+      if (kAllK || k < hM) {
+        zk[i] = z[cpad(t) + i * (NT + NT / 8)];
+        zm[i] = z[i == 0 && t == 0 ? cpad(hM) : cpad(M - t) - i * (NT + NT / 8)];
+      }
+    }
+    G.bar();
+    i64* D = G.buf;
+    i64* E = G.buf + even_off(M);
+#pragma unroll
+    for (int i = 0; i < PQ; ++i) {
+      const int k = t + NT * i;
+      if (kAllK || k < hM) {
+        if (d > 0) {
+          zk[i] = {fx::shr_rne(zk[i].x, d), fx::shr_rne(zk[i].y, d)};
+          zm[i] = {fx::shr_rne(zm[i].x, d), fx::shr_rne(zm[i].y, d)};
+        }
+        if (i == 0 && t == 0) {
+          D[0] = zk[i].x + zk[i].y;
+          D[cpad(hM)] = 2 * zm[i].x;
+          E[cpad(hM)] = 2 * zm[i].y;
+        } else {
+          const int4 w = __ldg(reinterpret_cast<const int4*>(ax.post + k));
+          const i64 er = zk[i].x + zm[i].x, ei = zk[i].y - zm[i].y;
+          const cpx r = fx::cmul({zk[i].y + zm[i].y, zm[i].x - zk[i].x}, {w.x, w.y, w.z, w.w});
+          const int pk = cpad(t) + i * (NT + NT / 8), pm = cpad(M - t) - i * (NT + NT / 8);
+          D[pk] = er + r.x;
+          D[pm] = er - r.x;
+          E[pk] = -(ei + r.y);
+          E[pm] = ei - r.y;
+        }
+      }
+    }
+  }
+  G.bar();
+  before_scan();
+  // 5. odd outputs: prefix sums of D, chunk by chunk
+  {
+    const int k0 = t * PP;
+    i64 s[PP], acc = 0;
+#pragma unroll
+    for (int i = 0; i < PP; ++i) {
+      if (kEven || k0 + i < M) acc += G.buf[8 % PP == 0 ? cpad(k0) + i : cpad(k0 + i)];
+      s[i] = acc;
+    }
+    i64 incl = acc;
+#pragma unroll
+    for (int w = 1; w < 32; w <<= 1) {
+      const i64 v = __shfl_up_sync(kAll, incl, w);
+      if ((t & 31) >= w) incl += v;
+    }
+    i64 excl = incl - acc;
+    if (NT > 32) {
+      // totals of the warps before this one (spare words after the padded differences)
+      i64* tot = G.buf + M + (M >> 3) + 2;
+      if ((t & 31) == 31) tot[t >> 5] = incl;
+      G.bar();
+#pragma unroll
+      for (int w = 0; w < NT / 32 - 1; ++w)
+        if ((t >> 5) > w) excl += tot[w];
+    }
+#pragma unroll
+    for (int i = 0; i < PP; ++i)
+      if (kEven || k0 + i < M) G.buf[8 % PP == 0 ? cpad(k0) + i : cpad(k0 + i)] = s[i] + excl;
+  }
+  G.bar();
+  return fx::kInBits + 1022 - ex - T + 2;
+}
+
+// ------------------------------------------------------------------------------------------------
+// passes
+// ------------------------------------------------------------------------------------------------
+// Lines per block: 4 (stores of 32-byte segments), or 2 of the longest.  Two blocks of 256 threads per
+// SM or four of 128 leave 128 registers a thread; capping at 80 or 64 for more warps costs more in
+// spills than it hides (1024^2 solve of one field: 54.5 us, 57.7, 62.2).
+template <int M>
+struct Bounds {
+  static constexpr int NT = group_threads(M);
+  static constexpr int kLines = NT == 128 ? 2 : 4;
+  static constexpr int kThreads = kLines * NT;
+  static constexpr int kBlocks = 512 / kThreads;
+};
+
+struct Smem {
+  i64* line;      // this group's line buffer
+  i64* lines;     // line buffer of group 0
+  unsigned* red;  // this group's reduction slots
+  int* q;         // [lines per block] scales
+};
+template <int M>
+constexpr size_t smem_bytes() {
+  return (size_t)Bounds<M>::kLines * (line_words(M) * 8 + kRedSlots * (group_threads(M) / 32) * 4 + 4) + 16;
+}
+template <int M>
+__device__ __forceinline__ Smem carve(int grp) {
+  constexpr int NT = group_threads(M), lpb = Bounds<M>::kLines;
+  extern __shared__ __align__(16) unsigned char fx_smem[];
+  Smem s;
+  s.lines = reinterpret_cast<i64*>(fx_smem);
+  s.line = s.lines + (size_t)grp * line_words(M);
+  unsigned* red = reinterpret_cast<unsigned*>(s.lines + (size_t)lpb * line_words(M));
+  s.red = red + grp * (kRedSlots * (NT / 32));
+  s.q = reinterpret_cast<int*>(red + lpb * (kRedSlots * (NT / 32)));
+  return s;
+}
+
+// pairs of a line that lies contiguously in memory
+template <int M>
+__device__ __forceinline__ void load_pairs(const double* src, int t, double (&u)[pairs(M)], double (&v)[pairs(M)]) {
+  constexpr int NT = group_threads(M), PP = pairs(M);
+  const double* lo = src - 1 + t;
+  const double* hi = src + 2 * M - 1 - t;
+#pragma unroll
+  for (int i = 0; i < PP; ++i) {
+    const bool mid = i == 0 && t == 0;
+    u[i] = v[i] = 0.0;
+    if (M == NT * PP || t + NT * i < M) {
+      u[i] = *(mid ? src + M - 1 : lo + NT * i);
+      if (!mid) v[i] = hi[-NT * i];
+    }
+  }
+}
+
+// f(i, middle, F_j, F_{n-j}) for the thread's pairs (of the middle pair only the first value)
+template <int M, class F>
+__device__ __forceinline__ void with_results(const Pairs<M>& w, int t, int q, F f) {
+  constexpr int NT = group_threads(M), PP = pairs(M);
+  if (fx::safe_scale(q)) {
+#pragma unroll
+    for (int i = 0; i < PP; ++i)
+      if (M == NT * PP || t + NT * i < M) {
+        const bool mid = i == 0 && t == 0;
+        f(i, mid, to_double(*w.a(i, mid), q), to_double(*w.b(i), q));
+      }
+  } else {
+#pragma unroll
+    for (int i = 0; i < PP; ++i)
+      if (M == NT * PP || t + NT * i < M) {
+        const bool mid = i == 0 && t == 0;
+        f(i, mid, to_double_slow(*w.a(i, mid), q), to_double_slow(*w.b(i), q));
+      }
+  }
+}
+
+// The results of the block's lines line0 .. line0 + lpb - 1 (of `total`, `per` lines to an array of
+// `stride` values), transposed: the block's lines at one index are adjacent in memory.
+template <int M>
+__device__ __forceinline__ void store_transposed(const Smem& sm, int line0, int total, int per, int64_t stride,
+                                                 double* out) {
+  constexpr int NT = group_threads(M), lpb = Bounds<M>::kLines;
+  __syncthreads();
+  const int b0 = line0 / per, J0 = line0 - b0 * per, w = threadIdx.x % lpb;
+  if (line0 + w >= total) return;
+  const int wrap = J0 + w >= per;
+  i64* buf = sm.lines + (size_t)w * line_words(M);
+  const int q = sm.q[w];
+  double* dst = out + (int64_t)(b0 + wrap) * stride + (J0 + w - (wrap ? per : 0));
+  if (fx::safe_scale(q)) {
+#pragma unroll 8
+    for (int I = threadIdx.x / lpb; I < 2 * M - 1; I += NT)
+      dst[(int64_t)I * per] = to_double(*result_at(buf, M, I + 1), q);
+  } else {
+#pragma unroll 1
+    for (int I = threadIdx.x / lpb; I < 2 * M - 1; I += NT)
+      dst[(int64_t)I * per] = to_double_slow(*result_at(buf, M, I + 1), q);
+  }
+}
+
+// x transform of rows as they lie in memory -> transposed intermediate; optional apply_bc(bc) on the
+// edges (fluid-ops.jl:249-275)
+template <int M>
+__global__ void __launch_bounds__(Bounds<M>::kThreads, Bounds<M>::kBlocks)
+k_fx_fwd(Geometry g, FxAxis ax, const double* __restrict__ in, double* __restrict__ out, int batch,
+         const double* __restrict__ bc, double bcfac) {
+  pdl_begin();
+  constexpr int NT = group_threads(M), PP = pairs(M), lpb = Bounds<M>::kLines;
+  const int grp = threadIdx.x / NT;
+  const Smem sm = carve<M>(grp);
+  const Group<NT> G{(int)threadIdx.x % NT, grp, sm.line, sm.red};
+  const int ncol = 2 * M - 1, nrow = g.ny - 1, total = batch * nrow;
+  const int row0 = blockIdx.x * lpb, row = row0 + grp;
+  if (row < total) {
+    const int b = row / nrow, J = row - b * nrow;
+    const double* src = in + (int64_t)b * g.nG + (int64_t)J * ncol;
+    double u[PP], v[PP];
+    load_pairs<M>(src, G.t, u, v);
+    if (bc) {
+      const double* r = bc + (int64_t)b * g.nbc;
+      if (J == 0 || J == nrow - 1) {
+        double e[PP], f[PP];
+        load_pairs<M>(r + (J == 0 ? g.B : g.T) + 1, G.t, e, f);
+#pragma unroll
+        for (int i = 0; i < PP; ++i) {
+          u[i] += bcfac * e[i];
+          v[i] += bcfac * f[i];
+        }
+      }
+      if (G.t == 1) {  // the pair of the row's first and last value
+        u[0] += bcfac * r[g.L + 1 + J];
+        v[0] += bcfac * r[g.R + 1 + J];
+      }
+    }
+    const int q = line_transform<M>(G, ax, u, v, [] {});
+    if (G.t == 0) sm.q[grp] = q;
+  }
+  store_transposed<M>(sm, row0, total, nrow, g.nG, out);
+}
+
+// y pass: columns of the transposed intermediate, S_y, times m, S_y (or S_y only), times 2^log2scale,
+// stored row-major
+template <int M>
+__global__ void __launch_bounds__(Bounds<M>::kThreads, Bounds<M>::kBlocks)
+k_fx_y(Geometry g, FxAxis ax, const double* __restrict__ in, double* __restrict__ out, int batch,
+       const double* mult, int64_t mstride, int log2scale) {
+  pdl_begin();
+  constexpr int NT = group_threads(M), PP = pairs(M), lpb = Bounds<M>::kLines;
+  const int grp = threadIdx.x / NT;
+  const Smem sm = carve<M>(grp);
+  const Group<NT> G{(int)threadIdx.x % NT, grp, sm.line, sm.red};
+  const int ncol = g.nx - 1, nrow = 2 * M - 1, total = batch * ncol;
+  const int col0 = blockIdx.x * lpb, col = col0 + grp;
+  if (col < total) {
+    const int b = col / ncol, I = col - b * ncol, t = G.t;
+    const Pairs<M> w(G.buf, t);
+    const double* m = mult ? mult + (int64_t)b * mstride + (int64_t)I * nrow : nullptr;
+    double u[PP], v[PP];
+    load_pairs<M>(in + (int64_t)b * g.nG + (int64_t)I * nrow, t, u, v);
+    int q;
+    // (one copy of the transform's code: two would not fit the instruction cache)
+#pragma unroll 1
+    for (int pass = 0;; ++pass) {
+      const bool more = pass == 0 && m;
+      q = line_transform<M>(G, ax, u, v, [&] {
+        if (more) load_pairs<M>(m, t, u, v);
+      });
+      if (!more) break;
+      with_results<M>(w, t, q, [&](int i, bool mid, double x, double y) {
+        u[i] *= x;
+        v[i] = mid ? 0.0 : v[i] * y;
+      });
+    }
+    if (G.t == 0) sm.q[grp] = q - (q == kNotFinite ? 0 : log2scale);
+  }
+  store_transposed<M>(sm, col0, total, ncol, g.nG, out);
+}
+
+// x transform of rows, in place where in == out: out = row, or out = sub_from - row
+template <int M>
+__global__ void __launch_bounds__(Bounds<M>::kThreads, Bounds<M>::kBlocks)
+k_fx_inv(Geometry g, FxAxis ax, const double* in, double* out, int batch, const double* sub_from) {
+  pdl_begin();
+  constexpr int NT = group_threads(M), PP = pairs(M), lpb = Bounds<M>::kLines;
+  const int grp = threadIdx.x / NT;
+  const Smem sm = carve<M>(grp);
+  const Group<NT> G{(int)threadIdx.x % NT, grp, sm.line, sm.red};
+  const int ncol = 2 * M - 1, nrow = g.ny - 1, row = blockIdx.x * lpb + grp, t = G.t;
+  if (row >= batch * nrow) return;
+  const int b = row / nrow, J = row - b * nrow;
+  const int64_t off = (int64_t)b * g.nG + (int64_t)J * ncol;
+  double u[PP], v[PP];
+  load_pairs<M>(in + off, t, u, v);
+  const int q = line_transform<M>(G, ax, u, v, [&] {
+    if (sub_from) load_pairs<M>(sub_from + off, t, u, v);
+  });
+  const Pairs<M> w(G.buf, t);
+  double* lo = out + off - 1 + t;
+  double* hi = out + off + 2 * M - 1 - t;
+  with_results<M>(w, t, q, [&](int i, bool mid, double x, double y) {
+    if (sub_from) {
+      x = u[i] - x;
+      y = v[i] - y;
+    }
+    *(mid ? out + off + M - 1 : lo + NT * i) = x;
+    if (!mid) hi[-NT * i] = y;
+  });
+}
+
+template <int M, typename K, typename... Args>
+cudaError_t launch(K k, int lines, cudaStream_t s, Args... args) {
+  const cudaError_t e = set_smem_limit((const void*)k, smem_bytes<M>());
+  if (e != cudaSuccess) return e;
+  return launch_k(k, dim3((lines + Bounds<M>::kLines - 1) / Bounds<M>::kLines), dim3(Bounds<M>::kThreads),
+                  smem_bytes<M>(), s, args...);
+}
+
+// the passes of one length (dstfx.cu has the entry points)
+template <int M>
+cudaError_t run_fwd(const Geometry& g, const FxAxis& ax, const double* in, double* out, int batch, const double* bc,
+                    double bcfac, cudaStream_t s) {
+  return launch<M>(k_fx_fwd<M>, batch * (g.ny - 1), s, g, ax, in, out, batch, bc, bcfac);
+}
+template <int M>
+cudaError_t run_y(const Geometry& g, const FxAxis& ay, const double* in, double* out, int batch, const double* mult,
+                  int64_t mstride, int log2scale, cudaStream_t s) {
+  return launch<M>(k_fx_y<M>, batch * (g.nx - 1), s, g, ay, in, out, batch, mult, mstride, log2scale);
+}
+template <int M>
+cudaError_t run_inv(const Geometry& g, const FxAxis& ax, const double* in, double* out, int batch,
+                    const double* sub_from, cudaStream_t s) {
+  return launch<M>(k_fx_inv<M>, batch * (g.ny - 1), s, g, ax, in, out, batch, sub_from);
+}
+
+#define IB_FX_RUN(PREFIX, M)                                                                                        \
+  PREFIX template cudaError_t run_fwd<M>(const Geometry&, const FxAxis&, const double*, double*, int, const double*, \
+                                         double, cudaStream_t);                                                     \
+  PREFIX template cudaError_t run_y<M>(const Geometry&, const FxAxis&, const double*, double*, int, const double*,   \
+                                       int64_t, int, cudaStream_t);                                                 \
+  PREFIX template cudaError_t run_inv<M>(const Geometry&, const FxAxis&, const double*, double*, int, const double*, \
+                                         cudaStream_t);
+
+// the accepted lengths, by the translation unit that compiles their kernels
+#define IB_FX_GROUP_1(X) X(4) X(24) X(60) X(108) X(180) X(288) X(450) X(640) X(900)
+#define IB_FX_GROUP_2(X) X(6) X(30) X(64) X(120) X(192) X(300) X(480) X(648) X(960)
+#define IB_FX_GROUP_3(X) X(8) X(32) X(72) X(128) X(200) X(320) X(486) X(720) X(972)
+#define IB_FX_GROUP_4(X) X(10) X(36) X(80) X(144) X(216) X(324) X(500) X(750) X(1000)
+#define IB_FX_GROUP_5(X) X(12) X(40) X(90) X(150) X(240) X(360) X(512) X(768) X(1024)
+#define IB_FX_GROUP_6(X) X(16) X(48) X(96) X(160) X(250) X(384) X(540) X(800)
+#define IB_FX_GROUP_7(X) X(18) X(50) X(100) X(162) X(256) X(400) X(576) X(810)
+#define IB_FX_GROUP_8(X) X(20) X(54) X(270) X(432) X(600) X(864)
+#define IB_FX_LENGTHS(X)                                                                              \
+  IB_FX_GROUP_1(X) IB_FX_GROUP_2(X) IB_FX_GROUP_3(X) IB_FX_GROUP_4(X) IB_FX_GROUP_5(X) IB_FX_GROUP_6(X) \
+  IB_FX_GROUP_7(X) IB_FX_GROUP_8(X)
+
+}  // namespace fxp
+}  // namespace ib

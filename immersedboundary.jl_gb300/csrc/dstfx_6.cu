@@ -1,0 +1,7 @@
+// The FP64 passes of every eighth length (kernels in dstfx.cuh).
+#include "dstfx.cuh"
+
+namespace ib::fxp {
+#define IB_FX_HERE(M) IB_FX_RUN(, M)
+IB_FX_GROUP_6(IB_FX_HERE)
+}  // namespace ib::fxp

@@ -106,11 +106,9 @@ template <typename T> struct AxisTables {
 // Tables of one axis for the FP64 passes (dstfx.cu), factors in the fixed-point form of fx.cuh.
 namespace fx { struct cwgt; struct wgt; }
 struct FxAxis {
-  int n, M, nstages;
-  int radix[kMaxStages];
-  int ns[kMaxStages];          // product of the radices before the stage
-  unsigned magic[kMaxStages];  // ceil(2^32 / ns): j / ns = umulhi(j, magic)
-  int twoff[kMaxStages];       // stage's twiddles in tw: [r - 1][k], r < radix, k < ns
+  int n, M;
+  int twoff[kMaxStages];       // stage's twiddles in tw: [r - 1][k], r < radix, k < ns (ns: product of the
+                               //   radices before it)
   const fx::cwgt* tw;          // e^{-2 pi i r k / (ns radix)}
   const fx::cwgt* post;        // [M/2+1] e^{-2 pi i k / n}
   const fx::wgt* sin2;         // [M] 2 sin(pi j / n)
@@ -123,8 +121,6 @@ struct FxTables {
 };
 
 bool dst_axis_supported(int n);
-// radix plan of an M-point FFT (number of stages, or -1): 4s and 8s, then 3s, then 5s
-int plan_radices(int M, int* radix);
 // both axes have warp-per-line tables: the solves use the dstw passes (transposed intermediate)
 bool wdst_axis_supported(int n);
 

@@ -1,6 +1,5 @@
 """The FP64 sine transforms (64-bit block fixed point, csrc/dstfx.cu) against scipy's RODFT00 in
-extended precision: every compiled-in axis length, lengths of the general radices, and the ends of
-the exponent range."""
+extended precision: every accepted axis length, and the ends of the exponent range."""
 import numpy as np
 import pytest
 from scipy import fft as sfft
@@ -9,10 +8,13 @@ from _util import Dev
 
 pytestmark = pytest.mark.gpu
 
-# compiled-in lengths 64 P cells (P = 2^k or 3 2^k) at both ends of their range, and lengths whose
-# half has factors 2, 3 and 5 in every stage position, at the edges of the thread-group sizes
-SHAPES = [(8, 12), (20, 16), (40, 60), (128, 100), (200, 192), (256, 300), (360, 384), (512, 400), (600, 768),
-          (1000, 1024), (1536, 1080), (2048, 1920), (96, 2048), (1024, 64), (500, 72)]
+# every length has kernels of its own: each is an axis here, beside one of 8 or 12 cells, and a few pairs
+# of long axes
+LENGTHS = [n for n in range(8, 2049, 4) if not [1 for p in (7, 11, 13, 17, 19, 23, 29, 31, 37, 41, 43, 47)
+                                                if n % p == 0]
+           and max(q for q in range(1, n + 1) if n % q == 0 and all(q % p for p in (2, 3, 5))) == 1]
+SHAPES = [(n, 8 if k % 2 else 12) for k, n in enumerate(LENGTHS)] + [(12 if k % 2 else 8, n) for k, n in enumerate(LENGTHS)]
+SHAPES += [(200, 192), (600, 400), (1000, 1024), (768, 2048)]
 
 
 @pytest.fixture(scope="module")
