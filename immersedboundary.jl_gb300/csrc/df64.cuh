@@ -11,7 +11,7 @@
 
 namespace ib {
 
-struct df64 {
+struct alignas(8) df64 {  // (one 8-byte load or store)
   float hi, lo;
 
   df64() = default;
