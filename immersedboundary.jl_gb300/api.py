@@ -413,10 +413,9 @@ class Solver:
 
     ``precision``: ``"fp64"`` (the reference's arithmetic; the sine transforms in 64-bit block
     fixed point, whose rounding error is below FP64's),
-    ``"mixed"`` (FP32 sine transforms refined with float-float residuals, ``refine_sweeps`` sweeps per
-    Poisson solve: 1 or 2 everywhere, or 0 = the library default of 2 with 1 for the Vort2Flux
-    solves of the third and coarser levels; state, stencils and the nonlinear term in float-float
-    arithmetic; Schur solve and forces FP64), or ``"mixed_tc"`` (the same solve with every sine
+    ``"mixed"`` (state, stencils and the nonlinear term in float-float arithmetic, the solves by the
+    same 64-bit fixed-point transforms; Schur solve and forces FP64.  ``refine_sweeps=1``: FP32 sine
+    transforms refined by one float-float residual sweep per solve instead), or ``"mixed_tc"`` (FP32 solves refined with float-float residuals, every sine
     transform a BF16x3 split-precision GEMM against the sine matrix on the tensor cores; both
     axes a multiple of 128 cells).
     """
@@ -582,10 +581,10 @@ class Solver:
         self._check(self.lib.ib_set_cg_preconditioner(self.handle, m, int(refresh_steps)))
 
     def set_vort2flux_order(self, order: str = "auto"):
-        """Mixed precision: ``"levels"`` (every level's boundary ring first, then all levels in
-        one batch), ``"sequential"`` (the reference's coarse-to-fine order) or ``"auto"`` (levels
-        up to 2^20 cells per level where the grid allows it).  FP64 solvers keep the reference
-        order."""
+        """``"levels"`` (every level's boundary ring first, then all levels in one batch),
+        ``"sequential"`` (the reference's coarse-to-fine order; in mixed precision with refined FP32
+        transforms) or ``"auto"`` (levels from four levels on, and with three up to 2^17 cells per
+        level)."""
         m = {"auto": _lib.IB_V2F_AUTO, "levels": _lib.IB_V2F_LEVELS, "sequential": _lib.IB_V2F_SEQUENTIAL}[order]
         self._check(self.lib.ib_set_vort2flux_order(self.handle, m))
 

@@ -64,14 +64,15 @@ void FxTables::release() {
   mem = nullptr;
 }
 
-cudaError_t fx_fwd(const Geometry& g, const FxAxis& ax, const double* in, double* out, int batch, const double* bc,
-                   double bcfac, cudaStream_t s) {
+template <typename T>
+cudaError_t fx_fwd(const Geometry& g, const FxAxis& ax, const T* in, double* out, int batch, const T* bc,
+                   cudaStream_t s) {
   if (ax.n != g.nx) return cudaErrorInvalidValue;
   if (batch <= 0) return cudaSuccess;
   ProfScope prof(kClassXPass, s);
   switch (ax.M) {
 #define IB_FX_CASE(M) \
-  case M: return fxp::run_fwd<M>(g, ax, in, out, batch, bc, bcfac, s);
+  case M: return fxp::run_fwd<M, T>(g, ax, in, out, batch, bc, s);
     IB_FX_LENGTHS(IB_FX_CASE)
 #undef IB_FX_CASE
     default: return cudaErrorInvalidValue;
@@ -92,18 +93,52 @@ cudaError_t fx_ypass(const Geometry& g, const FxAxis& ay, const double* in, doub
   }
 }
 
-cudaError_t fx_inv(const Geometry& g, const FxAxis& ax, const double* in, double* out, int batch,
-                   const double* sub_from, cudaStream_t s) {
-  if (ax.n != g.nx) return cudaErrorInvalidValue;
+cudaError_t fx_yspec(const Geometry& g, const FxAxis& ay, double* w, int batch, const double* mult, double* qrow,
+                     int64_t qls, cudaStream_t s) {
+  if (ay.n != g.ny) return cudaErrorInvalidValue;
   if (batch <= 0) return cudaSuccess;
-  ProfScope prof(kClassXPass, s);
-  switch (ax.M) {
+  ProfScope prof(kClassYPass, s);
+  switch (ay.M) {
 #define IB_FX_CASE(M) \
-  case M: return fxp::run_inv<M>(g, ax, in, out, batch, sub_from, s);
+  case M: return fxp::run_yspec<M>(g, ay, w, batch, mult, qrow, qls, s);
     IB_FX_LENGTHS(IB_FX_CASE)
 #undef IB_FX_CASE
     default: return cudaErrorInvalidValue;
   }
 }
+
+cudaError_t fx_yring(const Geometry& g, const FxAxis& ay, const double* w, double* out, int batch, const double* mult,
+                     const FxRings& r, cudaStream_t s) {
+  if (ay.n != g.ny) return cudaErrorInvalidValue;
+  if (batch <= 0) return cudaSuccess;
+  ProfScope prof(kClassYPass, s);
+  switch (ay.M) {
+#define IB_FX_CASE(M) \
+  case M: return fxp::run_yring<M>(g, ay, w, out, batch, mult, r, s);
+    IB_FX_LENGTHS(IB_FX_CASE)
+#undef IB_FX_CASE
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+template <typename T>
+cudaError_t fx_inv(const Geometry& g, const FxAxis& ax, const double* in, T* out, int batch, const T* sub_from,
+                   cudaStream_t s) {
+  if (ax.n != g.nx) return cudaErrorInvalidValue;
+  if (batch <= 0) return cudaSuccess;
+  ProfScope prof(kClassXPass, s);
+  switch (ax.M) {
+#define IB_FX_CASE(M) \
+  case M: return fxp::run_inv<M, T>(g, ax, in, out, batch, sub_from, s);
+    IB_FX_LENGTHS(IB_FX_CASE)
+#undef IB_FX_CASE
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+template cudaError_t fx_fwd<double>(const Geometry&, const FxAxis&, const double*, double*, int, const double*, cudaStream_t);
+template cudaError_t fx_fwd<df64>(const Geometry&, const FxAxis&, const df64*, double*, int, const df64*, cudaStream_t);
+template cudaError_t fx_inv<double>(const Geometry&, const FxAxis&, const double*, double*, int, const double*, cudaStream_t);
+template cudaError_t fx_inv<df64>(const Geometry&, const FxAxis&, const double*, df64*, int, const df64*, cudaStream_t);
 
 }  // namespace ib

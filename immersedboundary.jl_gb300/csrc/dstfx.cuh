@@ -243,19 +243,46 @@ constexpr int kNotFinite = 1 << 20;
 __device__ __forceinline__ double to_double(i64 v, int q) {
   return __longlong_as_double((i64)fx::from_fixed(v, q));
 }
+__device__ __forceinline__ df64 to_pair(i64 v, int q) {
+  const fx::pair_float p = fx::from_fixed_pair(v, q);
+  // r 2^e in two factors where the power alone is below the float range
+  const int e = 127 + p.e, k = e < 1 ? 100 : 0;
+  float lo = __int2float_rn(p.r) * __uint_as_float((unsigned)max(e + k, 0) << 23);
+  if (k) lo *= 0x1p-100f;
+  return df64(__uint_as_float(p.hi), lo);
+}
 // not finite, or at the ends of the exponent range (subnormal results, or overflow)
 static __device__ __noinline__ double to_double_slow(i64 v, int q) {
   if (q == kNotFinite) return __longlong_as_double(0x7ff8000000000000ll);
   return ldexp((double)v, -q);
 }
+// What a line's values are: doubles, or float-float pairs (the state of the mixed-precision path).
+template <typename T> struct Value;
+template <> struct Value<double> {
+  static constexpr unsigned kBad = 0x7ff00000u;          // magnitude of an infinity or NaN
+  static constexpr int kExpBit = 20, kScale = fx::kInBits + 1022;
+  static __device__ __forceinline__ unsigned mag(double x) { return fx::mag_hi((u64)__double_as_longlong(x)); }
+  static __device__ __forceinline__ i64 fixed(double x, int ex) { return fx::to_fixed((u64)__double_as_longlong(x), ex); }
+};
+template <> struct Value<df64> {
+  static constexpr unsigned kBad = 0x7f800000u;
+  static constexpr int kExpBit = 23, kScale = fx::kInBits + 126;
+  static __device__ __forceinline__ unsigned mag(df64 x) {
+    return max(__float_as_uint(x.hi) & 0x7fffffffu, __float_as_uint(x.lo) & 0x7fffffffu);
+  }
+  static __device__ __forceinline__ i64 fixed(df64 x, int ex) {
+    return fx::to_fixed_float(__float_as_uint(x.hi), ex) + fx::to_fixed_float(__float_as_uint(x.lo), ex);
+  }
+};
+
 // DST-I of a line given as pairs a[i] = y_j, b[i] = y_{n-j}, j = t + NT i (j = 0: a = y_{n/2}, b
 // unused); the results are in place after the closing barrier.  Returns their scale q
 // (F = value 2^-q), the same on every thread of the group.  `before_scan` runs before the last
 // phase, with few registers in use: a place for loads that are needed next.
-template <int M, class Hook>
+template <int M, typename T, class Hook>
 __device__ __forceinline__ int line_transform(const Group<group_threads(M)>& G, const FxAxis& ax,
-                                              const double (&a)[pairs(M)], const double (&b)[pairs(M)],
-                                              Hook before_scan) {
+                                              const T (&a)[pairs(M)], const T (&b)[pairs(M)], Hook before_scan) {
+  using V = Value<T>;
   constexpr int NT = group_threads(M), PP = pairs(M), n = 2 * M;
   constexpr bool kEven = M == NT * PP;  // every thread has PP pairs
   const int t = G.t;
@@ -263,26 +290,24 @@ __device__ __forceinline__ int line_transform(const Group<group_threads(M)>& G, 
   unsigned m = 0;
 #pragma unroll
   for (int i = 0; i < PP; ++i) {
-    m = max(m, fx::mag_hi((u64)__double_as_longlong(a[i])));
-    m = max(m, fx::mag_hi((u64)__double_as_longlong(b[i])));
+    m = max(m, max(V::mag(a[i]), V::mag(b[i])));
   }
   m = __reduce_max_sync(kAll, m);
   G.put(0, m);
   G.bar();
   m = G.get(0, m, [](unsigned x, unsigned y) { return max(x, y); });
-  if (m >= 0x7ff00000u) {
+  if (m >= V::kBad) {
     G.bar();
     return kNotFinite;
   }
-  const int ex = max(1, (int)(m >> 20));
+  const int ex = max(1, (int)(m >> V::kExpBit));
   // 2. integers, folded
   unsigned asum = 0;
 #pragma unroll
   for (int i = 0; i < PP; ++i) {
     const int j = t + NT * i;
     if (kEven || j < M) {
-      const i64 va = fx::to_fixed((u64)__double_as_longlong(a[i]), ex);
-      const i64 vb = fx::to_fixed((u64)__double_as_longlong(b[i]), ex);
+      const i64 va = V::fixed(a[i], ex), vb = V::fixed(b[i], ex);
       // upper bound of |va| + |vb| in units of 2^35
       asum += ((unsigned)((int)(va >> 32) ^ (int)(va >> 63)) >> 3) + ((unsigned)((int)(vb >> 32) ^ (int)(vb >> 63)) >> 3) + 2u;
       const int2 w = __ldg(reinterpret_cast<const int2*>(ax.sin2 + j));
@@ -301,13 +326,13 @@ __device__ __forceinline__ int line_transform(const Group<group_threads(M)>& G, 
   G.bar();
   asum = G.get(1, asum, [](unsigned x, unsigned y) { return x + y; });
   // 3. FFT of length M
-  int T = 0;
+  int shifts = 0;
   unsigned o = 0;
-  stages<M, 0, 1>(G, ax, T, o);
+  stages<M, 0, 1>(G, ax, shifts, o);
   // 4. split: even outputs and differences, at four times their value
   const int abits = 37 + 32 - __clz((int)(asum - 1u));  // 4 sum |y| <= 2^abits
-  const int d = max(excess(o, fx::kPostBits), abits - fx::kOutBits - T);
-  T += d;
+  const int d = max(excess(o, fx::kPostBits), abits - fx::kOutBits - shifts);
+  shifts += d;
   {
     constexpr int hM = M / 2, PQ = (hM + NT - 1) / NT;
     constexpr bool kAllK = hM == NT * PQ;  // exactly PQ values of k per thread
@@ -382,7 +407,7 @@ __device__ __forceinline__ int line_transform(const Group<group_threads(M)>& G, 
       if (kEven || k0 + i < M) G.buf[8 % PP == 0 ? cpad(k0) + i : cpad(k0 + i)] = s[i] + excl;
   }
   G.bar();
-  return fx::kInBits + 1022 - ex - T + 2;
+  return V::kScale - ex - shifts + 2;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -423,15 +448,15 @@ __device__ __forceinline__ Smem carve(int grp) {
 }
 
 // pairs of a line that lies contiguously in memory
-template <int M>
-__device__ __forceinline__ void load_pairs(const double* src, int t, double (&u)[pairs(M)], double (&v)[pairs(M)]) {
+template <int M, typename T>
+__device__ __forceinline__ void load_pairs(const T* src, int t, T (&u)[pairs(M)], T (&v)[pairs(M)]) {
   constexpr int NT = group_threads(M), PP = pairs(M);
-  const double* lo = src - 1 + t;
-  const double* hi = src + 2 * M - 1 - t;
+  const T* lo = src - 1 + t;
+  const T* hi = src + 2 * M - 1 - t;
 #pragma unroll
   for (int i = 0; i < PP; ++i) {
     const bool mid = i == 0 && t == 0;
-    u[i] = v[i] = 0.0;
+    u[i] = v[i] = T(0.0f);
     if (M == NT * PP || t + NT * i < M) {
       u[i] = *(mid ? src + M - 1 : lo + NT * i);
       if (!mid) v[i] = hi[-NT * i];
@@ -440,10 +465,19 @@ __device__ __forceinline__ void load_pairs(const double* src, int t, double (&u)
 }
 
 // f(i, middle, F_j, F_{n-j}) for the thread's pairs (of the middle pair only the first value)
-template <int M, class F>
+template <int M, typename T, class F>
 __device__ __forceinline__ void with_results(const Pairs<M>& w, int t, int q, F f) {
   constexpr int NT = group_threads(M), PP = pairs(M);
-  if (fx::safe_scale(q)) {
+  if constexpr (is_df64<T>::value) {
+    const bool bad = q == kNotFinite;
+    const df64 nan = df64(__uint_as_float(0x7fc00000u), __uint_as_float(0x7fc00000u));
+#pragma unroll
+    for (int i = 0; i < PP; ++i)
+      if (M == NT * PP || t + NT * i < M) {
+        const bool mid = i == 0 && t == 0;
+        f(i, mid, bad ? nan : to_pair(*w.a(i, mid), q), bad ? nan : to_pair(*w.b(i), q));
+      }
+  } else if (fx::safe_scale(q)) {
 #pragma unroll
     for (int i = 0; i < PP; ++i)
       if (M == NT * PP || t + NT * i < M) {
@@ -486,10 +520,10 @@ __device__ __forceinline__ void store_transposed(const Smem& sm, int line0, int 
 
 // x transform of rows as they lie in memory -> transposed intermediate; optional apply_bc(bc) on the
 // edges (fluid-ops.jl:249-275)
-template <int M>
+template <int M, typename T>
 __global__ void __launch_bounds__(Bounds<M>::kThreads, Bounds<M>::kBlocks)
-k_fx_fwd(Geometry g, FxAxis ax, const double* __restrict__ in, double* __restrict__ out, int batch,
-         const double* __restrict__ bc, double bcfac) {
+k_fx_fwd(Geometry g, FxAxis ax, const T* __restrict__ in, double* __restrict__ out, int batch,
+         const T* __restrict__ bc) {
   pdl_begin();
   constexpr int NT = group_threads(M), PP = pairs(M), lpb = Bounds<M>::kLines;
   const int grp = threadIdx.x / NT;
@@ -499,23 +533,22 @@ k_fx_fwd(Geometry g, FxAxis ax, const double* __restrict__ in, double* __restric
   const int row0 = blockIdx.x * lpb, row = row0 + grp;
   if (row < total) {
     const int b = row / nrow, J = row - b * nrow;
-    const double* src = in + (int64_t)b * g.nG + (int64_t)J * ncol;
-    double u[PP], v[PP];
-    load_pairs<M>(src, G.t, u, v);
+    T u[PP], v[PP];
+    load_pairs<M>(in + (int64_t)b * g.nG + (int64_t)J * ncol, G.t, u, v);
     if (bc) {
-      const double* r = bc + (int64_t)b * g.nbc;
+      const T* r = bc + (int64_t)b * g.nbc;
       if (J == 0 || J == nrow - 1) {
-        double e[PP], f[PP];
+        T e[PP], f[PP];
         load_pairs<M>(r + (J == 0 ? g.B : g.T) + 1, G.t, e, f);
 #pragma unroll
         for (int i = 0; i < PP; ++i) {
-          u[i] += bcfac * e[i];
-          v[i] += bcfac * f[i];
+          u[i] += e[i];
+          v[i] += f[i];
         }
       }
       if (G.t == 1) {  // the pair of the row's first and last value
-        u[0] += bcfac * r[g.L + 1 + J];
-        v[0] += bcfac * r[g.R + 1 + J];
+        u[0] += r[g.L + 1 + J];
+        v[0] += r[g.R + 1 + J];
       }
     }
     const int q = line_transform<M>(G, ax, u, v, [] {});
@@ -552,7 +585,7 @@ k_fx_y(Geometry g, FxAxis ax, const double* __restrict__ in, double* __restrict_
         if (more) load_pairs<M>(m, t, u, v);
       });
       if (!more) break;
-      with_results<M>(w, t, q, [&](int i, bool mid, double x, double y) {
+      with_results<M, double>(w, t, q, [&](int i, bool mid, double x, double y) {
         u[i] *= x;
         v[i] = mid ? 0.0 : v[i] * y;
       });
@@ -562,10 +595,131 @@ k_fx_y(Geometry g, FxAxis ax, const double* __restrict__ in, double* __restrict_
   store_transposed<M>(sm, col0, total, ncol, g.nG, out);
 }
 
-// x transform of rows, in place where in == out: out = row, or out = sub_from - row
+// Vort2Flux of all levels at once (v2f.cu), first y pass: columns of the transposed intermediate in
+// place, S_y times m; and the spectrum's sums for the two quarter rows,
+// qrow[b-1][s][I] = sum_j sin(pi j J_s / ny) spec[I][j], J_s = ny/4, 3ny/4 (arrays qls values apart), for
+// every level but the finest, whose lines no ring is made of.
 template <int M>
 __global__ void __launch_bounds__(Bounds<M>::kThreads, Bounds<M>::kBlocks)
-k_fx_inv(Geometry g, FxAxis ax, const double* in, double* out, int batch, const double* sub_from) {
+k_fx_yspec(Geometry g, FxAxis ax, double* w, int batch, const double* __restrict__ mult, double* __restrict__ qrow,
+           int64_t qls) {
+  pdl_begin();
+  constexpr int NT = group_threads(M), PP = pairs(M), lpb = Bounds<M>::kLines, n = 2 * M;
+  const int grp = threadIdx.x / NT;
+  const Smem sm = carve<M>(grp);
+  const Group<NT> G{(int)threadIdx.x % NT, grp, sm.line, sm.red};
+  const int ncol = g.nx - 1, nrow = n - 1, col = blockIdx.x * lpb + grp, t = G.t;
+  if (col >= batch * ncol) return;
+  const int b = col / ncol, I = col - b * ncol;
+  double* line = w + (int64_t)b * g.nG + (int64_t)I * nrow;
+  double u[PP], v[PP];
+  load_pairs<M>(line, t, u, v);
+  const int q = line_transform<M>(G, ax, u, v, [&] { load_pairs<M>(mult + (int64_t)I * nrow, t, u, v); });
+  double* lo = line - 1 + t;
+  double* hi = line + n - 1 - t;
+  double A = 0.0, B = 0.0, C = 0.0;  // sums over j = t mod NT, over n - j, and the middle value
+  with_results<M, double>(Pairs<M>(G.buf, t), t, q, [&](int i, bool mid, double x, double y) {
+    x *= u[i];
+    *(mid ? line + M - 1 : lo + NT * i) = x;
+    if (mid) {
+      C = x;
+    } else {
+      y *= v[i];
+      hi[-NT * i] = y;
+      A += x;
+      B += y;
+    }
+  });
+  if (b == 0) return;
+  // sin(pi j / 4) for j mod 8, which is one per thread; at 3/4 the even j change sign
+  auto quarter = [](int j) {
+    const double s = (j & 1) ? 0.70710678118654752440 : ((j & 3) == 2 ? 1.0 : 0.0);
+    return (j & 4) ? -s : s;
+  };
+  const double s = quarter(t) * A + quarter(n - t) * B;
+  double sa = s, sb = (t & 1) ? s : -s;
+  if (t == 0) {
+    sa = fma(quarter(M), C, sa);
+    sb = fma(-quarter(M), C, sb);  // (M is even)
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sa += __shfl_xor_sync(kAll, sa, o);
+    sb += __shfl_xor_sync(kAll, sb, o);
+  }
+  if (NT > 32) {
+    G.put(0, (unsigned)__double2loint(sa));
+    G.put(1, (unsigned)__double2hiint(sa));
+    G.put(2, (unsigned)__double2loint(sb));
+    G.put(3, (unsigned)__double2hiint(sb));
+    G.bar();
+    constexpr int W = NT / 32;
+    sa = sb = 0.0;
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      sa += __hiloint2double((int)G.red[W + k], (int)G.red[k]);
+      sb += __hiloint2double((int)G.red[3 * W + k], (int)G.red[2 * W + k]);
+    }
+  }
+  if (t == 0) {
+    double* dst = qrow + (b - 1) * qls + I;
+    dst[0] = sa;
+    dst[ncol] = sb;
+  }
+}
+
+// Last y pass of the same: the spectrum w plus m times the transform of apply_bc(ring), S_y, stored
+// row-major.  A ring's transform is a sum of products of 1-D transforms of its sides, at column
+// k = I + 1 and row j
+//   sin(pi j/ny) (Fb_k - (-1)^j Ft_k) + sin(pi k/nx) (Fl_j - (-1)^k Fr_j)
+// side: per ring Fb, Ft, Fl, Fr; sinx, siny: the sines.  The slots from r.n on have no ring.
+template <int M>
+__global__ void __launch_bounds__(Bounds<M>::kThreads, Bounds<M>::kBlocks)
+k_fx_yring(Geometry g, FxAxis ax, const double* __restrict__ w, double* __restrict__ out, int batch,
+           const double* __restrict__ mult, int nring, const double* __restrict__ side,
+           const double* __restrict__ sinx, const double* __restrict__ siny) {
+  pdl_begin();
+  constexpr int NT = group_threads(M), PP = pairs(M), lpb = Bounds<M>::kLines, n = 2 * M;
+  const int grp = threadIdx.x / NT;
+  const Smem sm = carve<M>(grp);
+  const Group<NT> G{(int)threadIdx.x % NT, grp, sm.line, sm.red};
+  const int ncol = g.nx - 1, nrow = n - 1, total = batch * ncol;
+  const int col0 = blockIdx.x * lpb, col = col0 + grp;
+  if (col < total) {
+    const int b = col / ncol, I = col - b * ncol, t = G.t;
+    double u[PP], v[PP];
+    load_pairs<M>(w + (int64_t)b * g.nG + (int64_t)I * nrow, t, u, v);
+    if (b < nring) {
+      const double* m = mult + (int64_t)I * nrow;
+      const double* sd = side + (int64_t)b * 2 * (ncol + nrow);
+      const double fb = sd[I], ft = sd[ncol + I];
+      const double* fl = sd + 2 * ncol;
+      const double* fr = fl + nrow;
+      const double sk = sinx[I], sr = (I & 1) ? -sk : sk;
+      const double fs = (t & 1) ? fb + ft : fb - ft;  // j has t's parity (t = 0: the middle's, even)
+      auto add = [&](double& x, int j) {
+        x = fma(m[j - 1], fma(siny[j - 1], fs, fma(sk, fl[j - 1], sr * fr[j - 1])), x);
+      };
+#pragma unroll
+      for (int i = 0; i < PP; ++i) {
+        const int j = t + NT * i;
+        if (M == NT * PP || j < M) {
+          const bool mid = i == 0 && t == 0;
+          add(u[i], mid ? M : j);
+          if (!mid) add(v[i], n - j);
+        }
+      }
+    }
+    const int q = line_transform<M>(G, ax, u, v, [] {});
+    if (t == 0) sm.q[grp] = q;
+  }
+  store_transposed<M>(sm, col0, total, ncol, g.nG, out);
+}
+
+// x transform of rows, in place where in is out's memory: out = row, or out = sub_from - row
+template <int M, typename T>
+__global__ void __launch_bounds__(Bounds<M>::kThreads, Bounds<M>::kBlocks)
+k_fx_inv(Geometry g, FxAxis ax, const double* in, T* out, int batch, const T* sub_from) {
   pdl_begin();
   constexpr int NT = group_threads(M), PP = pairs(M), lpb = Bounds<M>::kLines;
   const int grp = threadIdx.x / NT;
@@ -577,16 +731,17 @@ k_fx_inv(Geometry g, FxAxis ax, const double* in, double* out, int batch, const 
   const int64_t off = (int64_t)b * g.nG + (int64_t)J * ncol;
   double u[PP], v[PP];
   load_pairs<M>(in + off, t, u, v);
+  T a[PP], c[PP];
   const int q = line_transform<M>(G, ax, u, v, [&] {
-    if (sub_from) load_pairs<M>(sub_from + off, t, u, v);
+    if (sub_from) load_pairs<M>(sub_from + off, t, a, c);
   });
   const Pairs<M> w(G.buf, t);
-  double* lo = out + off - 1 + t;
-  double* hi = out + off + 2 * M - 1 - t;
-  with_results<M>(w, t, q, [&](int i, bool mid, double x, double y) {
+  T* lo = out + off - 1 + t;
+  T* hi = out + off + 2 * M - 1 - t;
+  with_results<M, T>(w, t, q, [&](int i, bool mid, T x, T y) {
     if (sub_from) {
-      x = u[i] - x;
-      y = v[i] - y;
+      x = a[i] - x;
+      y = c[i] - y;
     }
     *(mid ? out + off + M - 1 : lo + NT * i) = x;
     if (!mid) hi[-NT * i] = y;
@@ -602,10 +757,10 @@ cudaError_t launch(K k, int lines, cudaStream_t s, Args... args) {
 }
 
 // the passes of one length (dstfx.cu has the entry points)
-template <int M>
-cudaError_t run_fwd(const Geometry& g, const FxAxis& ax, const double* in, double* out, int batch, const double* bc,
-                    double bcfac, cudaStream_t s) {
-  return launch<M>(k_fx_fwd<M>, batch * (g.ny - 1), s, g, ax, in, out, batch, bc, bcfac);
+template <int M, typename T>
+cudaError_t run_fwd(const Geometry& g, const FxAxis& ax, const T* in, double* out, int batch, const T* bc,
+                    cudaStream_t s) {
+  return launch<M>(k_fx_fwd<M, T>, batch * (g.ny - 1), s, g, ax, in, out, batch, bc);
 }
 template <int M>
 cudaError_t run_y(const Geometry& g, const FxAxis& ay, const double* in, double* out, int batch, const double* mult,
@@ -613,18 +768,35 @@ cudaError_t run_y(const Geometry& g, const FxAxis& ay, const double* in, double*
   return launch<M>(k_fx_y<M>, batch * (g.nx - 1), s, g, ay, in, out, batch, mult, mstride, log2scale);
 }
 template <int M>
-cudaError_t run_inv(const Geometry& g, const FxAxis& ax, const double* in, double* out, int batch,
-                    const double* sub_from, cudaStream_t s) {
-  return launch<M>(k_fx_inv<M>, batch * (g.ny - 1), s, g, ax, in, out, batch, sub_from);
+cudaError_t run_yspec(const Geometry& g, const FxAxis& ay, double* w, int batch, const double* mult, double* qrow,
+                      int64_t qls, cudaStream_t s) {
+  return launch<M>(k_fx_yspec<M>, batch * (g.nx - 1), s, g, ay, w, batch, mult, qrow, qls);
+}
+template <int M>
+cudaError_t run_yring(const Geometry& g, const FxAxis& ay, const double* w, double* out, int batch, const double* mult,
+                      const FxRings& r, cudaStream_t s) {
+  return launch<M>(k_fx_yring<M>, batch * (g.nx - 1), s, g, ay, w, out, batch, mult, r.n, r.side, r.sinx, r.siny);
+}
+template <int M, typename T>
+cudaError_t run_inv(const Geometry& g, const FxAxis& ax, const double* in, T* out, int batch, const T* sub_from,
+                    cudaStream_t s) {
+  return launch<M>(k_fx_inv<M, T>, batch * (g.ny - 1), s, g, ax, in, out, batch, sub_from);
 }
 
-#define IB_FX_RUN(PREFIX, M)                                                                                        \
-  PREFIX template cudaError_t run_fwd<M>(const Geometry&, const FxAxis&, const double*, double*, int, const double*, \
-                                         double, cudaStream_t);                                                     \
+#define IB_FX_RUN_X(PREFIX, M, T)                                                                              \
+  PREFIX template cudaError_t run_fwd<M, T>(const Geometry&, const FxAxis&, const T*, double*, int, const T*,  \
+                                            cudaStream_t);                                                     \
+  PREFIX template cudaError_t run_inv<M, T>(const Geometry&, const FxAxis&, const double*, T*, int, const T*,  \
+                                            cudaStream_t);
+#define IB_FX_RUN(PREFIX, M)                                                                                         \
+  IB_FX_RUN_X(PREFIX, M, double)                                                                                     \
+  IB_FX_RUN_X(PREFIX, M, df64)                                                                                       \
   PREFIX template cudaError_t run_y<M>(const Geometry&, const FxAxis&, const double*, double*, int, const double*,   \
-                                       int64_t, int, cudaStream_t);                                                 \
-  PREFIX template cudaError_t run_inv<M>(const Geometry&, const FxAxis&, const double*, double*, int, const double*, \
-                                         cudaStream_t);
+                                       int64_t, int, cudaStream_t);                                                  \
+  PREFIX template cudaError_t run_yspec<M>(const Geometry&, const FxAxis&, double*, int, const double*, double*,     \
+                                           int64_t, cudaStream_t);                                                   \
+  PREFIX template cudaError_t run_yring<M>(const Geometry&, const FxAxis&, const double*, double*, int,              \
+                                           const double*, const FxRings&, cudaStream_t);
 
 // the accepted lengths, by the translation unit that compiles their kernels
 #define IB_FX_GROUP_1(X) X(4) X(24) X(60) X(108) X(180) X(288) X(450) X(640) X(900)

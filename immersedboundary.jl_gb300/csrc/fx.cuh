@@ -201,6 +201,18 @@ FX_HD i64 to_fixed(u64 bits, int ex) {
   return (r ^ sg) - sg;
 }
 
+// The same for a float given by its bits, ex the biased exponent (at least 1) of the largest float of
+// the line's values: x 2^q, q = kInBits + 126 - ex.
+FX_HD i64 to_fixed_float(unsigned bits, int ex) {
+  const int e = (int)(bits >> 23) & 255;
+  const unsigned m = (bits & 0x7fffffu) | (e > 0 ? 0x800000u : 0u);
+  int s = ex - (e > 0 ? e : 1);
+  if (s > 63) s = 63;
+  const i64 r = (i64)(((((u64)m << (kInBits - 23)) >> s) + 1) >> 1);
+  const i64 sg = (i64)((int)bits >> 31);
+  return (r ^ sg) - sg;
+}
+
 FX_HD int clz64(u64 v) {
 #if defined(__CUDA_ARCH__)
   return __clzll((long long)v);
@@ -221,6 +233,28 @@ FX_HD u64 from_fixed(i64 v, int q) {
   const u64 e = (u64)(unsigned)(1023 + 62 - q - lz);
   const u64 r = (e << 52) + (m >> 11) + ((m >> 10) & 1);
   return v == 0 ? 0 : (r | sg);
+}
+
+// The float-float number nearest v 2^-q: its first part as bits, the rest as an integer r times 2^e.
+// Beyond the float range: zero, or infinity.
+struct pair_float {
+  unsigned hi;
+  int r, e;
+};
+FX_HD pair_float from_fixed_pair(i64 v, int q) {
+  const unsigned sg = (unsigned)((u64)v >> 32) & 0x80000000u;
+  u64 m = v < 0 ? (u64)0 - (u64)v : (u64)v;
+  const int lz = clz64(m);
+  m <<= (lz & 63);
+  const unsigned t = (unsigned)(m >> 40) + ((unsigned)(m >> 39) & 1u);  // 24 bits, rounded
+  const int rem = (int)((i64)(m - ((u64)t << 40)) >> 8);                // what is left, in 2^8 units of m
+  const int eh = 127 + 63 - lz - q;                                     // biased exponent of the leading bit
+  pair_float p;
+  p.hi = sg | (eh > 254 ? 0x7f800000u : ((unsigned)(eh - 1) << 23) + t);
+  p.r = eh > 254 ? 0 : (sg ? -rem : rem);
+  p.e = 8 - lz - q;
+  if (v == 0 || eh < 1) p = {0u, 0, 0};
+  return p;
 }
 
 }  // namespace fx

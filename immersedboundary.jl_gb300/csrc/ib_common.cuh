@@ -178,18 +178,33 @@ struct YPassArgs {
 template <typename T>
 cudaError_t ypass(const Geometry& g, const DstAxis<T>& ax, const YPassArgs<T>& a, cudaStream_t s);
 
-// The FP64 passes (dstfx.cu), arrays of nG doubles.
-//   fx_fwd:   in [+ bcfac * apply_bc(bc) on the edges] -> x transform -> out transposed, column by
-//             column (element (I, J) of slot b at b*nG + I*(ny-1) + J); out != in
+// The fixed-point passes (dstfx.cu), arrays of nG values: doubles, or (first and last pass) float-float.
+//   fx_fwd:   in [+ apply_bc(bc, 1) on the edges] -> x transform -> out transposed, column by column
+//             (element (I, J) of slot b at b*nG + I*(ny-1) + J); out != in
 //   fx_ypass: per column S_y, times mult (per slot stride mstride, column-major), S_y (mult == nullptr:
 //             S_y only), times 2^log2scale -> out row-major; out != in
-//   fx_inv:   rows -> x transform -> out, or out = sub_from - (.) (out may be in or sub_from)
-cudaError_t fx_fwd(const Geometry& g, const FxAxis& ax, const double* in, double* out, int batch, const double* bc,
-                   double bcfac, cudaStream_t s);
+//   fx_inv:   rows -> x transform -> out, or out = sub_from - (.) (out may be in's memory or sub_from)
+template <typename T>
+cudaError_t fx_fwd(const Geometry& g, const FxAxis& ax, const T* in, double* out, int batch, const T* bc,
+                   cudaStream_t s);
 cudaError_t fx_ypass(const Geometry& g, const FxAxis& ay, const double* in, double* out, int batch, const double* mult,
                      int64_t mstride, int log2scale, cudaStream_t s);
-cudaError_t fx_inv(const Geometry& g, const FxAxis& ax, const double* in, double* out, int batch,
-                   const double* sub_from, cudaStream_t s);
+template <typename T>
+cudaError_t fx_inv(const Geometry& g, const FxAxis& ax, const double* in, T* out, int batch, const T* sub_from,
+                   cudaStream_t s);
+
+// The y passes of the all-levels Vort2Flux (v2f.cu): the multiplied spectrum in place with its sums for
+// the quarter rows of slots 1..batch-1; and S_y of the spectrum with the rings' share added, out
+// row-major (out != w).
+struct FxRings {
+  int n;                      // slots with a ring
+  const double* side;         // transforms of their sides: per slot bottom, top, left, right
+  const double *sinx, *siny;  // sin(pi (i+1) / n) along each axis
+};
+cudaError_t fx_yspec(const Geometry& g, const FxAxis& ay, double* w, int batch, const double* mult, double* qrow,
+                     int64_t qls, cudaStream_t s);
+cudaError_t fx_yring(const Geometry& g, const FxAxis& ay, const double* w, double* out, int batch, const double* mult,
+                     const FxRings& r, cudaStream_t s);
 
 // Warp-per-line passes (dstw_*.cu), for axes with wdst_axis_supported.  The intermediate of a
 // solve is stored transposed, column by column: element (I, J) of slot b at b*stride + I*(ny-1) + J.
@@ -386,7 +401,13 @@ struct RingPlan {
   float *vrow = nullptr, *ucolp = nullptr, *ucol = nullptr, *qline = nullptr, *sidex = nullptr, *sidey = nullptr;
   double *ringd = nullptr, *coef = nullptr;  // change of each level's ring (FP64), its coefficients
   double* dring = nullptr;                   // the change as float-float (df64 pairs)
-  cudaError_t build(const Geometry& g);
+  // fixed-point form (doubles): quarter rows and columns of levels 1.. (sums over the spectrum, then
+  // lines; qls values a level), ring sides and their transforms (qls a ring), sines along the axes, and
+  // the harmonic part of a ring in terms of the coefficients of the ring d levels up, d = 1..L-2:
+  // Aring (St-sides of Aring)^(d-1), [d-1][nK][nbc]
+  double *qfx = nullptr, *side = nullptr, *sinx = nullptr, *siny = nullptr, *Apow = nullptr;
+  cudaError_t build(const Geometry& g, const double* mult);  // mult: of the Poisson solve (device)
+  cudaError_t build_fx(const Geometry& g, cudaStream_t s);  // after build()
   void release();
 };
 cudaError_t v2f_yspec(const Geometry& g, const DstAxis<float>& ax, float* w, const float* m, int batch, float* vrow,
@@ -399,6 +420,10 @@ cudaError_t v2f_lines(const DstAxis<float>& ax, const float* in, int64_t in_b, i
 cudaError_t v2f_ring_eval(const Geometry& g, const RingPlan& rp, int l, const df64* xp_up, const float* x0_up,
                           df64* ring_l, cudaStream_t s);
 cudaError_t v2f_ring_coef(const Geometry& g, const RingPlan& rp, int l, cudaStream_t s);
+// the same on doubles: column sums of the spectrum of levels 1..; every ring from the quarter lines
+cudaError_t v2f_fx_colsum(const Geometry& g, const RingPlan& rp, const double* w, cudaStream_t s);
+template <typename S>
+cudaError_t v2f_fx_rings(const Geometry& g, const RingPlan& rp, S* rings, cudaStream_t s);
 
 // ----------------------------------------------------------------------------------------------
 // Programmatic dependent launch: while g_pdl is set (the capture of a static step's graph), the

@@ -45,9 +45,9 @@ extern "C" int ib_op_laplacian_inv_noalloc(ib_handle* h, int32_t batch, const do
   if (e != cudaSuccess) return ib_handle_fail(h, IB_ERR_CUDA, cudaGetErrorString(e));
   double* w = static_cast<double*>(wp);
   // x = F2D(mlap .* F2D(b)): x pass into the fixed work array, y pass out of it, x pass in place
-  e = ib::fx_fwd(v.g, v.ax, b, w, batch, nullptr, 1.0, v.stream);
+  e = ib::fx_fwd<double>(v.g, v.ax, b, w, batch, nullptr, v.stream);
   if (e == cudaSuccess) e = ib::fx_ypass(v.g, v.ay, w, x, batch, v.mlap, 0, 0, v.stream);
-  if (e == cudaSuccess) e = ib::fx_inv(v.g, v.ax, x, x, batch, nullptr, v.stream);
+  if (e == cudaSuccess) e = ib::fx_inv<double>(v.g, v.ax, x, x, batch, nullptr, v.stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(v.stream);
   if (e != cudaSuccess) return ib_handle_fail(h, IB_ERR_CUDA, cudaGetErrorString(e));
   return IB_OK;

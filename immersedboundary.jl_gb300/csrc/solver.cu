@@ -85,6 +85,9 @@ struct ib_handle {
   int coarse_from = 2;                          // first (0-based) level counted as coarse
   bool wdst = false;                            // both axes use the warp-per-line passes
   bool gdst = false;                            // mixed precision: transforms as tensor-core GEMMs
+  bool tuned_levels = false;                    // mixed precision: the order the autotuner chose
+  bool fx_solve = false;                        // mixed precision: solves in fixed point
+  bool v2f_fx = false;                          // Vort2Flux in fixed point (FP64 handles: always)
   int scheme = IB_SCHEME_CNAB;                  // time stepping (IB_SCHEME_*)
   int rkc_s = 0;                                // Runge-Kutta-Chebyshev: stages and their
   std::vector<double> rkc_mu, rkc_nu, rkc_mut, rkc_gamt;  // coefficients (index = stage)
@@ -228,17 +231,18 @@ SolveOp op_lap(const ib_handle* h) { return {h->mLap, h->mLap32, 0, h->d_zero, h
 SolveOp op_cn_all(const ib_handle* h) { return {h->mCN1, h->mCN1_32, h->g.nG, h->d_one, h->d_alpha, 1}; }
 SolveOp op_cn1(const ib_handle* h) { return {h->mCN1, h->mCN1_32, 0, h->d_one, h->d_alpha, 0}; }
 
-// FP64 solve of `batch` arrays: out = F2D(m .* F2D(in [+ apply_bc(bc, 1)])), optional
-// subtract epilogue out = sub_from - (...).  w: FP64 work of batch arrays (the transposed
+// Fixed-point solve of `batch` arrays (double or float-float): out = F2D(m .* F2D(in [+ apply_bc(bc,
+// 1)])), optional subtract epilogue out = sub_from - (...).  w: FP64 work of batch arrays (the transposed
 // intermediate).  The row-major intermediate is in `out`, or, where that holds sub_from, in h->w2
 // (at most nlevels arrays).
-cudaError_t poisson64(ib_handle* h, const double* in, double* out, int batch, const double* bc, const SolveOp& op,
-                      const double* sub_from, double* w) {
-  CE(fx_fwd(h->g, h->axx.d, in, w, batch, bc, 1.0, h->stream));
-  double* t = sub_from == out ? h->w2 : out;
-  if (t != out && batch > h->g.nlev) return cudaErrorInvalidValue;
+template <typename T>
+cudaError_t poisson_fx(ib_handle* h, const T* in, T* out, int batch, const T* bc, const SolveOp& op, const T* sub_from,
+                       double* w) {
+  CE(fx_fwd<T>(h->g, h->axx.d, in, w, batch, bc, h->stream));
+  double* t = sub_from == out ? h->w2 : reinterpret_cast<double*>(out);
+  if (sub_from == out && batch > h->g.nlev) return cudaErrorInvalidValue;
   CE(fx_ypass(h->g, h->axy.d, w, t, batch, op.m64, op.mstride, 0, h->stream));
-  return fx_inv(h->g, h->axx.d, t, out, batch, sub_from, h->stream);
+  return fx_inv<T>(h->g, h->axx.d, t, out, batch, sub_from, h->stream);
 }
 
 // Mixed-precision solve: FP32 sine transforms refined with float-float residuals.
@@ -386,15 +390,12 @@ cudaError_t poisson_mixed(ib_handle* h, const df64* in, df64* out, int batch, co
 // double -> FP64 transforms, df64 -> the mixed-precision solve.
 cudaError_t solve(ib_handle* h, const double* in, double* out, int batch, const double* bc, const SolveOp& op,
                   const double* sub_from) {
-  return poisson64(h, in, out, batch, bc, op, sub_from, h->w1);
+  return poisson_fx<double>(h, in, out, batch, bc, op, sub_from, h->w1);
 }
 cudaError_t solve(ib_handle* h, const df64* in, df64* out, int batch, const df64* bc, const SolveOp& op,
-                  const df64* sub_from, int sweeps = 0) {
-  return poisson_mixed(h, in, out, batch, bc, op, sub_from, h->w32, h->x032, h->x132, sweeps > 0 ? sweeps : h->refine);
-}
-cudaError_t solve(ib_handle* h, const double* in, double* out, int batch, const double* bc, const SolveOp& op,
-                  const double* sub_from, int /*sweeps*/) {
-  return poisson64(h, in, out, batch, bc, op, sub_from, h->w1);
+                  const df64* sub_from) {
+  if (h->fx_solve) return poisson_fx<df64>(h, in, out, batch, bc, op, sub_from, h->w1);
+  return poisson_mixed(h, in, out, batch, bc, op, sub_from, h->w32, h->x032, h->x132, h->refine);
 }
 
 // The handle's state arrays hold doubles (FP64 mode) or float-float pairs (mixed mode); both are
@@ -494,11 +495,79 @@ cudaError_t vort2flux_levels(ib_handle* h, df64* gam, df64* psi, df64* q, df64* 
   return q ? curl<df64>(g, psi, rings, q, L, s) : curl<df64>(g, psi, rings, q1, 1, s);
 }
 
+// Vort2Flux of all levels in one batch, in fixed point: no predictor and no sweeps, the rings as in
+// vort2flux_levels.
+//   spectra of Gamma / L of every level with zero rings (in w1), their sums for the quarter lines, the
+//   lines; rings coarse to fine; the rings' own spectrum added on the way back
+// The spectra stay in FP64, so the lines and rings carry no more error than a solve (2e-15 of psi apart
+// from the other order at 256^2, 8e-15 at 1024^2).  Against the level-by-level order it runs one chain of passes where that runs one per level, and a
+// call that wants the finest level's fluxes alone (the trial state, B's products) leaves out half of
+// the coarser levels' passes.
 template <typename S>
-cudaError_t vort2flux(ib_handle* h, S* gam, S* psi, S* q, S* q1, S* rings) {
+cudaError_t vort2flux_fx(ib_handle* h, S* gam, S* psi, S* q, S* q1, S* rings, bool may_fork) {
+  const Geometry& g = h->g;
+  const int L = g.nlev, ncol = g.nx - 1;
+  const int64_t nG = g.nG;
+  cudaStream_t s = h->stream;
+  const RingPlan& rp = h->rplan;
+  const int nf = q ? L : 1;               // finished levels
+  const int ns = std::min(nf, L - 1);     // of them, those with a ring
+  const bool fork = may_fork && h->side;
+  // transforms of m levels' quarter lines or ring sides (2 along x, 2 along y each), in place: as the
+  // rows of one array on a square grid; else of two, side by side where there is a side stream
+  auto lines = [&](double* v, int m) -> cudaError_t {
+    Geometry gx = g, gy = g;
+    gx.nG = gy.nG = rp.qls;
+    gx.ny = gy.ny = 3;
+    gy.nx = g.ny;
+    if (g.nx == g.ny) {
+      gx.ny = 5;
+      return fx_inv<double>(gx, h->axx.d, v, v, m, nullptr, s);
+    }
+    cudaStream_t sy = s;
+    if (fork) {
+      CE(cudaEventRecord(h->fork_ev[0], s));
+      CE(cudaStreamWaitEvent(h->side, h->fork_ev[0], 0));
+      sy = h->side;
+    }
+    CE(fx_inv<double>(gx, h->axx.d, v, v, m, nullptr, s));
+    CE(fx_inv<double>(gy, h->axy.d, v + 2 * ncol, v + 2 * ncol, m, nullptr, sy));
+    if (fork) {
+      CE(cudaEventRecord(h->fork_ev[1], h->side));
+      CE(cudaStreamWaitEvent(s, h->fork_ev[1], 0));
+    }
+    return cudaSuccess;
+  };
+  for (int l = 1; l < L; ++l) CE(coarsify<S>(g, gam + l * nG, gam + (l - 1) * nG, 1, nG, s));
+  CE(fx_fwd<S>(g, h->axx.d, gam, h->w1, L, nullptr, s));
+  CE(fx_yspec(g, h->axy.d, h->w1, L, h->mLap, rp.qfx, rp.qls, s));
+  CE(v2f_fx_colsum(g, rp, h->w1, s));
+  CE(lines(rp.qfx, L - 1));
+  CE(v2f_fx_rings<S>(g, rp, rings, s));
+  CE(lines(rp.side, ns));
+  const FxRings r{ns, rp.side, rp.sinx, rp.siny};
+  double* t = reinterpret_cast<double*>(psi);
+  CE(fx_yring(g, h->axy.d, h->w1, t, nf, h->mLap, r, s));
+  CE(fx_inv<S>(g, h->axx.d, t, psi, nf, nullptr, s));
+  return q ? curl<S>(g, psi, rings, q, L, s) : curl<S>(g, psi, rings, q1, 1, s);
+}
+
+// may_fork: whether the side stream may be used (not where a conditional graph body is captured)
+template <typename S>
+cudaError_t vort2flux(ib_handle* h, S* gam, S* psi, S* q, S* q1, S* rings, bool may_fork = true) {
+  if (h->v2f_levels && h->v2f_fx) return vort2flux_fx(h, gam, psi, q, q1, rings, may_fork);
   if constexpr (std::is_same<S, df64>::value) {
     if (h->v2f_levels) return vort2flux_levels(h, gam, psi, q, q1, rings);
   }
+  // one level's solve: FP64 and fixed-point handles alike, or the FP32 passes
+  auto level_solve = [&](const S* in, S* out, const S* ring, int sweeps) -> cudaError_t {
+    if constexpr (std::is_same<S, df64>::value) {
+      if (!h->v2f_fx)
+        return poisson_mixed(h, in, out, 1, ring, op_lap(h), nullptr, h->w32, h->x032, h->x132,
+                             sweeps > 0 ? sweeps : h->refine);
+    }
+    return poisson_fx<S>(h, in, out, 1, ring, op_lap(h), nullptr, h->w1);
+  };
   const Geometry& g = h->g;
   const int L = g.nlev;
   const int64_t nG = g.nG;
@@ -513,14 +582,13 @@ cudaError_t vort2flux(ib_handle* h, S* gam, S* psi, S* q, S* q1, S* rings) {
   for (int l = 1; l < L; ++l) CE(coarsify<S>(g, gam + l * nG, gam + (l - 1) * nG, 1, nG, s));
   // mixed precision: the coarse levels only feed the finer levels' boundary rings
   const int coarse = std::min(h->refine, h->refine_coarse);
-  CE(solve(h, gam + (L - 1) * nG, psi + (L - 1) * nG, 1, nullptr, op_lap(h), nullptr,
-           L - 1 >= h->coarse_from ? coarse : 0));
+  CE(level_solve(gam + (L - 1) * nG, psi + (L - 1) * nG, nullptr, L - 1 >= h->coarse_from ? coarse : 0));
   if (q) CE(curl_level(L - 1, nullptr));
   else if (L == 1) CE(curl<S>(g, psi, nullptr, q1, 1, s));
   for (int l = L - 2; l >= 0; --l) {
     S* ring = rings + (int64_t)l * g.nbc;
     CE(get_bc<S>(g, psi + (l + 1) * nG, ring, 1, S(1.0), s));
-    CE(solve(h, gam + l * nG, psi + l * nG, 1, ring, op_lap(h), nullptr, l >= h->coarse_from ? coarse : 0));
+    CE(level_solve(gam + l * nG, psi + l * nG, ring, l >= h->coarse_from ? coarse : 0));
     if (q) CE(l > 0 ? curl_level(l, ring) : curl<S>(g, psi, ring, q, 1, s));
     else if (l == 0) CE(curl<S>(g, psi, ring, q1, 1, s));
   }
@@ -585,7 +653,7 @@ cudaError_t enqueue_trial(ib_handle* h, int p) {
   // Gamma_s[l] = Ainv_l rhs[l] for every level in one batched solve (mixed precision: refined
   // from Gamma_n[l], the change over one step being what the FP32 sweeps carry)
   if constexpr (std::is_same<S, df64>::value) {
-    if (h->cn_pred)
+    if (h->cn_pred && !h->fx_solve)
       CE(poisson_mixed(h, view<S>(h->rhs), gs, L, nullptr, op_cn_all(h), nullptr, h->w32, h->x032, h->x132, 2, gam));
     else
       CE(solve(h, view<S>(h->rhs), gs, L, nullptr, op_cn_all(h), nullptr));
@@ -616,7 +684,7 @@ cudaError_t enqueue_project(ib_handle* h, int p) {
                           h->status + 1, h->d_box, h->box_ready, h->stream));
     bool done = false;
     if constexpr (std::is_same<S, df64>::value) {
-      if (h->cn_pred && h->cprev && h->wdst && h->r1) {
+      if (h->cprev && h->wdst && h->r1) {
         // c = Ainv_1 C^T E^T Fb refined from the previous step's c (kept in cprev), then
         // Gamma_s1 -= c
         df64* c = view<df64>(h->cprev);
@@ -764,7 +832,7 @@ cudaError_t schur_apply(ib_handle* h, const double* z, double* out) {
                         h->status + 1, h->d_box, h->box_ready, s));
   CE(solve(h, view<S>(h->gtmp), Gw, 1, nullptr, op_cn1(h), nullptr));
   if (g.nlev > 1) CE(cudaMemsetAsync(Gw + g.nG, 0, sizeof(S) * (g.nlev - 1) * g.nG, s));
-  CE(vort2flux<S>(h, Gw, view<S>(h->Pw), nullptr, view<S>(h->qw), view<S>(h->rings_w)));
+  CE(vort2flux<S>(h, Gw, view<S>(h->Pw), nullptr, view<S>(h->qw), view<S>(h->rings_w), false));
   return reg_gather<S>(g, view<S>(h->qw), nullptr, h->body_idx, h->weight, h->nb, out, 1, g.nq, h->nf, s);
 }
 
@@ -820,7 +888,7 @@ cudaError_t schur_columns(ib_handle* h, int c0, int n, double* Wa, double* Gb, d
   cudaStream_t s = h->stream;
   auto psolve = [&](const S* in, S* out, const S* bc, const SolveOp& op) -> cudaError_t {
     if constexpr (std::is_same<S, double>::value) {
-      return poisson64(h, in, out, n, bc, op, nullptr, Wb);
+      return poisson_fx<double>(h, in, out, n, bc, op, nullptr, Wb);
     } else {
       float* w = reinterpret_cast<float*>(Wb);
       return poisson_mixed(h, in, out, n, bc, op, nullptr, w, w + (int64_t)n * nG, nullptr, h->wdst ? 0 : 1);
@@ -914,10 +982,22 @@ int assemble_schur(ib_handle* h) {
 // Launch every kernel variant once outside of any capture (sets shared-memory attributes).
 int prime_kernels(ib_handle* h) {
   const Geometry& g = h->g;
-  CK(poisson64(h, h->w2, h->w2, 1, h->rings, op_lap(h), nullptr, h->w1));
-  CK(poisson64(h, h->w2, h->w2, 1, nullptr, op_lap(h), h->w2, h->w1));
+  CK(poisson_fx<double>(h, h->w2, h->w2, 1, h->rings, op_lap(h), nullptr, h->w1));
+  CK(poisson_fx<double>(h, h->w2, h->w2, 1, nullptr, op_lap(h), h->w2, h->w1));
+  CK(fx_yspec(g, h->axy.d, h->w1, 1, h->mLap, h->w2, 0, h->stream));
+  CK(fx_yring(g, h->axy.d, h->w1, h->w2, 1, h->mLap, FxRings{}, h->stream));
+  {  // x and y lines of the all-levels Vort2Flux (a row pass along y too)
+    Geometry gy = g;
+    gy.nx = g.ny;
+    gy.ny = 2;
+    CK(fx_inv<double>(gy, h->axy.d, h->w1, h->w1, 1, nullptr, h->stream));
+  }
   if (h->precision == IB_PREC_MIXED) {
     df64* w2 = view<df64>(h->w2);
+    if (h->fx_solve) {
+      CK(poisson_fx<df64>(h, w2, w2, 1, view<df64>(h->rings), op_lap(h), nullptr, h->w1));
+      CK(poisson_fx<df64>(h, w2, w2, 1, nullptr, op_cn1(h), w2, h->w1));
+    }
     for (int sw = 1; sw <= h->refine; ++sw) {
       CK(poisson_mixed(h, w2, w2, 1, view<df64>(h->rings), op_lap(h), nullptr, h->w32, h->x032, h->x132, sw));
       CK(poisson_mixed(h, w2, w2, 1, nullptr, op_cn1(h), w2, h->w32, h->x032, h->x132, sw));
@@ -1512,7 +1592,8 @@ int autotune(ib_handle* h, bool tune_form, bool tune_v2f, bool lv_base) {
     release();
     return fail(h, IB_ERR_CUDA, "autotuner scratch allocation");
   }
-  const bool wdst0 = h->wdst, gdst0 = h->gdst, lv0 = h->v2f_levels;
+  const bool wdst0 = h->wdst, gdst0 = h->gdst, lv0 = h->v2f_levels, fx0 = h->fx_solve;
+  h->fx_solve = h->v2f_fx = false;  // the candidates are the FP32 passes
   struct Cand { int form; bool levels; bool yalt; };
   std::vector<Cand> cands;
   std::vector<int> forms;
@@ -1561,7 +1642,7 @@ int autotune(ib_handle* h, bool tune_form, bool tune_v2f, bool lv_base) {
     h->gw32 = static_cast<float*>(p);
   }
   if (need_lv && !h->rplan.St) {
-    if ((e = h->rplan.build(g)) != cudaSuccess) {
+    if ((e = h->rplan.build(g, h->mLap)) != cudaSuccess) {
       release();
       return fail(h, IB_ERR_CUDA, "ring transfer tables", e);
     }
@@ -1600,6 +1681,7 @@ int autotune(ib_handle* h, bool tune_form, bool tune_v2f, bool lv_base) {
     }
   }
   release();
+  h->fx_solve = fx0;
   if (best < 0) {
     h->wdst = wdst0;
     h->gdst = gdst0;
@@ -1793,6 +1875,11 @@ int ib_create(const ib_problem* p, ib_handle** out) {
     if (std::strcmp(env, "stockham") == 0) { h->wdst = false; pin_form = true; }
     if (std::strcmp(env, "warp") == 0) { h->wdst = wsup; pin_form = true; }
   }
+  // Mixed handles solve in fixed point too, float-float in and out, unless the FP32 passes are asked for
+  // (one sweep, IBGB300_DST, IB_PREC_MIXED_TC): one such solve costs 1.1 FP32 transform solves at 256^2
+  // and two at 1024^2, where two to three FP32 solves made a refined one.  Steps, against FP32 in its
+  // better order: 256 x 192 x 3 247 -> 187 us, 1024^2 x 4 1114 -> 898, 2048^2 x 5 4372 -> 3932.
+  h->fx_solve = h->precision == IB_PREC_MIXED && h->refine >= 2 && !pin_form;
   // the setup-time autotuner (autotune() above) replaces these size rules unless switched off
   const char* tune_env = std::getenv("IBGB300_AUTOTUNE");
   const bool autotune_on = !(tune_env && tune_env[0] == '0');
@@ -1846,15 +1933,13 @@ int ib_create(const ib_problem* p, ib_handle** out) {
       if (std::strcmp(env, "sequential") == 0) { h->v2f_levels = false; pin_v2f = true; }
       if (std::strcmp(env, "levels") == 0) { h->v2f_levels = lv_ok; pin_v2f = true; }
     }
-    if (h->v2f_levels && !autotune_on && (e = h->rplan.build(g)) != cudaSuccess)
-      return bail(fail(h, IB_ERR_CUDA, "ring transfer tables", e));
   }
   AL(h->status, 4); AL(h->d_counter, 1); AL(h->d_box, 4);
   if (h->scheme == IB_SCHEME_RKC) {
     AL(h->rkY[0], L * nG); AL(h->rkY[1], L * nG); AL(h->rkF0, L * nG);
     AL(h->d_alpha_rkc, L); AL(h->d_fac_rkc, L);
   }
-  if (h->precision == IB_PREC_MIXED && h->cn_pred) AL(h->cprev, nG);
+  if (h->precision == IB_PREC_MIXED && h->cn_pred && !h->fx_solve) AL(h->cprev, nG);
   for (auto& ev : h->stress_ev)
     if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess) {
       ev = nullptr;
@@ -1915,13 +2000,31 @@ int ib_create(const ib_problem* p, ib_handle** out) {
     if (tune_form || tune_v2f) {
       int rc = autotune(h, tune_form, tune_v2f, lv_base);
       if (rc != IB_OK) return bail(rc);
-    } else if (mixed && h->v2f_levels && !h->rplan.St && (e = h->rplan.build(g)) != cudaSuccess) {
+    } else if (mixed && h->v2f_levels && !h->rplan.St && (e = h->rplan.build(g, h->mLap)) != cudaSuccess) {
       return bail(fail(h, IB_ERR_CUDA, "ring transfer tables", e));
     }
     if (mixed) {
       h->v2f_ok = lv_base && h->wdst && !h->gdst;
       if (h->tuned) h->v2f_auto = h->v2f_levels;
       else h->v2f_auto = h->v2f_auto && h->v2f_ok;
+    }
+    if (!mixed || h->fx_solve) {
+      // fixed-point Vort2Flux
+      h->tuned_levels = h->v2f_levels;
+      h->v2f_fx = true;
+      // by measurement (steps, all levels at once / level by level, us): 128^2 x 2 125 / 125, x 3 148 /
+      // 162; 256^2 x 3 196 / 209, x 4 205 / 258; 384 x 256 x 3 224 / 235; 512^2 x 3 344 / 332, x 4 404 /
+      // 422; 1024^2 x 3 837 / 819, x 4 997 / 1032; 2048^2 x 5 4442 / 4633
+      h->v2f_auto = L >= 4 || (L == 3 && (int64_t)g.nx * g.ny <= (int64_t(1) << 17));
+      if (!mixed)
+        if (const char* env = std::getenv("IBGB300_V2F")) {
+          if (std::strcmp(env, "sequential") == 0) h->v2f_auto = false;
+          if (std::strcmp(env, "levels") == 0) h->v2f_auto = L > 1;
+        }
+      if (!pin_v2f) h->v2f_levels = h->v2f_auto;
+      if (h->v2f_levels && ((!h->rplan.St && (e = h->rplan.build(g, h->mLap)) != cudaSuccess) ||
+                            (e = h->rplan.build_fx(g, h->stream)) != cudaSuccess))
+        return bail(fail(h, IB_ERR_CUDA, "ring transfer tables", e));
     }
   }
   if (nb > 0) {
@@ -2036,7 +2139,7 @@ int ib_set_state(ib_handle* h, const double* gamma, const double* q, const doubl
   // from its own psi (or zero) and zero rings
   // the projection's correction predicts the next one: a new state starts from zero
   if (h->cprev) CK(cudaMemsetAsync(h->cprev, 0, sizeof(double) * g.nG, s));
-  if (h->v2f_levels) {
+  if (h->precision == IB_PREC_MIXED && h->v2f_levels) {
     if (!psi) CK(cudaMemsetAsync(h->psi, 0, nGL, s));
     CK(cudaMemsetAsync(h->rings, 0, sizeof(double) * g.nlev * g.nbc, s));
     if (h->rings_w) CK(cudaMemsetAsync(h->rings_w, 0, sizeof(double) * g.nlev * g.nbc, s));
@@ -2245,19 +2348,22 @@ int ib_set_cg_preconditioner(ib_handle* h, int32_t mode, int32_t refresh_steps) 
 
 int ib_set_vort2flux_order(ib_handle* h, int32_t order) {
   if (!h || order < IB_V2F_AUTO || order > IB_V2F_SEQUENTIAL) return IB_ERR_INVALID;
-  if (h->precision != IB_PREC_MIXED) return IB_OK;
   DeviceGuard dev_guard_(h->device);
   CK(dev_guard_.err);
-  if (order == IB_V2F_LEVELS && !h->v2f_ok)
+  const bool mixed = h->precision == IB_PREC_MIXED;
+  if (mixed && order == IB_V2F_LEVELS && !h->v2f_ok)
     return fail(h, IB_ERR_UNSUPPORTED, "the all-levels Vort2Flux needs one-warp line passes on both axes");
-  const bool lv = order == IB_V2F_LEVELS || (order == IB_V2F_AUTO && h->v2f_auto);
-  if (lv == h->v2f_levels) return IB_OK;
+  const bool lv = (order == IB_V2F_LEVELS && h->g.nlev > 1) || (order == IB_V2F_AUTO && h->v2f_auto);
+  const bool fx = !mixed || (h->fx_solve && order != IB_V2F_SEQUENTIAL);
+  if (lv == h->v2f_levels && fx == h->v2f_fx) return IB_OK;
   CK(cudaStreamSynchronize(h->stream));
-  if (lv && !h->rplan.St) {
-    cudaError_t e = h->rplan.build(h->g);
+  if (lv) {
+    cudaError_t e = h->rplan.St ? cudaSuccess : h->rplan.build(h->g, h->mLap);
+    if (e == cudaSuccess && fx) e = h->rplan.build_fx(h->g, h->stream);
     if (e != cudaSuccess) return fail(h, IB_ERR_CUDA, "ring transfer tables", e);
   }
   h->v2f_levels = lv;
+  h->v2f_fx = fx;
   // the rings buffers then hold the other order's values: a predictor only, either is valid
   if (h->gexec[0]) {
     int rc = capture_graphs(h);
@@ -2393,7 +2499,7 @@ int ib_get_autotune(ib_handle* h, double* ms, int32_t* chosen) {
     for (int i = 0; i < 12; ++i) ms[i] = h->tune_ms[i];
   if (chosen)
     *chosen = h->tuned ? ((h->gdst ? IB_FORM_TENSOR : (h->wdst ? IB_FORM_WARP : IB_FORM_STOCKHAM)) * 2 +
-                          (h->v2f_levels ? 1 : 0)) * 2 + (h->axy32.d.wMinB == 8 ? 1 : 0)
+                          ((h->fx_solve ? h->tuned_levels : h->v2f_levels) ? 1 : 0)) * 2 + (h->axy32.d.wMinB == 8 ? 1 : 0)
                        : -1;
   return IB_OK;
 }
@@ -2470,7 +2576,7 @@ int ib_op_dst2(ib_handle* h, int32_t batch, const double* in, double* out) {
   double* w;
   CK(cudaMalloc(&w, sizeof(double) * batch * g.nG));
   // RODFT00 in both dimensions = 4 F_y F_x (F: the half-scaled transform of dstfx.cu)
-  cudaError_t e = fx_fwd(g, h->axx.d, in, w, batch, nullptr, 1.0, s);
+  cudaError_t e = fx_fwd<double>(g, h->axx.d, in, w, batch, nullptr, s);
   if (e == cudaSuccess) e = fx_ypass(g, h->axy.d, w, out, batch, nullptr, 0, 2, s);
   cudaStreamSynchronize(s);
   cudaFree(w);
@@ -2498,7 +2604,7 @@ int ib_op_laplacian_inv(ib_handle* h, int32_t batch, const double* b, double* x)
   if (batch < 1) return IB_ERR_INVALID;
   double* w;
   CK(cudaMalloc(&w, sizeof(double) * batch * g.nG));
-  cudaError_t e = poisson64(h, b, x, batch, nullptr, op_lap(h), nullptr, w);
+  cudaError_t e = poisson_fx<double>(h, b, x, batch, nullptr, op_lap(h), nullptr, w);
   cudaStreamSynchronize(s);
   cudaFree(w);
   CK(e);
@@ -2516,14 +2622,14 @@ static int cn_op(ib_handle* h, int32_t lev, const double* b, double* x, bool inv
   if (inverse) {
     SolveOp op = op_cn1(h);
     op.m64 = h->mCN1 + off;
-    e = poisson64(h, b, x, 1, nullptr, op, nullptr, w);
+    e = poisson_fx<double>(h, b, x, 1, nullptr, op, nullptr, w);
   } else {
     // A multiplier = 16 * scale / Lambda_expl = 16 * scale * cn2 ; build it on the device
     e = cudaMemcpyAsync(m, h->mCN2 + off, sizeof(double) * g.nG, cudaMemcpyDeviceToDevice, s);
     if (e == cudaSuccess) e = axpby<double>(m, m, 16.0 / (4.0 * g.nx * g.ny), 0.0, g.nG, s);
     SolveOp op = op_lap(h);
     op.m64 = m;
-    if (e == cudaSuccess) e = poisson64(h, b, x, 1, nullptr, op, nullptr, w);
+    if (e == cudaSuccess) e = poisson_fx<double>(h, b, x, 1, nullptr, op, nullptr, w);
   }
   cudaStreamSynchronize(s);
   cudaFree(w);
@@ -2971,7 +3077,7 @@ int ib_ensemble_create(ib_handle* const* members, int32_t n, ib_ensemble** out) 
   // static members fill the GPU between them: the level-by-level Vort2Flux there
   if (n >= 2)
     for (ib_handle* h : e->m)
-      if (h->motion != IB_MOTION_PRESCRIBED && h->v2f_levels) {
+      if (h->motion != IB_MOTION_PRESCRIBED && h->precision == IB_PREC_MIXED && h->v2f_levels && !h->v2f_fx) {
         const int rc = ib_set_vort2flux_order(h, IB_V2F_SEQUENTIAL);
         if (rc != IB_OK) return bail(efail(e, rc, "member Vort2Flux order: " + h->err));
       }

@@ -1,4 +1,5 @@
-// Multilevel Vort2Flux with all levels solved together (mixed precision, warp-per-line passes).
+// Multilevel Vort2Flux with all levels solved together: the ring transfer of the fixed-point form (both
+// precisions) and the kernels of the FP32 form (mixed precision, warp-per-line passes).
 //
 // Vort2Flux (src/streamfcn/fluid-ops.jl:438-472) solves the levels coarse to fine: level l's
 // Poisson problem takes its boundary ring from psi_{l+1} (get_bc!, fluid-ops.jl:210-239), so the
@@ -13,12 +14,13 @@
 // = 4 - 2 cos(pi (k+1)/n), i.e. by ~exp(-pi (k+1)/4) at the quarter lines: Kx (Ky) modes per
 // side give H there to FP64 rounding.  ring_l is then a small FP64 product per level:
 //   coef = St . sides(ring_{l+1}),  ring_l = ring(psi0_{l+1}) + Aring . coef.
-// psi0 on the quarter lines comes from the first refinement sweeps: the previous call's psi
+// FP32 form: psi0 on the quarter lines comes from the first refinement sweeps: the previous call's psi
 // plus an FP32 solve of its residual (x0) plus the next correction's spectrum evaluated on those
 // lines (row sums in the y pass, column sums over the spectrum, then 1-D transforms).  The
 // residual carries the rings of the previous call as a predictor, so psi0 above is psi with
 // those rings and the chain carries only the change:
 //   ring_l = get_bc(psi_old-ring_{l+1}) + Aring . coef(ring_{l+1} - ring_old_{l+1}).
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -295,45 +297,197 @@ k_ring_eval(Geometry g, const int4* __restrict__ pts, const df64* __restrict__ x
   else if (idx > g.R && idx < g.R + g.ny) sidey[nrow + idx - g.R - 1] = df;
 }
 
-// coef_l: the first Kx (Ky) sine coefficients of the bottom, top (left, right) ring sides,
+// ---- fixed-point form (doubles) ------------------------------------------------------------------
+//
+// Without a predictor: psi0 on the quarter lines is the lines' 1-D transforms of the spectrum's sums,
+// exact to FP64 rounding, and the rings' recurrence
+//   ring_l = r_l + A c_{l+1},  c_l = St . sides(ring_l),  r_l = get_bc(psi0_{l+1})
+// is unrolled: with T = St . sides(A), c0_m = St . sides(r_m),
+//   ring_l = r_l + sum_{m > l} A T^(m-l-1) c0_m
+// so two launches make every ring, where the recurrence takes two per level (at 200^2 x 5: 38 us of 10
+// launches).
+
+// Column sums of the spectrum, levels 1..:
+//   qcol[b-1][s][l] = sum_k sin(pi (k+1) I_s / nx) spec[b][k][l],  I_s = nx/4, 3nx/4
+// A block takes 16 rows l; each 16 threads take every 32nd group of eight k and sum the values of one
+// weight first (one FP64 addition a value); the groups' sums are added in order in shared memory.
+constexpr int kSumRows = 16, kSumGroups = 32;
+__global__ void __launch_bounds__(kSumRows * kSumGroups)
+k_spec_colsum(Geometry g, const double* __restrict__ w, double* __restrict__ qcol, int64_t qls) {
+  pdl_begin();
+  __shared__ double part[2][kSumGroups][kSumRows];
+  const int ncol = g.nx - 1, nrow = g.ny - 1, gr = threadIdx.x / kSumRows, r = threadIdx.x % kSumRows;
+  const int l = blockIdx.x * kSumRows + r, b = blockIdx.y + 1;
+  double a[6] = {0, 0, 0, 0, 0, 0};
+  if (l < nrow) {
+    const double* src = w + (int64_t)b * g.nG + l;
+#pragma unroll 4
+    for (int k0 = 8 * gr; k0 < ncol; k0 += 8 * kSumGroups) {
+      double v[6];
+#pragma unroll
+      for (int u = 0; u < 6; ++u) {
+        const int k = k0 + u + (u > 2);  // k + 1 = 1, 2, 3, 5, 6, 7 mod 8
+        v[u] = k < ncol ? src[(int64_t)k * nrow] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < 6; ++u) a[u] += v[u];
+    }
+  }
+  const double odd = 0.70710678118654752440 * ((a[0] + a[2]) - (a[3] + a[5])), even = a[1] - a[4];
+  part[0][gr][r] = odd + even;
+  part[1][gr][r] = odd - even;
+  __syncthreads();
+  if (gr >= 2 || l >= nrow) return;
+  double s = 0.0;
+#pragma unroll
+  for (int k = 0; k < kSumGroups; ++k) s += part[gr][k][r];
+  qcol[(b - 1) * qls + (int64_t)gr * nrow + l] = s;
+}
+
+// r_l: the values of get_bc from the quarter lines of the level above (their own array, q)
+__device__ __forceinline__ double ring0(const int4* pts, const double* q, int idx) {
+  const int4 p = pts[idx];
+  const double v = q[p.y];
+  return p.z >= 0 ? 0.125 * (v + q[p.w]) : 0.25 * v;
+}
+
+// coefficient j of side values f(i), i < len: sum_i St[j][i] f(i), by a block of kCoefThreads
+constexpr int kCoefThreads = 128;  // (few warps: an FP64 instruction takes a warp 16 cycles, reductions too)
+template <class F>
+__device__ __forceinline__ double block_coef(const double* row, int len, F f) {
+  constexpr int W = kCoefThreads / 32, U = 8;
+  __shared__ double red[W];
+  const int tid = threadIdx.x;
+  double s = 0.0;
+  for (int i0 = tid; i0 < len; i0 += U * kCoefThreads) {
+    double v[U], r[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * kCoefThreads;
+      v[u] = r[u] = 0.0;
+      if (i < len) {
+        r[u] = row[i];
+        v[u] = f(i);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i0 + u * kCoefThreads < len) s = fma(r[u], v[u], s);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((tid & 31) == 0) red[tid / 32] = s;
+  __syncthreads();
+  s = 0.0;
+#pragma unroll
+  for (int w = 0; w < W; ++w) s += red[w];
+  return s;
+}
+// its row of St and the first ring entry of its side
+struct CoefSide {
+  int row, first, len;
+};
+__device__ __forceinline__ CoefSide coef_side(const Geometry& g, int Kx, int Ky, int j) {
+  const int ncol = g.nx - 1, nrow = g.ny - 1;
+  if (j < 2 * Kx) return {(j < Kx ? j : j - Kx) * ncol, (j < Kx ? g.B : g.T) + 1, ncol};
+  const int jj = j - 2 * Kx;
+  return {Kx * ncol + (jj < Ky ? jj : jj - Ky) * nrow, (jj < Ky ? g.L : g.R) + 1, nrow};
+}
+
+// c0_m of the rings 1..L-2 (blockIdx.y + 1), one block per coefficient
+__global__ void __launch_bounds__(kCoefThreads)
+k_fx_coef(Geometry g, const int4* __restrict__ pts, const double* __restrict__ qfx, int64_t qls,
+          const double* __restrict__ St, int Kx, int Ky, double* __restrict__ coef) {
+  pdl_begin();
+  const int j = blockIdx.x, m = blockIdx.y + 1;
+  const CoefSide c = coef_side(g, Kx, Ky, j);
+  const double* q = qfx + m * qls;  // lines of level m + 1
+  const double s = block_coef(St + c.row, c.len, [&](int i) { return ring0(pts, q, c.first + i); });
+  if (threadIdx.x == 0) coef[(int64_t)m * (2 * Kx + 2 * Ky) + j] = s;
+}
+
+// every ring: 32 nodes of ring l = blockIdx.y per block, kRingWarps warps sharing the coefficients (the
+// coarsest level's is zero)
+constexpr int kRingWarps = 16;
+template <typename S>
+__global__ void __launch_bounds__(kRingWarps * 32)
+k_fx_rings(Geometry g, const int4* __restrict__ pts, const double* __restrict__ qfx, int64_t qls,
+           const double* __restrict__ Apow, const double* __restrict__ coef, int nK, S* __restrict__ rings,
+           double* __restrict__ side) {
+  pdl_begin();
+  __shared__ double part[kRingWarps][32];
+  const int w = threadIdx.x / 32, lane = threadIdx.x % 32, l = blockIdx.y;
+  const int idx = blockIdx.x * 32 + lane;
+  if (l == g.nlev - 1) {
+    if (w == 0 && idx < g.nbc) rings[(int64_t)l * g.nbc + idx] = S(0.0);
+    return;
+  }
+  double v = 0.0, h = 0.0;
+  if (idx < g.nbc) {
+    if (w == 0) v = ring0(pts, qfx + l * qls, idx);
+    // coefficients of the rings l+1..L-2 in a row, times A T^0, A T^1, ...
+    const int n = (g.nlev - 2 - l) * nK;
+    const double* a = Apow + idx;
+    const double* c = coef + (int64_t)(l + 1) * nK;
+    constexpr int U = 7;
+    int j = w;
+    for (; j + (U - 1) * kRingWarps < n; j += U * kRingWarps) {
+      double av[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) av[u] = a[(int64_t)(j + u * kRingWarps) * g.nbc];
+#pragma unroll
+      for (int u = 0; u < U; ++u) h = fma(av[u], __ldg(&c[j + u * kRingWarps]), h);
+    }
+    for (; j < n; j += kRingWarps) h = fma(a[(int64_t)j * g.nbc], __ldg(&c[j]), h);
+  }
+  part[w][lane] = h;
+  __syncthreads();
+  if (w != 0 || idx >= g.nbc) return;
+  h = 0.0;
+#pragma unroll
+  for (int k = 0; k < kRingWarps; ++k) h += part[k][lane];
+  v += h;
+  rings[(int64_t)l * g.nbc + idx] = S(v);
+  const int ncol = g.nx - 1, nrow = g.ny - 1;
+  double* sd = side + l * qls;
+  if (idx > g.B && idx < g.B + g.nx) sd[idx - g.B - 1] = v;
+  else if (idx > g.T && idx < g.T + g.nx) sd[ncol + idx - g.T - 1] = v;
+  else if (idx > g.L && idx < g.L + g.ny) sd[2 * ncol + idx - g.L - 1] = v;
+  else if (idx > g.R && idx < g.R + g.ny) sd[2 * ncol + nrow + idx - g.R - 1] = v;
+}
+
+// setup: T[i][j] = coefficient i of the ring Aring[j]; Apow[d+1][j] = sum_i T[i][j] Apow[d][i]
+__global__ void __launch_bounds__(kCoefThreads)
+k_coef_map(Geometry g, const double* __restrict__ AringT, const double* __restrict__ St, int Kx, int Ky,
+           double* __restrict__ T) {
+  const int i = blockIdx.x, j = blockIdx.y, nK = 2 * Kx + 2 * Ky;
+  const CoefSide c = coef_side(g, Kx, Ky, i);
+  const double* side = AringT + (int64_t)j * g.nbc + c.first;
+  const double s = block_coef(St + c.row, c.len, [&](int k) { return side[k]; });
+  if (threadIdx.x == 0) T[(int64_t)i * nK + j] = s;
+}
+__global__ void k_coef_next(int nbc, int nK, const double* __restrict__ T, const double* __restrict__ A,
+                            double* __restrict__ out) {
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
+  if (idx >= nbc) return;
+  double s = 0.0;
+  for (int i = 0; i < nK; ++i) s = fma(T[(int64_t)i * nK + j], A[(int64_t)i * nbc + idx], s);
+  out[(int64_t)j * nbc + idx] = s;
+}
+
+// FP32 form: coef_l, the first Kx (Ky) sine coefficients of the bottom, top (left, right) ring sides,
 // coef[j] = sum_i St[j][i] side_i (S convention, 2 sin).  One block of kCoefThreads per
 // coefficient (nK blocks spread the FP64 work over the SMs), a strided sum per thread, then a
 // fixed-order tree in shared memory; FP64.
-constexpr int kCoefThreads = 256;
 __global__ void __launch_bounds__(kCoefThreads)
 k_ring_coef(Geometry g, const double* __restrict__ ringd, const double* __restrict__ St, int Kx, int Ky,
             double* __restrict__ coef) {
   pdl_begin();
-  __shared__ double red[kCoefThreads];
-  const int j = blockIdx.x, tid = threadIdx.x;
-  const int nK = 2 * Kx + 2 * Ky;
-  if (j >= nK) return;
-  const int ncol = g.nx - 1, nrow = g.ny - 1;
-  const double* row;
-  const double* side;
-  int len;
-  if (j < 2 * Kx) {
-    const int k = j < Kx ? j : j - Kx;
-    row = St + (int64_t)k * ncol;
-    side = ringd + (j < Kx ? g.B : g.T) + 1;
-    len = ncol;
-  } else {
-    const int jj = j - 2 * Kx;
-    const int k = jj < Ky ? jj : jj - Ky;
-    row = St + (int64_t)Kx * ncol + (int64_t)k * nrow;
-    side = ringd + (jj < Ky ? g.L : g.R) + 1;
-    len = nrow;
-  }
-  double s = 0.0;
-  for (int i = tid; i < len; i += kCoefThreads) s = fma(row[i], side[i], s);
-  red[tid] = s;
-  __syncthreads();
-#pragma unroll
-  for (int o = kCoefThreads / 2; o > 0; o >>= 1) {
-    if (tid < o) red[tid] += red[tid + o];
-    __syncthreads();
-  }
-  if (tid == 0) coef[j] = red[0];
+  const int j = blockIdx.x;
+  const CoefSide c = coef_side(g, Kx, Ky, j);
+  const double* side = ringd + c.first;
+  const double s = block_coef(St + c.row, c.len, [&](int i) { return side[i]; });
+  if (threadIdx.x == 0) coef[j] = s;
 }
 
 template <int P>
@@ -341,27 +495,64 @@ size_t line_smem() {
   return (size_t)kLines * Shape<float, P, 32>::kStride * sizeof(float);
 }
 
-// harmonic decay g_k(J) = sinh(th (m-1-J)) / (2 n sinh(th m)), 2 cosh th = 4 - 2 cos(pi (k+1)/n),
-// for J = 0..m-2, written stably with exponentials
-void decay_table(int n, int m, int K, std::vector<double>& out) {
-  const double pi = 3.14159265358979323846;
-  out.assign((size_t)K * (m - 1), 0.0);
-  for (int k = 0; k < K; ++k) {
-    const double th = std::acosh(2.0 - std::cos(pi * (k + 1) / n));
-    const double den = 1.0 - std::exp(-2.0 * th * m);
-    for (int J = 0; J < m - 1; ++J) {
-      const double num = std::exp(-th * (J + 1)) * (1.0 - std::exp(-2.0 * th * (m - 1 - J)));
-      out[(size_t)k * (m - 1) + J] = num / den / (2.0 * n);
-    }
+// sin(pi m / n), the angle reduced in integers to at most pi/2 (a product of modes and nodes reaches
+// hundreds of periods, where the rounding of the angle alone would be 1e-13)
+double sin_pi(int64_t m, int n) {
+  m %= 2 * n;
+  const bool neg = m >= n;
+  if (neg) m -= n;
+  const double s = std::sin(3.14159265358979323846 * (double)std::min<int64_t>(m, n - m) / n);
+  return neg ? -s : s;
+}
+
+// th with 2 cosh th = 4 - 2 cos(pi k / n): cosh th = 1 + e, e = 2 sin^2(pi k / 2n)
+double decay_rate(int k, int n) {
+  const double s = std::sin(3.14159265358979323846 * k / (2.0 * n)), e = 2.0 * s * s;
+  return std::log1p(e + std::sqrt(e * (2.0 + e)));
+}
+
+// Response at distance J + 1 from a side to one of its mode coefficients (per 2 sin along the side), from the solves' own multipliers,
+//   out[k][J] = 1/4 sum_l mult(k, l) sin(pi (l+1)/m) sin(pi (l+1)(J+1)/m),  J = 0..m-2.
+// In exact arithmetic this is sinh(th (m-1-J)) / (2 n sinh(th m)), 2 cosh th = 4 - 2 cos(pi (k+1)/n); the
+// multipliers carry the cancellation of their cosines (1e-12 of the smallest eigenvalue at 512 cells),
+// which the rings have to share for the two Vort2Flux orders to agree to rounding.  sn: sin(pi i / m).
+__global__ void k_decay(int m, const double* __restrict__ mult, int64_t mode_stride, int64_t sum_stride,
+                        const double* __restrict__ sn, double* __restrict__ out) {
+  const int J = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
+  if (J >= m - 1) return;
+  const double* mk = mult + k * mode_stride;
+  double s = 0.0;
+  int a = 0;  // (l+1)(J+1) mod 2m
+  for (int l = 0; l < m - 1; ++l) {
+    a += J + 1;
+    if (a >= 2 * m) a -= 2 * m;
+    s = fma(mk[l * sum_stride] * sn[l + 1], sn[a], s);
   }
+  out[(int64_t)k * (m - 1) + J] = 0.25 * s;
+}
+
+cudaError_t decay_table(int m, int K, const double* mult, int64_t mode_stride, int64_t sum_stride,
+                        std::vector<double>& out) {
+  out.assign((size_t)K * (m - 1), 0.0);
+  std::vector<double> sn(2 * m);
+  for (int i = 0; i < 2 * m; ++i) sn[i] = sin_pi(i, m);
+  double* d = nullptr;  // sines, table
+  cudaError_t e = cudaMalloc(&d, sizeof(double) * (sn.size() + out.size()));
+  if (e != cudaSuccess) return e;
+  e = cudaMemcpy(d, sn.data(), sizeof(double) * sn.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    k_decay<<<dim3((m - 1 + 63) / 64, K), 64>>>(m, mult, mode_stride, sum_stride, d, d + sn.size());
+    e = cudaMemcpy(out.data(), d + sn.size(), sizeof(double) * out.size(), cudaMemcpyDeviceToHost);
+  }
+  cudaFree(d);
+  return e;
 }
 
 // modes kept for a side along an axis of n cells whose nearest quarter-line node is d cells
 // away: the smallest K with 2 sum_{k >= K} exp(-th_k d) below 1e-17
 int modes_kept(int n, int d) {
-  const double pi = 3.14159265358979323846;
   std::vector<double> e(n - 1);
-  for (int k = 0; k < n - 1; ++k) e[k] = std::exp(-std::acosh(2.0 - std::cos(pi * (k + 1) / n)) * d);
+  for (int k = 0; k < n - 1; ++k) e[k] = std::exp(-decay_rate(k + 1, n) * d);
   double tail = 0.0;
   int K = n - 1;
   for (int k = n - 2; k >= 0; --k) {
@@ -473,11 +664,58 @@ cudaError_t v2f_ring_coef(const Geometry& g, const RingPlan& rp, int l, cudaStre
                   (const double*)rp.St, rp.Kx, rp.Ky, rp.coef + (int64_t)l * rp.nK);
 }
 
+cudaError_t v2f_fx_colsum(const Geometry& g, const RingPlan& rp, const double* w, cudaStream_t s) {
+  return launch_k(k_spec_colsum, dim3((g.ny - 1 + kSumRows - 1) / kSumRows, g.nlev - 1), dim3(kSumRows * kSumGroups), 0,
+                  s, g, w, rp.qfx + 2 * (g.nx - 1), rp.qls);
+}
+
+template <typename S>
+cudaError_t v2f_fx_rings(const Geometry& g, const RingPlan& rp, S* rings, cudaStream_t s) {
+  if (g.nlev > 2)
+    CE_V(launch_k(k_fx_coef, dim3(rp.nK, g.nlev - 2), dim3(kCoefThreads), 0, s, g, (const int4*)rp.pts,
+                  (const double*)rp.qfx, rp.qls, (const double*)rp.St, rp.Kx, rp.Ky, rp.coef));
+  return launch_k(k_fx_rings<S>, dim3((g.nbc + 31) / 32, g.nlev), dim3(kRingWarps * 32), 0, s, g,
+                  (const int4*)rp.pts, (const double*)rp.qfx, rp.qls, (const double*)rp.Apow, (const double*)rp.coef,
+                  rp.nK, rings, rp.side);
+}
+template cudaError_t v2f_fx_rings<double>(const Geometry&, const RingPlan&, double*, cudaStream_t);
+template cudaError_t v2f_fx_rings<df64>(const Geometry&, const RingPlan&, df64*, cudaStream_t);
+
+cudaError_t RingPlan::build_fx(const Geometry& g, cudaStream_t s) {
+  if (Apow) return cudaSuccess;
+  const int L = g.nlev;
+  auto zero = [&](double*& dst, int64_t n) -> cudaError_t {
+    CE_V(cudaMalloc(&dst, sizeof(double) * n));
+    return cudaMemset(dst, 0, sizeof(double) * n);
+  };
+  auto sines = [&](double*& dst, int n) -> cudaError_t {
+    std::vector<double> sn(n - 1);
+    for (int i = 1; i < n; ++i) sn[i - 1] = sin_pi(i, n);
+    CE_V(cudaMalloc(&dst, sizeof(double) * (n - 1)));
+    return cudaMemcpy(dst, sn.data(), sizeof(double) * (n - 1), cudaMemcpyHostToDevice);
+  };
+  const int64_t one = (int64_t)nK * g.nbc;
+  CE_V(zero(qfx, (L - 1) * qls));
+  CE_V(zero(side, (L - 1) * qls));
+  CE_V(sines(sinx, g.nx));
+  CE_V(sines(siny, g.ny));
+  CE_V(zero(Apow, std::max(L - 2, 1) * one));
+  if (L < 3) return cudaSuccess;
+  CE_V(cudaMemcpyAsync(Apow, Aring, sizeof(double) * one, cudaMemcpyDeviceToDevice, s));
+  double* T = nullptr;
+  CE_V(cudaMalloc(&T, sizeof(double) * nK * nK));
+  k_coef_map<<<dim3(nK, nK), kCoefThreads, 0, s>>>(g, Aring, St, Kx, Ky, T);
+  for (int d = 1; d < L - 2; ++d)
+    k_coef_next<<<dim3((g.nbc + 127) / 128, nK), 128, 0, s>>>(g.nbc, nK, T, Apow + (d - 1) * one, Apow + d * one);
+  const cudaError_t e = cudaGetLastError(), e2 = cudaStreamSynchronize(s);
+  cudaFree(T);
+  return e != cudaSuccess ? e : e2;
+}
+
 // Host tables: truncation, St, Aring and the quarter-line nodes of each ring entry.
-cudaError_t RingPlan::build(const Geometry& g) {
+cudaError_t RingPlan::build(const Geometry& g, const double* mult) {
   const int nx = g.nx, ny = g.ny, ncol = nx - 1, nrow = ny - 1, L = g.nlev;
   const int nx4 = nx / 4, ny4 = ny / 4;
-  const double pi = 3.14159265358979323846;
   Kx = modes_kept(nx, ny4);  // bottom / top modes, nearest quarter-line node ny/4 cells away
   Ky = modes_kept(ny, nx4);
   nK = 2 * Kx + 2 * Ky;
@@ -485,13 +723,13 @@ cudaError_t RingPlan::build(const Geometry& g) {
   nchunk = (ncol + kColChunk - 1) / kColChunk;
   std::vector<double> st((size_t)Kx * ncol + (size_t)Ky * nrow);
   for (int k = 0; k < Kx; ++k)
-    for (int i = 0; i < ncol; ++i) st[(size_t)k * ncol + i] = 2.0 * std::sin(pi * (double)(k + 1) * (i + 1) / nx);
+    for (int i = 0; i < ncol; ++i) st[(size_t)k * ncol + i] = 2.0 * sin_pi((int64_t)(k + 1) * (i + 1), nx);
   for (int k = 0; k < Ky; ++k)
     for (int j = 0; j < nrow; ++j)
-      st[(size_t)Kx * ncol + (size_t)k * nrow + j] = 2.0 * std::sin(pi * (double)(k + 1) * (j + 1) / ny);
+      st[(size_t)Kx * ncol + (size_t)k * nrow + j] = 2.0 * sin_pi((int64_t)(k + 1) * (j + 1), ny);
   std::vector<double> gx, hy;
-  decay_table(nx, ny, Kx, gx);  // [k][J]: bottom-side mode k at row J
-  decay_table(ny, nx, Ky, hy);  // [l][I]: left-side mode l at column I
+  CE_V(decay_table(ny, Kx, mult, nrow, 1, gx));  // [k][J]: bottom-side mode k at row J
+  CE_V(decay_table(nx, Ky, mult, 1, nrow, hy));  // [l][I]: left-side mode l at column I
   auto stx = [&](int k, int I) { return st[(size_t)k * ncol + I]; };
   auto sty = [&](int k, int J) { return st[(size_t)Kx * ncol + (size_t)k * nrow + J]; };
   // harmonic response at node (J, I) per coefficient, accumulated with weight wt
@@ -574,10 +812,12 @@ cudaError_t RingPlan::build(const Geometry& g) {
 
 void RingPlan::release() {
   for (void* p : {(void*)St, (void*)Aring, (void*)pts, (void*)vrow, (void*)ucolp, (void*)ucol, (void*)qline,
-                  (void*)sidex, (void*)sidey, (void*)ringd, (void*)dring, (void*)coef})
+                  (void*)sidex, (void*)sidey, (void*)ringd, (void*)dring, (void*)coef, (void*)qfx, (void*)side,
+                  (void*)sinx, (void*)siny, (void*)Apow})
     if (p) cudaFree(p);
   St = nullptr; Aring = nullptr; pts = nullptr; vrow = nullptr; ucolp = nullptr; ucol = nullptr; qline = nullptr;
   sidex = nullptr; sidey = nullptr; ringd = nullptr; dring = nullptr; coef = nullptr;
+  qfx = side = sinx = siny = Apow = nullptr;
 }
 
 }  // namespace ib

@@ -45,8 +45,10 @@ extern "C" {
  * every mode) */
 #define IB_PREC_FP64 0   /* FP64 throughout (the reference's arithmetic); the sine transforms run in 64-bit
                             block fixed point, with less rounding error than in FP64 */
-#define IB_PREC_MIXED 1  /* FP32 sine transforms refined with float-float residuals (refine_sweeps);
-                            state and stencils in float-float (two-float) arithmetic */
+#define IB_PREC_MIXED 1  /* state and stencils in float-float (two-float) arithmetic; solves by the
+                            64-bit block fixed-point transforms, or (refine_sweeps 1, IBGB300_DST, and
+                            Vort2Flux in an order set to IB_V2F_SEQUENTIAL) by FP32 transforms refined
+                            with float-float residuals */
 #define IB_PREC_MIXED_TC 2  /* as IB_PREC_MIXED, with every sine transform a BF16x3 split-precision
                                GEMM against the sine matrix on the tensor cores (FP32 accumulation);
                                both axes a multiple of 128 cells; Vort2Flux level by level */
@@ -89,9 +91,10 @@ typedef struct ib_problem {
   int32_t precision;            /* IB_PREC_* */
   int32_t device;               /* CUDA device ordinal */
   int32_t history_capacity;     /* steps of C_D / C_L kept on the device (0 -> 4096) */
-  int32_t refine_sweeps;        /* IB_PREC_MIXED: residual sweeps per solve: 1 or 2 everywhere, or
+  int32_t refine_sweeps;        /* IB_PREC_MIXED: residual sweeps per FP32 solve: 1 or 2 everywhere, or
                                    0 (default): 2, except 1 for the Vort2Flux solves of the third
-                                   and coarser levels (they only feed boundary rings) */
+                                   and coarser levels (they only feed boundary rings); with 0 or 2
+                                   most solves are in fixed point, without sweeps */
   int32_t scheme;               /* IB_SCHEME_* (0: CNAB) */
   int32_t rkc_stages;           /* IB_SCHEME_RKC: stages s >= 2, or 0: the fewest whose stability
                                    interval covers 1.5 x dt x the finest level's viscous spectral
@@ -126,8 +129,8 @@ int ib_get_state(ib_handle* h, double* gamma, double* q, double* psi, double* no
  * and, for moving bodies, the previous step's Fb; FP64 in the column-major layouts above after
  * a 56-byte header (magic "IBGB300C", int32 version 1, nx, ny, nlevels, npoints, moving flag,
  * two zeros, double t, int64 steps).  Loading checks that the handle's grid, levels, points and motion match.  An FP64
- * handle restarts to the same bits as an uninterrupted run; a mixed-precision one restarts its
- * solves' predictors from zero and agrees to the refinement tolerance. */
+ * handle restarts to the same bits as an uninterrupted run; a mixed-precision one restarts the
+ * predictors of its FP32 solves from zero and agrees to the refinement tolerance. */
 int ib_checkpoint_save(ib_handle* h, const char* path);
 int ib_checkpoint_load(ib_handle* h, const char* path);
 
@@ -174,14 +177,15 @@ int ib_set_cg_options(ib_handle* h, double tol, int32_t maxiter, int32_t warm_st
 #define IB_PC_SCHUR_REF 1
 int ib_set_cg_preconditioner(ib_handle* h, int32_t mode, int32_t refresh_steps);
 
-/* Order of the mixed-precision Vort2Flux (fluid-ops.jl:438-472 solves the levels coarse to fine,
- * each taking its boundary ring from the coarser solution).  IB_V2F_LEVELS finds every level's
- * ring first (harmonic ring transfer) and solves all levels in one batch; IB_V2F_SEQUENTIAL
- * keeps the reference's level order; IB_V2F_AUTO (the default) takes LEVELS up to 2^20 cells per
- * level where the grid has one-warp line passes.  The handle's step graphs are captured again;
- * a handle in an ensemble must not change it (the ensemble holds its own capture).  FP64
- * handles keep the reference order (accepted, no effect).  IB_ERR_UNSUPPORTED for LEVELS on a
- * grid without one-warp line passes. */
+/* Order of Vort2Flux (fluid-ops.jl:438-472 solves the levels coarse to fine, each taking its
+ * boundary ring from the coarser solution).  IB_V2F_LEVELS finds every level's ring first
+ * (harmonic ring transfer) and solves all levels in one batch; IB_V2F_SEQUENTIAL keeps the
+ * reference's level order; IB_V2F_AUTO (the default) takes LEVELS from four levels on, and with
+ * three up to 2^17 cells per level (solves by FP32 transforms: as the autotuner measured).  The
+ * orders agree to rounding.  The handle's step graphs are captured again; a handle in an ensemble
+ * must not change it (the ensemble holds its own capture).  A mixed-precision handle set to
+ * SEQUENTIAL runs Vort2Flux with the refined FP32 transforms.  IB_ERR_UNSUPPORTED for LEVELS on a
+ * mixed-precision handle whose grid has no one-warp line passes. */
 #define IB_V2F_AUTO 0
 #define IB_V2F_LEVELS 1
 #define IB_V2F_SEQUENTIAL 2

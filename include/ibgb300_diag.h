@@ -21,7 +21,8 @@ typedef struct ib_info {
   int64_t device_bytes;      /* device memory held by the handle */
   double setup_ms;           /* wall time of ib_create (tables, delta weights, Schur inverse) */
   int32_t vort2flux_order;   /* the order in effect: IB_V2F_LEVELS or IB_V2F_SEQUENTIAL */
-  int32_t transform_form;    /* the sine-transform passes in effect: IB_FORM_* */
+  int32_t transform_form;    /* the sine-transform passes in effect (of a mixed-precision handle: its
+                                FP32 passes): IB_FORM_* */
   int32_t scheme;            /* IB_SCHEME_* */
   int32_t rkc_stages;        /* stages of the Runge-Kutta-Chebyshev scheme (0 for CNAB) */
   int32_t sm_count;          /* streaming multiprocessors of the handle's device */
@@ -39,7 +40,8 @@ int ib_get_info(ib_handle* h, ib_info* info);
  * level-1 Vort2Flux) for transform form IB_FORM_*, Vort2Flux order (levels = 1: all levels in
  * one batch) and warp y-pass occupancy (y8 = 1: the variant compiled for 8 resident blocks per
  * SM), -1 where the candidate was not tried; *chosen = the index in effect (-1 when the tuner
- * did not run: IBGB300_AUTOTUNE=0 or every choice pinned).  No counterpart in the reference,
+ * did not run: IBGB300_AUTOTUNE=0 or every choice pinned).  The candidates are the FP32 passes of
+ * mixed-precision handles; their fixed-point solves have nothing to choose.  No counterpart in the reference,
  * whose FFTW plans are chosen by FFTW's own EXHAUSTIVE planner (fluid-ops.jl:25). */
 int ib_get_autotune(ib_handle* h, double* ms /* [12] */, int32_t* chosen);
 
