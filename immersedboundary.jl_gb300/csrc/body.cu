@@ -206,7 +206,7 @@ __global__ void k_unit_columns(double* f, int nf, int col0, int ncols) {
 // update_stress! (states.jl:53-84): one block per body, fixed-order block reduction.
 __global__ void k_update_stress(const double* __restrict__ fb, int nb, const int* __restrict__ body_start,
                                 const double* __restrict__ ds, double h, double dt, double* __restrict__ out,
-                                double* __restrict__ stress) {
+                                double* __restrict__ stress, double* __restrict__ mirror) {
   pdl_begin();
   __shared__ double sx[256], sy[256];
   const int body = blockIdx.x;
@@ -217,8 +217,13 @@ __global__ void k_update_stress(const double* __restrict__ fb, int nb, const int
     ax += fx;
     ay += fy;
     if (stress) {
-      stress[2 * s0 + p] = fx / ds[s0 + p];
-      stress[2 * s0 + n + p] = fy / ds[s0 + p];
+      const double tx = fx / ds[s0 + p], ty = fy / ds[s0 + p];
+      stress[2 * s0 + p] = tx;
+      stress[2 * s0 + n + p] = ty;
+      if (mirror) {
+        mirror[2 * gridDim.x + 2 * s0 + p] = tx;
+        mirror[2 * gridDim.x + 2 * s0 + n + p] = ty;
+      }
     }
   }
   sx[threadIdx.x] = ax;
@@ -234,6 +239,10 @@ __global__ void k_update_stress(const double* __restrict__ fb, int nb, const int
   if (threadIdx.x == 0) {
     out[2 * body] = 2 * sx[0];
     out[2 * body + 1] = 2 * sy[0];
+    if (mirror) {
+      mirror[2 * body] = 2 * sx[0];
+      mirror[2 * body + 1] = 2 * sy[0];
+    }
   }
 }
 
@@ -306,8 +315,9 @@ cudaError_t unit_columns(double* f, int nf, int col0, int ncols, cudaStream_t s)
 }
 
 cudaError_t update_stress_hd(const double* fb, int nb, int nbodies, const int* body_start, const double* ds, double h,
-                             double dt, double* cd_cl_out, double* stress_out, cudaStream_t s) {
-  return launch_k(k_update_stress, dim3(nbodies), dim3(256), 0, s, fb, nb, body_start, ds, h, dt, cd_cl_out, stress_out);
+                             double dt, double* cd_cl_out, double* stress_out, double* mirror, cudaStream_t s) {
+  return launch_k(k_update_stress, dim3(nbodies), dim3(256), 0, s, fb, nb, body_start, ds, h, dt, cd_cl_out, stress_out,
+                  mirror);
 }
 
 template cudaError_t reg_gather<double>(const Geometry&, const double*, const double*, const int*, const double*, int,

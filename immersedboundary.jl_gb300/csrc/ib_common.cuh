@@ -351,9 +351,11 @@ cudaError_t unit_scatter_rot(const Geometry& g, const int* body_idx, const doubl
                              int ncols, T* gam, cudaStream_t s);
 
 // forces -> coefficients (update_stress!): out[2b] = C_D, out[2b+1] = C_L of body b;
-// stress (optional) = per-body column-major (n x 2) surface stress blocks
+// stress (optional) = per-body column-major (n x 2) surface stress blocks; mirror (optional, host
+// memory): out, then stress, once more
 cudaError_t update_stress_hd(const double* fb, int nb, int nbodies, const int* body_start, const double* ds,
-                             double h, double dt, double* cd_cl_out, double* stress_out, cudaStream_t s);
+                             double h, double dt, double* cd_cl_out, double* stress_out, double* mirror,
+                             cudaStream_t s);
 
 // ----------------------------------------------------------------------------------------------
 // moving bodies and the Schur CG (cg.cu)

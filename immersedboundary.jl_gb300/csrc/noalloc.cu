@@ -3,8 +3,8 @@
 // Some callers cannot call cudaMalloc in the loop that solves: programs whose device memory is
 // owned by another allocator or memory pool (a Julia or Python host that hands this library
 // only the arrays it already owns), and time-critical loops that must not pay for an
-// allocation's implicit synchronisation of the whole device.  ib_op_laplacian_inv allocates its
-// work buffer on every call; this variant keeps that work buffer in a fixed array compiled into
+// allocation's implicit synchronisation of the whole device.  ib_op_laplacian_inv allocates a
+// work buffer on its first and on its largest calls; this variant has it in a fixed array compiled into
 // the library instead, and runs the same transform kernels as ib_op_laplacian_inv on the same
 // handle.
 //

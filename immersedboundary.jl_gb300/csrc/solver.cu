@@ -109,6 +109,7 @@ struct ib_handle {
   int *body_start = nullptr, *body_idx = nullptr;
   double *bmat = nullptr, *binv_cm = nullptr, *binv_rm = nullptr, *ftmp = nullptr;
   double *cdcl = nullptr, *stress = nullptr, *hist = nullptr;
+  double* h_stress = nullptr;  // host copy of cdcl, then stress, written by the same kernel
   int hist_cap = 4096;
   int* d_counter = nullptr;
   // moving bodies (IB_MOTION_PRESCRIBED)
@@ -158,6 +159,8 @@ struct ib_handle {
   int warm_start = IB_WARM_PREVIOUS;
   std::vector<int> cg_iters;
   std::vector<double> cg_res;
+  // Host memory that kernels write: a call that has waited for its stream reads it without a copy (a copy
+  // to pageable memory and its wait took 8 us of a 128^2 step's 270, the three of ib_get_stress 25).
   int* status = nullptr;  // [0] out of grid, [1] non-finite flux, [2] singular Schur matrix, [3] pipeline timeout
   int* d_box = nullptr;   // face box of the body windows (E^T scatter scratch)
   bool box_ready = false; // static bodies: d_box computed once at setup
@@ -172,6 +175,9 @@ struct ib_handle {
   double setup_ms = 0.0;
   std::string err;
   std::vector<void*> allocs;
+  std::mutex op_mu;              // operator calls' work array (OpWork)
+  double* op_work = nullptr;
+  int64_t op_cap = 0;
 
   template <typename T>
   cudaError_t alloc(T** p, size_t count) {
@@ -667,7 +673,8 @@ cudaError_t enqueue_trial(ib_handle* h, int p) {
 cudaError_t enqueue_stress(ib_handle* h) {
   ib::Range nvtx_range("stress");
   cudaStream_t s = h->stream;
-  CE(update_stress_hd(h->fb, h->nb, h->nbodies, h->body_start, h->ds, h->g.h, h->dt, h->cdcl, h->stress, s));
+  CE(update_stress_hd(h->fb, h->nb, h->nbodies, h->body_start, h->ds, h->g.h, h->dt, h->cdcl, h->stress,
+                      h->h_stress, s));
   return launch_k(k_hist_append, dim3(1), dim3(64), 0, s, (const double*)h->cdcl, h->hist, h->hist_cap, 2 * h->nbodies,
                   h->d_counter);
 }
@@ -837,9 +844,8 @@ cudaError_t schur_apply(ib_handle* h, const double* z, double* out) {
 }
 
 int check_status(ib_handle* h) {
-  int st[4] = {0, 0, 0, 0};
-  CK(cudaMemcpyAsync(st, h->status, sizeof(st), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
+  const volatile int* st = h->status;
   if (st[0]) return fail(h, IB_ERR_BODY_OUT_OF_GRID, "body point within 7 cells of the finest-grid edge");
   if (st[1]) return fail(h, IB_ERR_NONFINITE, "infinite flux");
   if (st[2]) return fail(h, IB_ERR_SINGULAR, "zero or non-finite pivot in the Schur matrix");
@@ -1053,7 +1059,10 @@ void destroy_handle(ib_handle* h) {
   if (h->h_cgout) cudaFreeHost(h->h_cgout);
   if (h->loop_stream) cudaStreamDestroy(h->loop_stream);
   for (void* p : h->allocs) cudaFree(p);
+  if (h->op_work) cudaFree(h->op_work);
   if (h->h_q0) cudaFreeHost(h->h_q0);
+  if (h->status) cudaFreeHost(h->status);
+  if (h->h_stress) cudaFreeHost(h->h_stress);
   if (h->h_sc) cudaFreeHost(h->h_sc);
   delete h->mlp;
   h->axx.release();
@@ -1192,7 +1201,7 @@ int learn_validate_schur(ib_handle* h) {
   int rows = 0;
   int* status_save = reinterpret_cast<int*>(save + npw + nrw);  // the 4 status flags
   e = m.heldout(q, t, kRows, &rows);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(status_save, h->status, 4 * sizeof(int), cudaMemcpyDeviceToDevice, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(status_save, h->status, 4 * sizeof(int), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(save, h->Pw, sizeof(double) * npw, cudaMemcpyDeviceToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(save + npw, h->rings_w, sizeof(double) * nrw, cudaMemcpyDeviceToDevice, s);
   for (int j = 0; j < rows && e == cudaSuccess; ++j) {
@@ -1204,7 +1213,7 @@ int learn_validate_schur(ib_handle* h) {
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(h->Pw, save, sizeof(double) * npw, cudaMemcpyDeviceToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(h->rings_w, save + npw, sizeof(double) * nrw, cudaMemcpyDeviceToDevice, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(h->status, status_save, 4 * sizeof(int), cudaMemcpyDeviceToDevice, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(h->status, status_save, 4 * sizeof(int), cudaMemcpyDeviceToHost, s);
   std::vector<double> hd(3 * (size_t)std::max(rows, 1));
   if (e == cudaSuccess && rows > 0)
     e = cudaMemcpyAsync(hd.data(), dots, sizeof(double) * 3 * rows, cudaMemcpyDeviceToHost, s);
@@ -1934,7 +1943,7 @@ int ib_create(const ib_problem* p, ib_handle** out) {
       if (std::strcmp(env, "levels") == 0) { h->v2f_levels = lv_ok; pin_v2f = true; }
     }
   }
-  AL(h->status, 4); AL(h->d_counter, 1); AL(h->d_box, 4);
+  AL(h->d_counter, 1); AL(h->d_box, 4);
   if (h->scheme == IB_SCHEME_RKC) {
     AL(h->rkY[0], L * nG); AL(h->rkY[1], L * nG); AL(h->rkF0, L * nG);
     AL(h->d_alpha_rkc, L); AL(h->d_fac_rkc, L);
@@ -1948,6 +1957,19 @@ int ib_create(const ib_problem* p, ib_handle** out) {
   AL(h->cdcl, 2 * (h->nbodies > 0 ? h->nbodies : 1));
   AL(h->hist, (int64_t)h->hist_cap * 2 * (h->nbodies > 0 ? h->nbodies : 1));
   AL(h->stress, h->nf);
+  {
+    const size_t n = sizeof(double) * (2 * (h->nbodies > 0 ? h->nbodies : 1) + h->nf);
+    if ((e = cudaMallocHost(&h->status, 4 * sizeof(int))) != cudaSuccess) {
+      h->status = nullptr;
+      return bail(fail(h, IB_ERR_CUDA, "pinned status", e));
+    }
+    std::memset(h->status, 0, 4 * sizeof(int));
+    if ((e = cudaMallocHost(&h->h_stress, n)) != cudaSuccess) {
+      h->h_stress = nullptr;
+      return bail(fail(h, IB_ERR_CUDA, "pinned stress", e));
+    }
+    std::memset(h->h_stress, 0, n);
+  }
   if ((e = cudaMallocHost(&h->h_q0, sizeof(double) * kQ0Slots * (2 * L + 6 * (h->nbodies + 1)))) != cudaSuccess) {
     h->h_q0 = nullptr;
     return bail(fail(h, IB_ERR_CUDA, "pinned staging", e));
@@ -2426,11 +2448,9 @@ int ib_get_stress(ib_handle* h, double* cd, double* cl, double* fb_surface) {
   CK(dev_guard_.err);
   const int nbd = h->nbodies;
   if (nbd == 0) return IB_OK;
-  std::vector<double> v(2 * nbd);
-  CK(cudaMemcpyAsync(v.data(), h->cdcl, sizeof(double) * 2 * nbd, cudaMemcpyDeviceToHost, h->stream));
-  if (fb_surface && h->nf)
-    CK(cudaMemcpyAsync(fb_surface, h->stress, sizeof(double) * h->nf, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
+  const double* v = h->h_stress;
+  if (fb_surface && h->nf) std::memcpy(fb_surface, v + 2 * nbd, sizeof(double) * h->nf);
   for (int b = 0; b < nbd; ++b) {
     if (cd) cd[b] = v[2 * b];
     if (cl) cl[b] = v[2 * b + 1];
@@ -2570,16 +2590,57 @@ int ib_profile_steps(ib_handle* h, int32_t n, const double* t, const double* uv,
   CK(cudaStreamSynchronize(s));       \
   return IB_OK;
 
+}  // extern "C"
+
+namespace {
+// Work array of one operator call.  Up to the size of a step's work array it is the handle's own, kept
+// from call to call (allocating and releasing it made a 64 x 48 Poisson call 34 us instead of 29) and locked
+// until the call's kernels have finished, since calls from several threads may share a handle; larger
+// ones are allocated for the call.
+struct OpWork {
+  ib_handle* h;
+  std::unique_lock<std::mutex> lock;
+  void* own = nullptr;
+
+  explicit OpWork(ib_handle* handle) : h(handle), lock(handle->op_mu) {}
+  cudaError_t get(double** p, int64_t n) {
+    const int64_t most = std::max<int64_t>((int64_t)h->g.nlev * h->g.nG, (int64_t)h->g.nlev * h->g.nbc);
+    if (n > most) {
+      const cudaError_t e = cudaMalloc(&own, sizeof(double) * n);
+      *p = static_cast<double*>(own);
+      return e;
+    }
+    if (n > h->op_cap) {
+      if (h->op_work) cudaFree(h->op_work);
+      h->op_work = nullptr;
+      h->op_cap = 0;
+      const cudaError_t e = cudaMalloc(&h->op_work, sizeof(double) * n);
+      if (e != cudaSuccess) return e;
+      h->op_cap = n;
+    }
+    *p = h->op_work;
+    return cudaSuccess;
+  }
+  void done() {
+    cudaStreamSynchronize(h->stream);
+    if (own) cudaFree(own);
+    own = nullptr;
+  }
+};
+}  // namespace
+
+extern "C" {
+
 int ib_op_dst2(ib_handle* h, int32_t batch, const double* in, double* out) {
   OP_BEGIN();
   if (batch < 1) return IB_ERR_INVALID;
+  OpWork work(h);
   double* w;
-  CK(cudaMalloc(&w, sizeof(double) * batch * g.nG));
+  CK(work.get(&w, (int64_t)batch * g.nG));
   // RODFT00 in both dimensions = 4 F_y F_x (F: the half-scaled transform of dstfx.cu)
   cudaError_t e = fx_fwd<double>(g, h->axx.d, in, w, batch, nullptr, s);
   if (e == cudaSuccess) e = fx_ypass(g, h->axy.d, w, out, batch, nullptr, 0, 2, s);
-  cudaStreamSynchronize(s);
-  cudaFree(w);
+  work.done();
   CK(e);
   OP_END();
 }
@@ -2602,11 +2663,11 @@ int ib_op_sine_lines_tc(ib_handle* h, int32_t axis, int32_t rows, const float* i
 int ib_op_laplacian_inv(ib_handle* h, int32_t batch, const double* b, double* x) {
   OP_BEGIN();
   if (batch < 1) return IB_ERR_INVALID;
+  OpWork work(h);
   double* w;
-  CK(cudaMalloc(&w, sizeof(double) * batch * g.nG));
+  CK(work.get(&w, (int64_t)batch * g.nG));
   cudaError_t e = poisson_fx<double>(h, b, x, batch, nullptr, op_lap(h), nullptr, w);
-  cudaStreamSynchronize(s);
-  cudaFree(w);
+  work.done();
   CK(e);
   OP_END();
 }
@@ -2711,11 +2772,11 @@ int ib_op_nonlinear(ib_handle* h, int32_t lev, const double* q, double u, double
 
 int ib_op_vort2flux(ib_handle* h, double* gamma, double* psi, double* q) {
   OP_BEGIN();
+  OpWork work(h);
   double* rings;
-  CK(cudaMalloc(&rings, sizeof(double) * g.nlev * g.nbc));
+  CK(work.get(&rings, (int64_t)g.nlev * g.nbc));
   cudaError_t e = vort2flux<double>(h, gamma, psi, q, nullptr, rings);
-  cudaStreamSynchronize(s);
-  cudaFree(rings);
+  work.done();
   CK(e);
   OP_END();
 }
