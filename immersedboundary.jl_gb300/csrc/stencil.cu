@@ -119,43 +119,65 @@ __global__ void k_coarsify(Geometry g, T* __restrict__ gc, const T* __restrict__
   }
 }
 
-// Multilevel curl! (fluid-ops.jl:138-182); bc == nullptr means a zero ring.  One block row per
-// flux row: blockIdx.y runs over the batch's rows (ny rows of qx, then ny + 1 rows of qy), so
-// an element's indices need no division.
+// Multilevel curl! (fluid-ops.jl:138-182); bc == nullptr means a zero ring.  A thread takes kCurlRows
+// rows of one column of nodes and the column to its right: its own column's values make the qx of the
+// column and, against the right one (which its neighbour loads too), the qy.  The thread of the last
+// column also has qx of the boundary to its right, the last strip the top row of qy.
+//
+// Bound by memory (24 bytes a node), in FP64 also by its two operations a node.  Measured against one
+// thread per flux value: 1024^2 x 4 levels, FP64 45 -> 24 us, float-float 46 -> 16.5; 2048^2 x 5 199 -> 77.
+// (2 rows a thread: 23, 21, 88; 8: 25, 17, 76 and more on small grids.)
+constexpr int kCurlX = 128, kCurlRows = 4;
 template <typename T>
-__global__ void k_curl(Geometry g, const T* __restrict__ psi, const T* __restrict__ bc, T* __restrict__ q, int batch) {
+__global__ void __launch_bounds__(kCurlX)
+k_curl(Geometry g, const T* __restrict__ psi, const T* __restrict__ bc, T* __restrict__ q) {
   pdl_begin();
   const int nx = g.nx, ny = g.ny, ncol = nx - 1;
-  const int rows = 2 * ny + 1;
-  const int b = blockIdx.y / rows, row = blockIdx.y - b * rows;
+  const int I = blockIdx.x * kCurlX + threadIdx.x, J0 = blockIdx.y * kCurlRows, b = blockIdx.z;
+  if (I >= nx) return;
   const T* p = psi + (int64_t)b * g.nG;
   const T* c = bc ? bc + (int64_t)b * g.nbc : nullptr;
-  T* qb = q + (int64_t)b * g.nq;
-#define BC(i) (c ? c[(i)] : T(0))
-  if (row < ny) {
-    const int J = row;
-    for (int I = blockIdx.x * blockDim.x + threadIdx.x; I <= nx; I += gridDim.x * blockDim.x) {
-      T v;
-      if (I == 0) v = BC(g.L + J + 1) - BC(g.L + J);
-      else if (I == nx) v = BC(g.R + J + 1) - BC(g.R + J);
-      else if (J == 0) v = p[I - 1] - BC(g.B + I);
-      else if (J == ny - 1) v = BC(g.T + I) - p[(ny - 2) * ncol + I - 1];
-      else v = p[J * ncol + I - 1] - p[(J - 1) * ncol + I - 1];
-      qb[J * (nx + 1) + I] = v;
+  T* qx = q + (int64_t)b * g.nq + (int64_t)J0 * (nx + 1) + I;
+  T* qy = q + (int64_t)b * g.nq + g.nu + (int64_t)J0 * nx + I;
+  auto ring = [&](int i) -> T { return c ? c[i] : T(0); };
+  T l[kCurlRows + 1], r[kCurlRows + 1];  // nodes (J0 + u, I), (J0 + u, I + 1)
+  if (I > 0 && I < nx - 1 && J0 > 0 && J0 + kCurlRows < ny) {
+    const T* n = p + (J0 - 1) * ncol + I - 1;
+#pragma unroll
+    for (int u = 0; u <= kCurlRows; ++u) l[u] = n[u * ncol];
+#pragma unroll
+    for (int u = 0; u < kCurlRows; ++u) r[u] = n[u * ncol + 1];
+#pragma unroll
+    for (int u = 0; u < kCurlRows; ++u) {
+      qx[u * (nx + 1)] = l[u + 1] - l[u];
+      qy[u * nx] = l[u] - r[u];
     }
-  } else {
-    const int J = row - ny;
-    for (int I = blockIdx.x * blockDim.x + threadIdx.x; I < nx; I += gridDim.x * blockDim.x) {
-      T v;
-      if (J == 0) v = BC(g.B + I) - BC(g.B + I + 1);
-      else if (J == ny) v = BC(g.T + I) - BC(g.T + I + 1);
-      else if (I == 0) v = BC(g.L + J) - p[(J - 1) * ncol];
-      else if (I == nx - 1) v = p[(J - 1) * ncol + nx - 2] - BC(g.R + J);
-      else v = p[(J - 1) * ncol + I - 1] - p[(J - 1) * ncol + I];
-      qb[g.nu + J * nx + I] = v;
+    return;
+  }
+  auto node = [&](int j, int i) -> T {
+    if (i == 0) return ring(g.L + j);
+    if (i == nx) return ring(g.R + j);
+    if (j == 0) return ring(g.B + i);
+    if (j == ny) return ring(g.T + i);
+    return p[(j - 1) * ncol + i - 1];
+  };
+#pragma unroll
+  for (int u = 0; u <= kCurlRows; ++u) {
+    l[u] = r[u] = T(0);
+    if (J0 + u <= ny) {
+      l[u] = node(J0 + u, I);
+      r[u] = node(J0 + u, I + 1);
     }
   }
-#undef BC
+#pragma unroll
+  for (int u = 0; u < kCurlRows; ++u) {
+    if (J0 + u >= ny) break;
+    qx[u * (nx + 1)] = l[u + 1] - l[u];
+    if (I == nx - 1) qx[u * (nx + 1) + 1] = r[u + 1] - r[u];
+    // (the ring's corners belong to its rows here)
+    qy[u * nx] = J0 + u == 0 ? ring(g.B + I) - ring(g.B + I + 1) : l[u] - r[u];
+  }
+  if (J0 + kCurlRows >= ny) qy[(ny - J0) * nx] = ring(g.T + I) - ring(g.T + I + 1);
 }
 
 // rot! = C^T (fluid-ops.jl:117-129)
@@ -184,18 +206,19 @@ __global__ void k_rot(Geometry g, const T* __restrict__ q, T* __restrict__ gam, 
 // One block per tile of kNTY x kNTX cells: the products its cells share are formed once into shared
 // memory, then each cell combines its four.
 //
-// FP64 is bound by its pipe (18 operations a cell; one takes 6.9 us at 1024^2 x 4 levels), float-float
-// by instruction issue.  Measured there: FP64 325 us (averages, face products and combination, 30
-// operations a cell) -> 191 us, float-float 111 -> 94 us; 200^2 x 5 in
-// FP64 21.8 -> 14.4.  (4 rows a tile: 203 and 106; 16 rows: 189 and 100.)  A warp walking up its columns
-// with the products in registers has fewer operations but waits for each row's loads: 207 and 105.
+// FP64 is bound by its pipe (19 operations a cell; one takes 7 us at 1024^2 x 4 levels; 84% busy),
+// float-float by instruction issue.  Measured there: FP64 325 us (averages, face products and combination,
+// 30 operations a cell) -> 191 us -> 157 with the ring's edge terms under one branch of the block and the
+// viscous term as two multiply-adds (predicated off, an FP64 instruction still takes its turn), float-float
+// 111 -> 94 -> 92 us.  (4 rows a tile of 64: 164 and 94; 16 rows of 32: 156 and 98.)  A warp walking up its
+// columns with the products in registers has fewer operations but waits for each row's loads.
 constexpr int kNTX = 32, kNTY = 8;
 template <typename T>
 __global__ void __launch_bounds__(kNTX * kNTY) k_nonlin_rhs(Geometry g, NonlinArgs<T> a) {
   pdl_begin();
   __shared__ T sM[kNTY + 2][kNTX];  // 2 Qy G at nodes (J0 + r, I0 + 1 + c)
   __shared__ T sN[kNTY][kNTX + 2];  // 2 Qx G at nodes (J0 + 1 + r, I0 + c)
-  __shared__ T sK[6];               // the level's 2 q0x, 2 q0y, 1/(4 hc^2), alpha; dt beta0, dt beta1
+  __shared__ T sK[7];               // the level's 2 q0x, 2 q0y, 1/(4 hc^2), alpha; dt beta0, dt beta1; 1 - 4 alpha
   const int nx = g.nx, ny = g.ny, ncol = nx - 1, nrow = ny - 1, l = blockIdx.z;
   const int J0 = blockIdx.y * kNTY, I0 = blockIdx.x * kNTX, tid = threadIdx.x;
   const T* __restrict__ qx = a.q + (int64_t)l * g.nq;
@@ -204,12 +227,13 @@ __global__ void __launch_bounds__(kNTX * kNTY) k_nonlin_rhs(Geometry g, NonlinAr
   const T* __restrict__ bc = a.bcn + (int64_t)l * g.nbc;
   // the level's constants, converted once per block (a double-to-float-float conversion costs
   // FP64 operations, which GB300 runs at 1/64 of its FP32 rate)
-  if (tid < 6) {
+  if (tid < 7) {
     sK[tid] = (T)(tid == 0 ? 2.0 * a.q0[2 * l]
                 : tid == 1 ? 2.0 * a.q0[2 * l + 1]
                 : tid == 2 ? 0.25 * a.inv_hc2[l]
                 : tid == 3 ? (a.alpha ? a.alpha[l] : 0.0)
-                : tid == 4 ? a.dtb0 : a.dtb1);
+                : tid == 4 ? a.dtb0
+                : tid == 5 ? a.dtb1 : (a.alpha ? 1.0 - 4.0 * a.alpha[l] : 1.0));
   }
   __syncthreads();
   // circulation at node (j, i) next to the interior, the ring on the boundary
@@ -241,14 +265,18 @@ __global__ void __launch_bounds__(kNTX * kNTY) k_nonlin_rhs(Geometry g, NonlinAr
     const T gc = *p;
     const T gl = I > 0 ? p[-1] : T(0), gr = I < ncol - 1 ? p[1] : T(0);
     const T gd = J > 0 ? p[-ncol] : T(0), gu = J < nrow - 1 ? p[ncol] : T(0);
-    const T lap = xscale(gc, 4.0f) - ((gl + gr) + (gd + gu));
-    r = (gc - sK[3] * lap) + r;
+    const T nb = (gl + gr) + (gd + gu);
+    if constexpr (std::is_same<T, double>::value) r = fma(sK[3], nb, fma(sK[6], gc, r));
+    else r = (gc - sK[3] * (xscale(gc, 4.0f) - nb)) + r;
   }
-  const T* ed = a.edges + (int64_t)l * (2 * ncol + 2 * nrow);
-  if (J == 0) r += ed[I];
-  if (J == nrow - 1) r += ed[ncol + I];
-  if (I == 0) r += ed[2 * ncol + J];
-  if (I == ncol - 1) r += ed[2 * ncol + nrow + J];
+  // (one branch of the whole block: four predicated additions would cost every warp their issue)
+  if (J0 == 0 || J0 + kNTY >= nrow || I0 == 0 || I0 + kNTX >= ncol) {
+    const T* ed = a.edges + (int64_t)l * (2 * ncol + 2 * nrow);
+    if (J == 0) r += ed[I];
+    if (J == nrow - 1) r += ed[ncol + I];
+    if (I == 0) r += ed[2 * ncol + J];
+    if (I == ncol - 1) r += ed[2 * ncol + nrow + J];
+  }
   a.rhs[t] = r;
 }
 
@@ -334,17 +362,13 @@ cudaError_t coarsify(const Geometry& g, T* gc, const T* gf, int batch, int64_t s
 }
 template <typename T>
 cudaError_t curl(const Geometry& g, const T* psi, const T* bc, T* q, int batch, cudaStream_t s) {
-  if (batch <= 0) return cudaSuccess;
-  const int64_t rows = (int64_t)batch * (2 * g.ny + 1);
-  if (rows > 65535) {
-    for (int b = 0; b < batch; ++b) {
-      cudaError_t e = curl<T>(g, psi + (int64_t)b * g.nG, bc ? bc + (int64_t)b * g.nbc : nullptr, q + (int64_t)b * g.nq, 1, s);
-      if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
+  for (int b = 0; b < batch; b += 65535) {
+    const dim3 grid((g.nx + kCurlX - 1) / kCurlX, (g.ny + kCurlRows - 1) / kCurlRows, std::min(batch - b, 65535));
+    const cudaError_t e = launch_k(k_curl<T>, grid, dim3(kCurlX), 0, s, g, psi + (int64_t)b * g.nG,
+                                   bc ? bc + (int64_t)b * g.nbc : nullptr, q + (int64_t)b * g.nq);
+    if (e != cudaSuccess) return e;
   }
-  const dim3 grid((g.nx + 1 + kThreads - 1) / kThreads, (unsigned)rows);
-  return launch_k(k_curl<T>, grid, dim3(kThreads), 0, s, g, psi, bc, q, batch);
+  return cudaSuccess;
 }
 template <typename T>
 cudaError_t rot(const Geometry& g, const T* q, T* gam, int batch, cudaStream_t s) {
