@@ -508,9 +508,13 @@ __device__ __forceinline__ void store_transposed(const Smem& sm, int line0, int 
   const int q = sm.q[w];
   double* dst = out + (int64_t)(b0 + wrap) * stride + (J0 + w - (wrap ? per : 0));
   if (fx::safe_scale(q)) {
+    // (NT indices on, the same parity: a constant step in the buffer)
+    const int I0 = threadIdx.x / lpb;
+    const i64* r = result_at(buf, M, I0 + 1);
+    dst += (int64_t)I0 * per;
+    const int64_t step = (int64_t)NT * per;
 #pragma unroll 8
-    for (int I = threadIdx.x / lpb; I < 2 * M - 1; I += NT)
-      dst[(int64_t)I * per] = to_double(*result_at(buf, M, I + 1), q);
+    for (int I = I0; I < 2 * M - 1; I += NT, r += Pairs<M>::kStride, dst += step) *dst = to_double(*r, q);
   } else {
 #pragma unroll 1
     for (int I = threadIdx.x / lpb; I < 2 * M - 1; I += NT)

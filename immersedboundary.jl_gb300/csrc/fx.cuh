@@ -60,7 +60,7 @@ FX_HD i64 mad(int a, int b, i64 c) { return (i64)a * b + c; }
 // arithmetic shift right by d < 31 (the same on every thread of a line), rounded to nearest even
 FX_HD i64 shr_rne(i64 v, int d) {
   if (d == 0) return v;
-  v += ((1 << (d - 1)) - 1) + (int)((v >> d) & 1);
+  v += (i64)(u64)(((1u << (d - 1)) - 1u) + (((unsigned)v >> d) & 1u));
 #if defined(__CUDA_ARCH__)
   const int hi = (int)(v >> 32);
   return (i64)((u64)(unsigned)__funnelshift_r((unsigned)v, (unsigned)hi, d) | ((u64)(unsigned)(hi >> d) << 32));
