@@ -406,46 +406,54 @@ k_fx_coef(Geometry g, const int4* __restrict__ pts, const double* __restrict__ q
   if (threadIdx.x == 0) coef[(int64_t)m * (2 * Kx + 2 * Ky) + j] = s;
 }
 
-// every ring: 32 nodes of ring l = blockIdx.y per block, kRingWarps warps sharing the coefficients (the
-// coarsest level's is zero)
-constexpr int kRingWarps = 16;
-template <typename S>
+// every ring: N nodes of ring l = blockIdx.y per block, whose lanes' 32 / N groups share the coefficients
+// with those of its kRingWarps warps (the coarsest level's ring is zero)
+//
+// Bound by the FP64 pipe, and by the finest ring's blocks, which have the longest sums: small blocks spread
+// them.  With k_fx_coef, 200^2 x 5 and 1024^2 x 4: 32 nodes and 16 warps a block 12.7, 17.4 us; 8 and 8
+// 10.3, 15.8.  At 2048^2 x 5, where every SM has blocks enough, 16 nodes (37.4) over 8 (40.3).
+constexpr int kRingWarps = 8;
+template <typename S, int N>
 __global__ void __launch_bounds__(kRingWarps * 32)
 k_fx_rings(Geometry g, const int4* __restrict__ pts, const double* __restrict__ qfx, int64_t qls,
            const double* __restrict__ Apow, const double* __restrict__ coef, int nK, S* __restrict__ rings,
            double* __restrict__ side) {
   pdl_begin();
-  __shared__ double part[kRingWarps][32];
-  const int w = threadIdx.x / 32, lane = threadIdx.x % 32, l = blockIdx.y;
-  const int idx = blockIdx.x * 32 + lane;
+  constexpr int kGroups = 32 / N, kStep = kRingWarps * kGroups;
+  __shared__ double part[kRingWarps][N];
+  const int w = threadIdx.x / 32, lane = threadIdx.x % 32, node = lane % N, l = blockIdx.y;
+  const int idx = blockIdx.x * N + node;
+  const bool out = w == 0 && lane < N && idx < g.nbc;
   if (l == g.nlev - 1) {
-    if (w == 0 && idx < g.nbc) rings[(int64_t)l * g.nbc + idx] = S(0.0);
+    if (out) rings[(int64_t)l * g.nbc + idx] = S(0.0);
     return;
   }
   double v = 0.0, h = 0.0;
+  if (out) v = ring0(pts, qfx + l * qls, idx);
   if (idx < g.nbc) {
-    if (w == 0) v = ring0(pts, qfx + l * qls, idx);
     // coefficients of the rings l+1..L-2 in a row, times A T^0, A T^1, ...
     const int n = (g.nlev - 2 - l) * nK;
     const double* a = Apow + idx;
     const double* c = coef + (int64_t)(l + 1) * nK;
     constexpr int U = 7;
-    int j = w;
-    for (; j + (U - 1) * kRingWarps < n; j += U * kRingWarps) {
+    int j = w * kGroups + lane / N;
+    for (; j + (U - 1) * kStep < n; j += U * kStep) {
       double av[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) av[u] = a[(int64_t)(j + u * kRingWarps) * g.nbc];
+      for (int u = 0; u < U; ++u) av[u] = a[(int64_t)(j + u * kStep) * g.nbc];
 #pragma unroll
-      for (int u = 0; u < U; ++u) h = fma(av[u], __ldg(&c[j + u * kRingWarps]), h);
+      for (int u = 0; u < U; ++u) h = fma(av[u], __ldg(&c[j + u * kStep]), h);
     }
-    for (; j < n; j += kRingWarps) h = fma(a[(int64_t)j * g.nbc], __ldg(&c[j]), h);
+    for (; j < n; j += kStep) h = fma(a[(int64_t)j * g.nbc], __ldg(&c[j]), h);
   }
-  part[w][lane] = h;
+#pragma unroll
+  for (int o = N; o < 32; o <<= 1) h += __shfl_xor_sync(0xffffffffu, h, o);
+  if (lane < N) part[w][lane] = h;
   __syncthreads();
-  if (w != 0 || idx >= g.nbc) return;
+  if (!out) return;
   h = 0.0;
 #pragma unroll
-  for (int k = 0; k < kRingWarps; ++k) h += part[k][lane];
+  for (int k = 0; k < kRingWarps; ++k) h += part[k][node];
   v += h;
   rings[(int64_t)l * g.nbc + idx] = S(v);
   const int ncol = g.nx - 1, nrow = g.ny - 1;
@@ -674,9 +682,10 @@ cudaError_t v2f_fx_rings(const Geometry& g, const RingPlan& rp, S* rings, cudaSt
   if (g.nlev > 2)
     CE_V(launch_k(k_fx_coef, dim3(rp.nK, g.nlev - 2), dim3(kCoefThreads), 0, s, g, (const int4*)rp.pts,
                   (const double*)rp.qfx, rp.qls, (const double*)rp.St, rp.Kx, rp.Ky, rp.coef));
-  return launch_k(k_fx_rings<S>, dim3((g.nbc + 31) / 32, g.nlev), dim3(kRingWarps * 32), 0, s, g,
-                  (const int4*)rp.pts, (const double*)rp.qfx, rp.qls, (const double*)rp.Apow, (const double*)rp.coef,
-                  rp.nK, rings, rp.side);
+  const int N = g.nbc <= 6144 ? 8 : 16;
+  return launch_k(N == 8 ? k_fx_rings<S, 8> : k_fx_rings<S, 16>, dim3((g.nbc + N - 1) / N, g.nlev),
+                  dim3(kRingWarps * 32), 0, s, g, (const int4*)rp.pts, (const double*)rp.qfx, rp.qls,
+                  (const double*)rp.Apow, (const double*)rp.coef, rp.nK, rings, rp.side);
 }
 template cudaError_t v2f_fx_rings<double>(const Geometry&, const RingPlan&, double*, cudaStream_t);
 template cudaError_t v2f_fx_rings<df64>(const Geometry&, const RingPlan&, df64*, cudaStream_t);
