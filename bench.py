@@ -635,19 +635,27 @@ def algorithmic_step_bytes(wl, precision: str) -> float:
     return 8.0 * wl.nlevels * (5 * nG + 2 * nq) + 8.0 * nf * nf
 
 
-def pass_model(wl, precision: str, levels: bool = False):
+def fixed_solves(precision: str, refine: int) -> bool:
+    """Whether the solves of an arm run in 64-bit block fixed point (else FP32 transforms with sweeps)."""
+    return precision == "fp64" or (precision == "mixed" and refine != 1 and not os.environ.get("IBGB300_DST"))
+
+
+def pass_model(wl, fixed: bool, levels: bool = False):
     """Algorithmic DRAM bytes and flops of the x and y passes of one step (per step; the bytes per
     launch follow from the launches counted while timing).
 
-    FP64 (every solve one forward and one inverse transform per axis): arrays = the trial CN
-    solve over L levels + 2L Vort2Flux solves + the projection; x forward 8 in + 8 out, x inverse
-    8 + 8 (+8 for the subtracted trial Gamma), y 8 in + 8 multiplier + 8 out, per element.
-    Mixed (default sweep policy): two-sweep solves (CN over L levels, Vort2Flux levels 1-2 twice,
+    Fixed point (8-byte values, two transforms per axis and solve): x forward 8 in + 8 out, x inverse
+    8 + 8, y 8 in + 8 multiplier + 8 out, per element, for the trial CN solve over L levels, the
+    projection (x inverse +8 for the subtracted trial Gamma) and Vort2Flux twice: level by level L
+    solves each; all levels at once (`levels`) on every level an x forward and a y pass that keeps the
+    spectrum (24), and on the finished levels (all, or level 1 for the trial call) a y pass back (24)
+    and an x inverse.
+    FP32 (default sweep policy): two-sweep solves (CN over L levels, Vort2Flux levels 1-2 twice,
     projection) move per element in x 12 (float-float in, FP32 out) + 8 + 24 (residual: b, x0,
     the stored float-float r1, out) + 8 + 16 (r1, x1, out) + 20 (x0, x1, correction, float-float
     out) and in y 3 x 12; one-sweep solves (Vort2Flux levels 3.. twice) 12 + 8 + 16 + 16 in x and
     2 x 12 in y.  A length-n sine line costs ~2.5 n log2 n flops.
-    With the all-levels Vort2Flux (`levels`): the CN and projection solves as above, and per
+    With the FP32 all-levels Vort2Flux: the CN and projection solves as above, and per
     Vort2Flux call on every level x 28 (residual from the previous psi: Gamma, psi, r1 out, FP32
     out) + 8 + 24 (residual of x0 on r1, in place) and y 12 + 12 (solve, spectrum), then on the
     finished levels (all, or level 1 for the trial call) x 8 + 16 + 28 (psi += x0 + d1 + d2, read
@@ -658,10 +666,11 @@ def pass_model(wl, precision: str, levels: bool = False):
     L = wl.nlevels
     fx = 2.5 * wl.nx * np.log2(wl.nx) * (wl.ny - 1)
     fy = 2.5 * wl.ny * np.log2(wl.ny) * (wl.nx - 1)
-    if precision == "fp64":
-        arrays = 3 * L + 1
-        return {"x": (nG * (32 * arrays + 8), fx * 2 * arrays, 2 * arrays),
-                "y": (nG * 24 * arrays, fy * 2 * arrays, arrays)}
+    if fixed:
+        solves = (L + 1) if levels else (3 * L + 1)
+        half = (2 * L + L + 1) if levels else 0   # forward halves of every level, backward ones of the finished
+        return {"x": (nG * (32 * solves + 8 + 16 * half), fx * (2 * solves + half), 2 * solves + half),
+                "y": (nG * 24 * (solves + half), fy * (2 * solves + half), solves + half)}
     if levels:
         two = L + 1                     # two-sweep CN solves: trial over L levels, projection
         fin = L + 1                     # finished Vort2Flux levels: all (projection) + level 1 (trial)
@@ -729,19 +738,23 @@ def run_ours(args, rank, world, local):
     out = {
         "metric": baseline_metric(), "value": value, "unit": "cell-steps/s", "n_gpus": world, "steps": K,
         "warmup": W, "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "weak",
-        "vs_baseline": None, "dtype": "f64" if prec == "fp64" else "f32 transforms + float-float (2xf32) residual/state",
+        "vs_baseline": None,
+        "dtype": ("f64" if prec == "fp64" else "i64 fixed-point transforms, float-float (2xf32) state"
+                  if fixed_solves(prec, args.refine_sweeps) else
+                  "f32 transforms + float-float (2xf32) residual/state"),
         "data": "synthetic: seeded PCG64 vorticity noise 1e-4 on the finest level",
         "config": bench_config(wl),
         "arm": {"precision": prec,
                 "refine_sweeps": (("2 on every solve" if info.vort2flux_order == L.IB_V2F_LEVELS else
                                    {0: "2 (1 on levels >= 3 of Vort2Flux)"}.get(args.refine_sweeps, args.refine_sweeps))
-                                  if prec == "mixed" else 0),
+                                  if prec == "mixed" and not fixed_solves(prec, args.refine_sweeps) else 0),
                 "vort2flux": ("all levels in one batch, rings first (harmonic ring transfer)"
                               if info.vort2flux_order == L.IB_V2F_LEVELS else "level by level (the reference's order)"),
                 "parallelism": "replicas",
                 "transforms": {0: "Stockham FFT passes", 1: "warp-per-line FFT passes",
                                2: "BF16x3 tensor-core sine GEMMs",
-                               3: "64-bit block fixed-point FFT passes"}.get(int(info.transform_form)),
+                               3: "64-bit block fixed-point FFT passes"}.get(
+                                   3 if fixed_solves(prec, args.refine_sweeps) else int(info.transform_form)),
                 "autotune": arm["solver"].autotune(),
                 "device_bytes": int(info.device_bytes),
                 "setup_s": info.setup_ms / 1e3, "host_wall_ms_per_step": arm["host_s"] / K * 1e3},
@@ -757,7 +770,8 @@ def run_ours(args, rank, world, local):
         return
     solver, st, prob, ts, uv, tp = arm["solver"], arm["state"], arm["prob"], arm["ts"], arm["uv"], arm["tp"]
     # dominant kernel class: event-timed launches over further steps
-    model = pass_model(wl, prec, levels=prec == "mixed" and info.vort2flux_order == L.IB_V2F_LEVELS)
+    fixed = fixed_solves(prec, args.refine_sweeps)
+    model = pass_model(wl, fixed, levels=info.vort2flux_order == L.IB_V2F_LEVELS)
     prof = {}
     npf = min(K, 20)
     base = W + K
@@ -779,7 +793,7 @@ def run_ours(args, rank, world, local):
     fp64, fp32 = C.c_double(), C.c_double()
     lib.ib_measure_fp_peaks(local, C.byref(fp64), C.byref(fp32))
     achieved = bytes_per_launch / per_launch_s / 1e9
-    form = {0: "stockham", 1: "warp", 2: "tensor", 3: "fixed"}.get(int(info.transform_form), "stockham")
+    form = {0: "stockham", 1: "warp", 2: "tensor", 3: "fixed"}.get(3 if fixed else int(info.transform_form), "stockham")
     v2f = "levels" if info.vort2flux_order == L.IB_V2F_LEVELS else "sequential"
     meas = measured_traffic(args.workload, prec, f"{form}/{v2f}", dom)
     traffic = meas[0] if meas else None
@@ -791,7 +805,8 @@ def run_ours(args, rank, world, local):
                    "stockham": {"x": "k_xpass (x-direction sine pass)",
                                 "y": "k_ypass (y-direction sine pass + spectral op)"},
                    "fixed": {"x": "k_fx_fwd/k_fx_inv (x-direction block fixed-point sine passes)",
-                             "y": "k_fx_y (y-direction block fixed-point sine passes + spectral op)"},
+                             "y": "k_fx_y/k_fx_yspec/k_fx_yring (y-direction block fixed-point sine passes + "
+                                  "spectral op)"},
                    "tensor": {"x": "k_gpro + k_sgemm (x-direction BF16x3 sine GEMMs)",
                               "y": "k_sgemm (y-direction BF16x3 sine GEMMs)"}}[form][dom],
         "bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
@@ -901,7 +916,7 @@ def main():
     ap.add_argument("--no-configs", action="store_true",
                     help="skip the per-configuration summaries (2048^2 four cylinders, moving plate)")
     ap.add_argument("--precision", default="mixed", choices=["mixed", "fp64", "mixed_tc"],
-                    help="arithmetic of the timed arm (mixed: FP32 transforms + FP64 residual refinement)")
+                    help="arithmetic of the timed arm (mixed: float-float state, fixed-point solves)")
     ap.add_argument("--no-fp64-arm", action="store_true", help="skip timing the FP64 GPU path beside it")
     ap.add_argument("--refine-sweeps", type=int, default=0,
                     help="mixed precision: residual sweeps per solve (0: default policy, 1 or 2 everywhere)")

@@ -1,5 +1,5 @@
-// The FP64 sine-transform passes: tables and entry points (kernels in dstfx.cuh, compiled by length in
-// dstfx_1.cu ... dstfx_8.cu).
+// The fixed-point sine-transform passes (FP64 and float-float lines): tables and entry points (kernels in
+// dstfx.cuh, compiled by length in dstfx_1.cu ... dstfx_8.cu).
 #include "dstfx.cuh"
 
 #include <cmath>

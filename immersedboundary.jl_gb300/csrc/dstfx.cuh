@@ -1,4 +1,5 @@
-// The kernels of the FP64 sine-transform passes (launched by dstfx.cu): every line is transformed in 64-bit block fixed point (fx.cuh).
+// The kernels of the FP64 and float-float sine-transform passes (launched by dstfx.cu): every line is
+// transformed in 64-bit block fixed point (fx.cuh).
 //
 // Replaces, like dst.cu, the FFTW RODFT00 plan + `LaplacianInv` call of the reference
 // (src/streamfcn/fluid-ops.jl:19-56) and the CN multipliers of `A_Ainv_linearmaps`
@@ -12,7 +13,7 @@
 //      registers, write in place; the bits the results occupy (one OR per value) give the next
 //      stage's shift.  Complex values are padded one slot in eight
 //   3. split into even outputs and differences D_k; the odd outputs are D's exact prefix sums
-//   4. doubles leave by their bits (leading-zero count, round, pack)
+//   4. doubles (or float-float pairs) leave by their bits (leading-zero count, round, pack)
 // A line with an infinity or NaN becomes NaN throughout, as the FP64 transform made it.  Sums of
 // integers do not depend on their order, so results are the same bits for any NT.
 //
@@ -20,13 +21,13 @@
 // pass), so that the next pass's lines lie in memory: 32 or 64 bytes at a time, written without
 // waiting, where a transposing load would stall the block.
 //
-// What bounds it: the integer pipes and the latency between them (ncu, 1024-cell lines: ALU 59% and
-// FMA-heavy 46% busy, 2.5 of 4 instructions issued per clock), and the latency of a line's chain where
+// What bounds it: the integer pipes (ncu, 1024-cell lines: ALU 57% and FMA-heavy 45% busy, an instruction
+// issued in 58% of cycles, waits mostly for a busy pipe), and the latency of a line's chain where
 // a launch has few lines.  Measured against the FP64-arithmetic passes (shared-memory Stockham, one
-// warp per line at 2048 cells), which the FP64 pipe's two lanes per SM bound: a 2048^2 Poisson solve
-// of two fields 2.09 -> 0.53 ms, a 1024^2 x 4-level two-body step 3.75 -> 1.16 ms, 384 x 256 x 4 RKC
-// 0.88 -> 0.40, 200^2 x 5 0.81 -> 0.39, 128^2 x 3 0.53 -> 0.28, with a quarter of their error on the
-// 2048^2 solve (4.3e-15 against 1.8e-14).
+// warp per line at 2048 cells), which the FP64 pipe's two lanes per SM bound: a 2048^2 Poisson call
+// on two fields 2.09 -> 0.53 ms with a quarter of the error (4.3e-15 against 1.8e-14); steps by these
+// passes alone: 1024^2 x 4 3.75 -> 1.16 ms, 384 x 256 x 4 RKC 0.88 -> 0.40, 200^2 x 5 0.81 -> 0.39, 128^2 x
+// 3 0.53 -> 0.28.
 #pragma once
 
 #include "fx.cuh"

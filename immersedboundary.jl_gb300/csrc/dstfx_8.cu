@@ -1,4 +1,4 @@
-// The FP64 passes of every eighth length (kernels in dstfx.cuh).
+// The fixed-point passes of every eighth length (kernels in dstfx.cuh).
 #include "dstfx.cuh"
 
 namespace ib::fxp {

@@ -1,4 +1,4 @@
-// Block fixed-point arithmetic of the FP64 sine transforms (dstfx.cu).
+// Block fixed-point arithmetic of the sine transforms (dstfx.cu).
 //
 // GB300 issues an FP64 instruction for 2 lanes per SM and clock; a 64-bit integer add runs at 54
 // and a 32 x 32 + 64 multiply-add (IMAD.WIDE) at 63 (measured, independent chains on a full GPU),

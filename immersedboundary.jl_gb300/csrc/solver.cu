@@ -3,11 +3,11 @@
 //
 // Step sequence (reference: src/streamfcn/cnab/timestepping.jl:253-290), FP64:
 //   d  trial state   trial_rings -> nonlin_rhs (all levels) -> X(Gamma), X(rhs) -> Y(CN) -> X
-//                    -> trial Vort2Flux (coarse-to-fine chain, curl on level 1 only)
+//                    -> trial Vort2Flux (curl on level 1 only)
 //   e  forces        E(qs1 + q0) -> Binv gemv
 //   f  stress        C_D, C_L per body -> device history
 //   g  projection    rot(E^T Fb) -> Ainv_1 -> Gamma_1 = Gamma_s1 - (.)   (buffers swap)
-//   h  Vort2Flux     coarsify + chain of Poisson solves + curl on every level
+//   h  Vort2Flux     coarsify + Poisson solves (all levels at once, or coarse to fine) + curl
 // The explicit CN operator A_l, which the reference applies with two sine transforms, is the
 // 5-point stencil it diagonalises (I - alpha_l rot curl); it is fused into the nonlinear-term
 // kernel, so each level's trial solve is one Poisson-type solve (equal up to round-off).
