@@ -2380,7 +2380,8 @@ int ib_set_vort2flux_order(ib_handle* h, int32_t order) {
   if (lv == h->v2f_levels && fx == h->v2f_fx) return IB_OK;
   CK(cudaStreamSynchronize(h->stream));
   if (lv) {
-    cudaError_t e = h->rplan.St ? cudaSuccess : h->rplan.build(h->g, h->mLap);
+    cudaError_t e = cudaSuccess;
+    if (!h->rplan.St && (e = h->rplan.build(h->g, h->mLap)) != cudaSuccess) h->rplan.release();
     if (e == cudaSuccess && fx) e = h->rplan.build_fx(h->g, h->stream);
     if (e != cudaSuccess) return fail(h, IB_ERR_CUDA, "ring transfer tables", e);
   }

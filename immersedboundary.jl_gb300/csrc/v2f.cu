@@ -690,38 +690,49 @@ cudaError_t v2f_fx_rings(const Geometry& g, const RingPlan& rp, S* rings, cudaSt
 template cudaError_t v2f_fx_rings<double>(const Geometry&, const RingPlan&, double*, cudaStream_t);
 template cudaError_t v2f_fx_rings<df64>(const Geometry&, const RingPlan&, df64*, cudaStream_t);
 
+// Everything is ordered by s, which does not wait for the legacy stream; a failed call leaves nothing
+// behind, so that the next one starts again.
 cudaError_t RingPlan::build_fx(const Geometry& g, cudaStream_t s) {
   if (Apow) return cudaSuccess;
   const int L = g.nlev;
-  auto zero = [&](double*& dst, int64_t n) -> cudaError_t {
-    CE_V(cudaMalloc(&dst, sizeof(double) * n));
-    return cudaMemset(dst, 0, sizeof(double) * n);
-  };
-  auto sines = [&](double*& dst, int n) -> cudaError_t {
-    std::vector<double> sn(n - 1);
-    for (int i = 1; i < n; ++i) sn[i - 1] = sin_pi(i, n);
-    CE_V(cudaMalloc(&dst, sizeof(double) * (n - 1)));
-    return cudaMemcpy(dst, sn.data(), sizeof(double) * (n - 1), cudaMemcpyHostToDevice);
-  };
   const int64_t one = (int64_t)nK * g.nbc;
-  CE_V(zero(qfx, (L - 1) * qls));
-  CE_V(zero(side, (L - 1) * qls));
-  CE_V(sines(sinx, g.nx));
-  CE_V(sines(siny, g.ny));
-  CE_V(zero(Apow, std::max(L - 2, 1) * one));
-  if (L < 3) return cudaSuccess;
-  CE_V(cudaMemcpyAsync(Apow, Aring, sizeof(double) * one, cudaMemcpyDeviceToDevice, s));
   double* T = nullptr;
-  CE_V(cudaMalloc(&T, sizeof(double) * nK * nK));
-  k_coef_map<<<dim3(nK, nK), kCoefThreads, 0, s>>>(g, Aring, St, Kx, Ky, T);
-  for (int d = 1; d < L - 2; ++d)
-    k_coef_next<<<dim3((g.nbc + 127) / 128, nK), 128, 0, s>>>(g.nbc, nK, T, Apow + (d - 1) * one, Apow + d * one);
-  const cudaError_t e = cudaGetLastError(), e2 = cudaStreamSynchronize(s);
-  cudaFree(T);
-  return e != cudaSuccess ? e : e2;
+  const cudaError_t e = [&]() -> cudaError_t {
+    auto zero = [&](double*& dst, int64_t n) -> cudaError_t {
+      CE_V(cudaMalloc(&dst, sizeof(double) * n));
+      return cudaMemsetAsync(dst, 0, sizeof(double) * n, s);
+    };
+    auto sines = [&](double*& dst, int n) -> cudaError_t {
+      std::vector<double> sn(n - 1);
+      for (int i = 1; i < n; ++i) sn[i - 1] = sin_pi(i, n);
+      CE_V(cudaMalloc(&dst, sizeof(double) * (n - 1)));
+      return cudaMemcpy(dst, sn.data(), sizeof(double) * (n - 1), cudaMemcpyHostToDevice);
+    };
+    CE_V(zero(qfx, (L - 1) * qls));
+    CE_V(zero(side, (L - 1) * qls));
+    CE_V(sines(sinx, g.nx));
+    CE_V(sines(siny, g.ny));
+    CE_V(zero(Apow, std::max(L - 2, 1) * one));
+    if (L < 3) return cudaStreamSynchronize(s);
+    CE_V(cudaMemcpyAsync(Apow, Aring, sizeof(double) * one, cudaMemcpyDeviceToDevice, s));
+    CE_V(cudaMalloc(&T, sizeof(double) * nK * nK));
+    k_coef_map<<<dim3(nK, nK), kCoefThreads, 0, s>>>(g, Aring, St, Kx, Ky, T);
+    for (int d = 1; d < L - 2; ++d)
+      k_coef_next<<<dim3((g.nbc + 127) / 128, nK), 128, 0, s>>>(g.nbc, nK, T, Apow + (d - 1) * one, Apow + d * one);
+    CE_V(cudaGetLastError());
+    return cudaStreamSynchronize(s);
+  }();
+  if (e != cudaSuccess) cudaStreamSynchronize(s);
+  if (T) cudaFree(T);
+  if (e != cudaSuccess) {
+    for (double** p : {&qfx, &side, &sinx, &siny, &Apow}) {
+      if (*p) cudaFree(*p);
+      *p = nullptr;
+    }
+  }
+  return e;
 }
 
-// Host tables: truncation, St, Aring and the quarter-line nodes of each ring entry.
 cudaError_t RingPlan::build(const Geometry& g, const double* mult) {
   const int nx = g.nx, ny = g.ny, ncol = nx - 1, nrow = ny - 1, L = g.nlev;
   const int nx4 = nx / 4, ny4 = ny / 4;
