@@ -542,6 +542,7 @@ __global__ void k_decay(int m, const double* __restrict__ mult, int64_t mode_str
 cudaError_t decay_table(int m, int K, const double* mult, int64_t mode_stride, int64_t sum_stride,
                         std::vector<double>& out) {
   out.assign((size_t)K * (m - 1), 0.0);
+  if (K == 0) return cudaSuccess;  // no mode of this side reaches the quarter lines
   std::vector<double> sn(2 * m);
   for (int i = 0; i < 2 * m; ++i) sn[i] = sin_pi(i, m);
   double* d = nullptr;  // sines, table

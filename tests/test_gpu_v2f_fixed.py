@@ -35,9 +35,10 @@ def _solve(ib, lib, dev, nx, ny, L, precision, order):
 
 
 # the smallest axis, axes with modes cut off and with all kept, both orders of a rectangle's axes, lines of
-# one and several warps, one to three rings above a ring
+# one and several warps, one to three rings above a ring; so long and narrow that no mode of one axis is kept
 @pytest.mark.parametrize("nx,ny,L", [(8, 8, 2), (8, 12, 4), (12, 8, 3), (36, 60, 5), (64, 48, 3), (200, 192, 5), (96, 300, 4),
-                                     (300, 96, 4), (256, 256, 2), (600, 400, 3), (1024, 128, 4), (512, 1200, 3)])
+                                     (300, 96, 4), (256, 256, 2), (600, 400, 3), (1024, 128, 4), (512, 1200, 3),
+                                     (8, 768, 4), (1200, 12, 4)])
 def test_all_levels_equal_level_by_level(ib, lib, dev, nx, ny, L):
     want = _solve(ib, lib, dev, nx, ny, L, "fp64", "sequential")
     # four line passes a level, each rounding at 2^-53 of its line's largest value, amplified by at most
