@@ -584,7 +584,7 @@ class Solver:
         """``"levels"`` (every level's boundary ring first, then all levels in one batch),
         ``"sequential"`` (the reference's coarse-to-fine order; in mixed precision with refined FP32
         transforms) or ``"auto"`` (levels from four levels on, and with three up to 2^17 cells per
-        level)."""
+        level, but for long, narrow grids)."""
         m = {"auto": _lib.IB_V2F_AUTO, "levels": _lib.IB_V2F_LEVELS, "sequential": _lib.IB_V2F_SEQUENTIAL}[order]
         self._check(self.lib.ib_set_vort2flux_order(self.handle, m))
 

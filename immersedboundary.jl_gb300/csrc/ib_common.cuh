@@ -423,6 +423,8 @@ cudaError_t v2f_ring_eval(const Geometry& g, const RingPlan& rp, int l, const df
                           df64* ring_l, cudaStream_t s);
 cudaError_t v2f_ring_coef(const Geometry& g, const RingPlan& rp, int l, cudaStream_t s);
 // the same on doubles: column sums of the spectrum of levels 1..; every ring from the quarter lines
+// multiply-adds of k_fx_rings (without building a plan)
+int64_t v2f_ring_work(const Geometry& g);
 cudaError_t v2f_fx_colsum(const Geometry& g, const RingPlan& rp, const double* w, cudaStream_t s);
 template <typename S>
 cudaError_t v2f_fx_rings(const Geometry& g, const RingPlan& rp, S* rings, cudaStream_t s);

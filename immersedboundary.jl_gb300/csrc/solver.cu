@@ -2037,7 +2037,14 @@ int ib_create(const ib_problem* p, ib_handle** out) {
       // by measurement (steps, all levels at once / level by level, us): 128^2 x 2 125 / 125, x 3 148 /
       // 162; 256^2 x 3 196 / 209, x 4 205 / 258; 384 x 256 x 3 224 / 235; 512^2 x 3 344 / 332, x 4 404 /
       // 422; 1024^2 x 3 837 / 819, x 4 997 / 1032; 2048^2 x 5 4442 / 4633
-      h->v2f_auto = L >= 4 || (L == 3 && (int64_t)g.nx * g.ny <= (int64_t(1) << 17));
+      // Long, narrow grids keep all modes of their long sides, and the rings' sums outweigh the passes saved
+      // (Vort2Flux calls, all levels / level by level, us, and sums in 2^20: 256 x 32 x 4 99 / 122, 0.9; 512 x
+      // 64 x 4 127 / 137, 3.4; 1024 x 128 x 4 169 / 170, 7.0; 1024 x 64 x 4 204 / 168, 12.8; 2048 x 256 x 4
+      // 291 / 221, 12.0; 1200 x 12 x 4 227 / 160, 16.7).  Large square ones have as many, beside longer passes
+      // (2048^2 x 5: 9.6)
+      const int64_t cells = (int64_t)g.nx * g.ny;
+      h->v2f_auto = (L >= 4 || (L == 3 && cells <= (int64_t(1) << 17))) &&
+                    v2f_ring_work(g) <= std::max<int64_t>(int64_t(1) << 22, 4 * cells);
       if (!mixed)
         if (const char* env = std::getenv("IBGB300_V2F")) {
           if (std::strcmp(env, "sequential") == 0) h->v2f_auto = false;

@@ -734,6 +734,11 @@ cudaError_t RingPlan::build_fx(const Geometry& g, cudaStream_t s) {
   return e;
 }
 
+int64_t v2f_ring_work(const Geometry& g) {
+  const int64_t nK = 2 * (modes_kept(g.nx, g.ny / 4) + modes_kept(g.ny, g.nx / 4)), L = g.nlev;
+  return nK * g.nbc * (L - 1) * (L - 2) / 2;
+}
+
 cudaError_t RingPlan::build(const Geometry& g, const double* mult) {
   const int nx = g.nx, ny = g.ny, ncol = nx - 1, nrow = ny - 1, L = g.nlev;
   const int nx4 = nx / 4, ny4 = ny / 4;

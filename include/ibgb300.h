@@ -181,7 +181,8 @@ int ib_set_cg_preconditioner(ib_handle* h, int32_t mode, int32_t refresh_steps);
  * boundary ring from the coarser solution).  IB_V2F_LEVELS finds every level's ring first
  * (harmonic ring transfer) and solves all levels in one batch; IB_V2F_SEQUENTIAL keeps the
  * reference's level order; IB_V2F_AUTO (the default) takes LEVELS from four levels on, and with
- * three up to 2^17 cells per level (solves by FP32 transforms: as the autotuner measured).  The
+ * three up to 2^17 cells per level, but for long, narrow grids (solves by FP32 transforms: as the
+ * autotuner measured).  The
  * orders agree to rounding.  The handle's step graphs are captured again; a handle in an ensemble
  * must not change it (the ensemble holds its own capture).  A mixed-precision handle set to
  * SEQUENTIAL runs Vort2Flux with the refined FP32 transforms.  IB_ERR_UNSUPPORTED for LEVELS on a

@@ -1,5 +1,8 @@
 """Vort2Flux of all levels at once in fixed point (csrc/solver.cu, csrc/v2f.cu) against the reference's
 coarse-to-fine order, FP64 and float-float state."""
+import ctypes
+import importlib
+
 import numpy as np
 import pytest
 
@@ -51,3 +54,17 @@ def test_all_levels_equal_level_by_level(ib, lib, dev, nx, ny, L):
             top = np.abs(want[0][l]).max()
             assert np.abs(got[0][l] - want[0][l]).max() < t * top, l
             assert np.abs(got[1][l] - want[1][l]).max() < 2 * t * top, l  # a flux is a difference of two psi
+
+
+# the rule that chooses the order: levels, and the size of the ring transfer on long, narrow grids
+@pytest.mark.parametrize("nx,ny,L,order", [(128, 128, 2, 2), (128, 128, 3, 1), (512, 512, 3, 2), (512, 512, 4, 1), (512, 64, 4, 1),
+                                           (1024, 64, 4, 2), (64, 1024, 4, 2), (8, 768, 4, 2)])
+def test_order_by_size(ib, lib, nx, ny, L, order):
+    h = 4.0 / nx
+    grid = ib.UniformGrid(h, (-2.0, -2.0 + nx * h), (-0.5 * ny * h, 0.5 * ny * h))
+    prob = ib.Problem(ib.StreamFcnFluid(ib.MultiLevel(grid, L), (1.0, 0.0), 100.0), ib.BodyGroup(), ib.SchemeCNAB(0.01))
+    s = ib.initsolver(prob, ib.initstate(prob))
+    info = importlib.import_module("ibgb300._lib").IbInfo()
+    assert lib.ib_get_info(s.handle, ctypes.byref(info)) == 0
+    assert info.vort2flux_order == order  # IB_V2F_LEVELS 1, IB_V2F_SEQUENTIAL 2
+    s.close()
