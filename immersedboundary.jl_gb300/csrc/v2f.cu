@@ -539,22 +539,33 @@ __global__ void k_decay(int m, const double* __restrict__ mult, int64_t mode_str
   out[(int64_t)k * (m - 1) + J] = 0.25 * s;
 }
 
-cudaError_t decay_table(int m, int K, const double* mult, int64_t mode_stride, int64_t sum_stride,
-                        std::vector<double>& out) {
-  out.assign((size_t)K * (m - 1), 0.0);
-  if (K == 0) return cudaSuccess;  // no mode of this side reaches the quarter lines
-  std::vector<double> sn(2 * m);
-  for (int i = 0; i < 2 * m; ++i) sn[i] = sin_pi(i, m);
-  double* d = nullptr;  // sines, table
-  cudaError_t e = cudaMalloc(&d, sizeof(double) * (sn.size() + out.size()));
-  if (e != cudaSuccess) return e;
-  e = cudaMemcpy(d, sn.data(), sizeof(double) * sn.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) {
-    k_decay<<<dim3((m - 1 + 63) / 64, K), 64>>>(m, mult, mode_stride, sum_stride, d, d + sn.size());
-    e = cudaMemcpy(out.data(), d + sn.size(), sizeof(double) * out.size(), cudaMemcpyDeviceToHost);
-  }
-  cudaFree(d);
-  return e;
+// St of one axis of n cells: 2 sin(pi (k+1) (i+1) / n), i < n - 1; sn: sin(pi i / n), i < 2 n
+__global__ void k_modes(int n, const double* __restrict__ sn, double* __restrict__ St) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
+  if (i < n - 1) St[(int64_t)k * (n - 1) + i] = 2.0 * sn[(int)((int64_t)(k + 1) * (i + 1) % (2 * n))];
+}
+
+// AringT[j][idx]: harmonic response of ring entry idx (one or two nodes of the level above) to
+// coefficient j; gx [k][J]: bottom-side mode k at row J, hy [k][I]: left-side mode k at column I.
+// On the host these nbc nK sums were most of the tables' time.
+__global__ void k_ring_response(Geometry g, const int4* __restrict__ pts, const double* __restrict__ St, int Kx, int Ky,
+                                const double* __restrict__ gx, const double* __restrict__ hy,
+                                double* __restrict__ AringT) {
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
+  if (idx >= g.nbc) return;
+  const int ncol = g.nx - 1, nrow = g.ny - 1;
+  const int4 p = pts[idx];
+  auto node = [&](int at, double wt) {
+    const int J = at / ncol, I = at - J * ncol;
+    if (j < 2 * Kx) {
+      const int k = j < Kx ? j : j - Kx;
+      return wt * St[(int64_t)k * ncol + I] * gx[(int64_t)k * nrow + (j < Kx ? J : nrow - 1 - J)];
+    }
+    const int k = j - 2 * Kx < Ky ? j - 2 * Kx : j - 2 * Kx - Ky;
+    return wt * St[(int64_t)Kx * ncol + (int64_t)k * nrow + J] *
+           hy[(int64_t)k * ncol + (j - 2 * Kx < Ky ? I : ncol - 1 - I)];
+  };
+  AringT[(int64_t)j * g.nbc + idx] = p.z < 0 ? node(p.x, 0.25) : node(p.x, 0.125) + node(p.z, 0.125);
 }
 
 // modes kept for a side along an axis of n cells whose nearest quarter-line node is d cells
@@ -747,29 +758,6 @@ cudaError_t RingPlan::build(const Geometry& g, const double* mult) {
   nK = 2 * Kx + 2 * Ky;
   qls = 2 * (int64_t)ncol + 2 * (int64_t)nrow;
   nchunk = (ncol + kColChunk - 1) / kColChunk;
-  std::vector<double> st((size_t)Kx * ncol + (size_t)Ky * nrow);
-  for (int k = 0; k < Kx; ++k)
-    for (int i = 0; i < ncol; ++i) st[(size_t)k * ncol + i] = 2.0 * sin_pi((int64_t)(k + 1) * (i + 1), nx);
-  for (int k = 0; k < Ky; ++k)
-    for (int j = 0; j < nrow; ++j)
-      st[(size_t)Kx * ncol + (size_t)k * nrow + j] = 2.0 * sin_pi((int64_t)(k + 1) * (j + 1), ny);
-  std::vector<double> gx, hy;
-  CE_V(decay_table(ny, Kx, mult, nrow, 1, gx));  // [k][J]: bottom-side mode k at row J
-  CE_V(decay_table(nx, Ky, mult, 1, nrow, hy));  // [l][I]: left-side mode l at column I
-  auto stx = [&](int k, int I) { return st[(size_t)k * ncol + I]; };
-  auto sty = [&](int k, int J) { return st[(size_t)Kx * ncol + (size_t)k * nrow + J]; };
-  // harmonic response at node (J, I) per coefficient, accumulated with weight wt
-  auto add_node = [&](double* a, int J, int I, double wt) {
-    for (int k = 0; k < Kx; ++k) {
-      a[k] += wt * stx(k, I) * gx[(size_t)k * nrow + J];
-      a[Kx + k] += wt * stx(k, I) * gx[(size_t)k * nrow + (ny - 2 - J)];
-    }
-    for (int k = 0; k < Ky; ++k) {
-      a[2 * Kx + k] += wt * sty(k, J) * hy[(size_t)k * ncol + I];
-      a[2 * Kx + Ky + k] += wt * sty(k, J) * hy[(size_t)k * ncol + (nx - 2 - I)];
-    }
-  };
-  std::vector<double> A((size_t)g.nbc * nK, 0.0);
   std::vector<int4> P(g.nbc);
   for (int idx = 0; idx < g.nbc; ++idx) {
     // the nodes get_bc! reads (fluid-ops.jl:210-239): column nx/4-1 or 3nx/4-1 (left / right
@@ -796,15 +784,7 @@ cudaError_t RingPlan::build(const Geometry& g, const double* mult) {
       q1 = qb + I1;
       if (ib & 1) { J2 = J; I2 = nx4 - 2 + t; q2 = qb + I2; }
     }
-    double* a = A.data() + (size_t)idx * nK;
-    if (J2 < 0) {
-      add_node(a, J1, I1, 0.25);
-      P[idx] = make_int4(J1 * ncol + I1, q1, -1, -1);
-    } else {
-      add_node(a, J1, I1, 0.125);
-      add_node(a, J2, I2, 0.125);
-      P[idx] = make_int4(J1 * ncol + I1, q1, J2 * ncol + I2, q2);
-    }
+    P[idx] = J2 < 0 ? make_int4(J1 * ncol + I1, q1, -1, -1) : make_int4(J1 * ncol + I1, q1, J2 * ncol + I2, q2);
   }
   auto up = [&](auto*& dst, const auto& src) -> cudaError_t {
     const size_t bytes = src.size() * sizeof(src[0]);
@@ -813,12 +793,37 @@ cudaError_t RingPlan::build(const Geometry& g, const double* mult) {
     return e;
   };
   cudaError_t e;
-  if ((e = up(St, st)) != cudaSuccess) return e;
-  std::vector<double> AT((size_t)nK * g.nbc);  // [nK][nbc]: the evaluation kernel reads it by node
-  for (int idx = 0; idx < g.nbc; ++idx)
-    for (int j = 0; j < nK; ++j) AT[(size_t)j * g.nbc + idx] = A[(size_t)idx * nK + j];
-  if ((e = up(Aring, AT)) != cudaSuccess) return e;
   if ((e = up(pts, P)) != cudaSuccess) return e;
+  if ((e = cudaMalloc(&St, sizeof(double) * ((int64_t)Kx * ncol + (int64_t)Ky * nrow))) != cudaSuccess) return e;
+  if ((e = cudaMalloc(&Aring, sizeof(double) * (int64_t)nK * g.nbc)) != cudaSuccess) return e;
+  {
+    // sines and decay tables, for the length of this block
+    std::vector<double> sn(2 * (size_t)(nx + ny));
+    for (int i = 0; i < 2 * nx; ++i) sn[i] = sin_pi(i, nx);
+    for (int i = 0; i < 2 * ny; ++i) sn[2 * nx + i] = sin_pi(i, ny);
+    double* d = nullptr;
+    const int64_t ngx = (int64_t)Kx * nrow, nhy = (int64_t)Ky * ncol;
+    if ((e = cudaMalloc(&d, sizeof(double) * ((int64_t)sn.size() + ngx + nhy))) != cudaSuccess) return e;
+    double *snx = d, *sny = d + 2 * nx, *gx = sny + 2 * ny, *hy = gx + ngx;
+    e = cudaMemcpy(d, sn.data(), sizeof(double) * sn.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+      // (on a long, narrow grid no mode of the short sides reaches the quarter lines)
+      if (Kx > 0) {
+        k_modes<<<dim3((ncol + 127) / 128, Kx), 128>>>(nx, snx, St);
+        k_decay<<<dim3((nrow + 63) / 64, Kx), 64>>>(ny, mult, nrow, 1, sny, gx);
+      }
+      if (Ky > 0) {
+        k_modes<<<dim3((nrow + 127) / 128, Ky), 128>>>(ny, sny, St + (int64_t)Kx * ncol);
+        k_decay<<<dim3((ncol + 63) / 64, Ky), 64>>>(nx, mult, 1, nrow, snx, hy);
+      }
+      k_ring_response<<<dim3((g.nbc + 127) / 128, nK), 128>>>(g, pts, St, Kx, Ky, gx, hy, Aring);
+      e = cudaGetLastError();
+    }
+    const cudaError_t es = cudaStreamSynchronize(nullptr);  // the handle's stream does not wait for this one
+    cudaFree(d);
+    if (e == cudaSuccess) e = es;
+    if (e != cudaSuccess) return e;
+  }
   auto zero = [&](auto*& dst, int64_t n) -> cudaError_t {
     cudaError_t e2 = cudaMalloc(&dst, sizeof(*dst) * n);
     if (e2 == cudaSuccess) e2 = cudaMemset(dst, 0, sizeof(*dst) * n);
@@ -833,7 +838,7 @@ cudaError_t RingPlan::build(const Geometry& g, const double* mult) {
   if ((e = zero(sidey, (int64_t)L * 2 * nrow)) != cudaSuccess) return e;
   if ((e = zero(ringd, (int64_t)L * g.nbc)) != cudaSuccess) return e;
   if ((e = zero(coef, (int64_t)L * nK)) != cudaSuccess) return e;
-  return cudaSuccess;
+  return cudaStreamSynchronize(nullptr);
 }
 
 void RingPlan::release() {
