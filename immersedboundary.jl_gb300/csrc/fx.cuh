@@ -247,7 +247,10 @@ FX_HD pair_float from_fixed_pair(i64 v, int q) {
   const int lz = clz64(m);
   m <<= (lz & 63);
   const unsigned t = (unsigned)(m >> 40) + ((unsigned)(m >> 39) & 1u);  // 24 bits, rounded
-  const int rem = (int)((i64)(m - ((u64)t << 40)) >> 8);                // what is left, in 2^8 units of m
+  // what is left, in 2^8 units of m.  At a tie it is -2^31, which has no negative in an int: one unit less
+  // becomes the same float
+  int rem = (int)((i64)(m - ((u64)t << 40)) >> 8);
+  rem = rem < -0x7fffffff ? -0x7fffffff : rem;
   const int eh = 127 + 63 - lz - q;                                     // biased exponent of the leading bit
   pair_float p;
   p.hi = sg | (eh > 254 ? 0x7f800000u : ((unsigned)(eh - 1) << 23) + t);

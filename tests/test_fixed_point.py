@@ -1,0 +1,57 @@
+"""The fixed-point arithmetic of the sine transforms (csrc/fx.cuh), compiled for the host."""
+import ctypes
+import shutil
+import subprocess
+from fractions import Fraction
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+HERE = Path(__file__).resolve().parent
+CSRC = HERE.parent / "immersedboundary.jl_gb300" / "csrc"
+
+
+@pytest.fixture(scope="module")
+def fx(tmp_path_factory):
+    cxx = shutil.which("g++") or shutil.which("c++")
+    assert cxx, "no C++ compiler"
+    out = tmp_path_factory.mktemp("fx") / "fx_lines.so"
+    subprocess.run([cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-x", "c++", "-I", str(CSRC),
+                    str(HERE / "fx_lines.cpp"), "-o", str(out)], check=True)
+    return ctypes.CDLL(str(out))
+
+
+def _ptr(a):
+    return a.ctypes.data_as(ctypes.c_void_p)
+
+
+def _integers(rng):
+    """Integers of every size up to 63 bits, and about every tie of a 24-bit rounding: halves of a unit in the
+    last place, and what is dropped after 32 bits around them."""
+    v = [int(x) >> int(s) for x, s in zip(rng.integers(1, 2 ** 63 - 1, 4000), rng.integers(0, 63, 4000))]
+    for bits in range(25, 64):
+        for _ in range(8):
+            top = int(rng.integers(2 ** 23, 2 ** 24)) << (bits - 24)
+            tie = top + (1 << (bits - 25))
+            low = max(bits - 56, 0)
+            v += [tie, tie - 1, tie + 1, tie + (1 << low), tie + (255 << low >> 8), tie - (1 << low)]
+    v = [x for x in v if 0 < x < 2 ** 63]
+    return np.array(v + [-x for x in v] + [0], dtype=np.int64)
+
+
+@pytest.mark.parametrize("q", [0, 55, 100, -60])
+def test_float_float_is_the_nearest(fx, q):
+    v = _integers(np.random.default_rng(q + 1000))
+    hi, r, e = np.empty(v.size, np.uint32), np.empty(v.size, np.int32), np.empty(v.size, np.int32)
+    fx.to_pair(v.size, _ptr(v), q, _ptr(hi), _ptr(r), _ptr(e))
+    first = hi.view(np.float32)
+    # the rest as the kernels form it: to FP32, then an exact power of two
+    rest = r.astype(np.float32)
+    for x, a, b, k in zip(v.tolist(), first.tolist(), rest.tolist(), e.tolist()):
+        want = Fraction(x) * Fraction(2) ** -q
+        got = Fraction(a) + Fraction(b) * Fraction(2) ** k
+        # the first part is nearest: what is left is half a unit of 24 bits at most
+        assert abs(want - Fraction(a)) <= abs(want) * Fraction(1, 2 ** 24), x
+        # 24 more bits of the rest, of which those below the 56th bit of the value may be cut off
+        assert abs(got - want) <= abs(want) * Fraction(1, 2 ** 47), x
