@@ -192,9 +192,10 @@ FX_HD i64 to_fixed(u64 bits, int ex) {
   const unsigned hi = mag_hi(bits);
   const int e = (int)(hi >> 20);
   const unsigned mh = (hi & 0xfffffu) | (e > 0 ? 0x100000u : 0u);
-  const u64 m = (((u64)mh << 32) | (unsigned)bits) << 11;
-  // m 2^-(64 - kInBits) is the value of the largest exponent
-  int s = 63 - kInBits + ex - (e > 0 ? e : 1);
+  const u64 m = (((u64)mh << 32) | (unsigned)bits) << 10;
+  // m 2^-(63 - kInBits) is the value of the largest exponent; m < 2^63, so that nothing is left of a value below
+  // half a unit however far it is shifted
+  int s = 62 - kInBits + ex - (e > 0 ? e : 1);
   if (s > 63) s = 63;
   const i64 r = (i64)(((m >> s) + 1) >> 1);
   const i64 sg = (i64)bits >> 63;

@@ -55,3 +55,21 @@ def test_float_float_is_the_nearest(fx, q):
         assert abs(want - Fraction(a)) <= abs(want) * Fraction(1, 2 ** 24), x
         # 24 more bits of the rest, of which those below the 56th bit of the value may be cut off
         assert abs(got - want) <= abs(want) * Fraction(1, 2 ** 47), x
+
+
+def test_doubles_become_the_nearest_integer(fx):
+    """Of a line whose largest value is 1.75: values of every size below it, at and about the halves of a unit, and
+    far below one."""
+    rng = np.random.default_rng(5)
+    ex = fx.exponent(ctypes.c_double(1.75))
+    q = 55 + 1022 - ex
+    x = [float(m) * 2.0 ** -k for m, k in zip(rng.uniform(1, 2, 4000), rng.integers(0, 120, 4000))]
+    x += [m * 2.0 ** -q for m in (0.25, 0.499, 0.5, 0.501, 0.999, 1.0, 1.499, 1.5, 2.5, 3.5)]
+    x += [np.nextafter(0.5, 0.0) * 2.0 ** -q, np.nextafter(0.25, 1.0) * 2.0 ** -q, 1.75, 1e-17, 1e-20, 1e-100, 1e-300,
+          2.0 ** -1022, 5e-324, 0.0]
+    x = np.array(x + [-v for v in x])
+    v = np.empty(x.size, np.int64)
+    fx.to_units(x.size, _ptr(x), ex, _ptr(v))
+    for a, b in zip(x.tolist(), v.tolist()):
+        u = abs(Fraction(a)) * Fraction(2) ** q
+        assert abs(b) == int(u + Fraction(1, 2)) and b * a >= 0, (a, b)  # (ties away from zero)
