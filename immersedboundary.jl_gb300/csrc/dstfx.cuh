@@ -40,9 +40,12 @@ namespace fxp {
 using fx::cpx;
 using fx::cwgt;
 using fx::i64;
+using fx::Radices;
+using fx::radices;
 using fx::u64;
 using fx::wgt;
 
+static_assert(fx::kMaxRadices == kMaxStages, "a stage per radix");
 constexpr unsigned kAll = 0xffffffffu;
 constexpr int kRedSlots = 2 + kMaxStages;  // reductions of one transform: largest, sum, one per stage
 
@@ -65,49 +68,6 @@ __host__ __device__ constexpr int line_words(int M) { return (even_off(M) + cpad
 // and six (x) 30.8, 128 and three 34.5; 1024^2 with 64 and eight 54.5, 128 and four 64.7.
 constexpr int group_threads(int M) { return M <= 128 ? 32 : M <= 512 ? 64 : 128; }
 constexpr int pairs(int M) { return (M + group_threads(M) - 1) / group_threads(M); }
-
-// Radices of the FFT of M points: eights where many values lie in a thread's registers (M >= 384), fours
-// where lines are short; a left-over 2 makes a six with a 3, or an eight.
-struct Radices {
-  int n, r[kMaxStages];
-};
-constexpr Radices radices(int M) {
-  Radices p{};
-  int twos = 0, threes = 0, fives = 0, eights = 0, fours = 0, sixes = 0;
-  const bool large = M >= 384;
-  for (; M % 2 == 0; M /= 2) ++twos;
-  for (; M % 3 == 0; M /= 3) ++threes;
-  for (; M % 5 == 0; M /= 5) ++fives;
-  const int over = large ? twos % 3 : twos % 2;  // large: twos left over by eights; else by fours
-  if (over == 1 && threes > 0) {
-    sixes = 1;
-    --twos;
-    --threes;
-  }
-  if (large) {
-    while (twos % 3 != 0 && twos >= 2) {
-      ++fours;
-      twos -= 2;
-    }
-  } else if (twos % 2 != 0 && twos >= 3) {
-    eights = 1;
-    twos -= 3;
-  }
-  if (large) {
-    eights = twos / 3;
-    twos %= 3;
-  } else {
-    fours = twos / 2;
-    twos %= 2;
-  }
-  for (int i = 0; i < eights; ++i) p.r[p.n++] = 8;
-  for (int i = 0; i < fours; ++i) p.r[p.n++] = 4;
-  for (int i = 0; i < sixes; ++i) p.r[p.n++] = 6;
-  for (int i = 0; i < twos; ++i) p.r[p.n++] = 2;
-  for (int i = 0; i < threes; ++i) p.r[p.n++] = 3;
-  for (int i = 0; i < fives; ++i) p.r[p.n++] = 5;
-  return p;
-}
 
 // barrier of a line's group of threads
 template <int NT>
@@ -309,8 +269,9 @@ __device__ __forceinline__ int line_transform(const Group<group_threads(M)>& G, 
     const int j = t + NT * i;
     if (kEven || j < M) {
       const i64 va = V::fixed(a[i], ex), vb = V::fixed(b[i], ex);
-      // upper bound of |va| + |vb| in units of 2^35
-      asum += ((unsigned)((int)(va >> 32) ^ (int)(va >> 63)) >> 3) + ((unsigned)((int)(vb >> 32) ^ (int)(vb >> 63)) >> 3) + 2u;
+      // upper bound of |va| + |vb| in units of 2^(kInBits - 20)
+      asum += ((unsigned)((int)(va >> 32) ^ (int)(va >> 63)) >> (fx::kInBits - 52)) +
+              ((unsigned)((int)(vb >> 32) ^ (int)(vb >> 63)) >> (fx::kInBits - 52)) + 2u;
       const int2 w = __ldg(reinterpret_cast<const int2*>(ax.sin2 + j));
       const i64 p = fx::mul(va + vb, {w.x, w.y}), df = va - vb;
       if (i == 0 && t == 0) {
@@ -331,7 +292,7 @@ __device__ __forceinline__ int line_transform(const Group<group_threads(M)>& G, 
   unsigned o = 0;
   stages<M, 0, 1>(G, ax, shifts, o);
   // 4. split: even outputs and differences, at four times their value
-  const int abits = 37 + 32 - __clz((int)(asum - 1u));  // 4 sum |y| <= 2^abits
+  const int abits = fx::kInBits - 18 + 32 - __clz((int)(asum - 1u));  // 4 sum |y| <= 2^abits
   const int d = max(excess(o, fx::kPostBits), abits - fx::kOutBits - shifts);
   shifts += d;
   {

@@ -7,14 +7,16 @@
 // tabulated factor 3 multiply-adds and a rounding shift.
 //
 // A line of doubles becomes integers v = round(x 2^q) with q from the line's largest magnitude,
-// max |v| < 2^55.  Adds are exact.  Products with a factor w (stored as w 2^60 = h 2^30 + l, h and
+// max |v| <= 2^57.  Adds are exact.  Products with a factor w (stored as w 2^60 = h 2^30 + l, h and
 // l 32-bit, |l| <= 2^29) are rounded to one unit.  Between the stages of the transform the line is
 // shifted down, all of it by the same count and rounded to nearest even, only as far as its
 // largest value then asks for (block floating point).  The noise of a transform is below that of
-// the FP64 transform it replaces: against 80-bit sums, over lines of 8 to 2048 cells, Gaussian,
-// smooth, alternating, single-mode, single-spike and exponentially spread data, its error is
-// 0.02 to 0.9 of the FP64 one's (mostly below 0.2, where the final rounding to a double dominates;
-// 0.9 on lines whose values spread over e^60).
+// the FP64 transform it replaces (tests/test_fixed_point.py, over lines of 8 to 2048 cells against sums in
+// extended precision): its error is 0.04 to 0.18 of the FP64 one's in the mean of a kind of data, most where
+// one value stands out of its line.  With inputs of 55 bits it was 0.06 to 0.45, and up to 4 times as large for
+// single lines of that sort, where the rounding of the folded small values, 1 / sin(pi j / n) times as large in
+// terms of the inputs, shows; with 56 up to 2.3 times.  The shifts that the two bits more ask for cost 0.5% at most
+// (2048^2 solve of two fields 533 -> 536 us, eight 1024^2 x 4 FP64 steps 8473 -> 8518 us).
 //
 // Plain C++ (host and device), so that the arithmetic can be checked without a GPU.
 #pragma once
@@ -46,14 +48,14 @@ struct alignas(16) cwgt {
 };
 
 // Bounds that keep every intermediate in range:
-//   inputs |v| < 2^55, so the folded line (4 times the largest input) stays below 2^57 (more bits
-//   would only add shifts: 56 gain 0.9 -> 0.75 of the FP64 error on a line of a few huge values);
+//   inputs |v| <= 2^57, so the folded line (4 times the largest input) stays within 2^59, which only the middle
+//   value can reach;
 //   components of a stage's inputs below 2^59: a radix-8 stage sums 8 complex values, a factor
 //   sqrt(1/2) meets sums below 2^61, where the split of a product's factor ends;
 //   components of the FFT's result below 2^60 before the real split, which sums pairs of them;
 //   the odd outputs, prefix sums bounded by the sum of the line's magnitudes, below 2^63
 //   (the differences they sum may wrap, the sums do not).
-constexpr int kInBits = 55, kStageBits = 59, kPostBits = 60, kOutBits = 63;
+constexpr int kInBits = 57, kStageBits = 59, kPostBits = 60, kOutBits = 63;
 
 FX_HD i64 mad(int a, int b, i64 c) { return (i64)a * b + c; }
 
@@ -180,6 +182,50 @@ template <> struct Dft<5> {
     v[3] = sub(r2, i2);
   }
 };
+
+// Radices of the FFT of M points: eights where many values lie in a thread's registers (M >= 384), fours
+// where lines are short; a left-over 2 makes a six with a 3, or an eight.
+constexpr int kMaxRadices = 10;
+struct Radices {
+  int n, r[kMaxRadices];
+};
+constexpr Radices radices(int M) {
+  Radices p{};
+  int twos = 0, threes = 0, fives = 0, eights = 0, fours = 0, sixes = 0;
+  const bool large = M >= 384;
+  for (; M % 2 == 0; M /= 2) ++twos;
+  for (; M % 3 == 0; M /= 3) ++threes;
+  for (; M % 5 == 0; M /= 5) ++fives;
+  const int over = large ? twos % 3 : twos % 2;  // large: twos left over by eights; else by fours
+  if (over == 1 && threes > 0) {
+    sixes = 1;
+    --twos;
+    --threes;
+  }
+  if (large) {
+    while (twos % 3 != 0 && twos >= 2) {
+      ++fours;
+      twos -= 2;
+    }
+  } else if (twos % 2 != 0 && twos >= 3) {
+    eights = 1;
+    twos -= 3;
+  }
+  if (large) {
+    eights = twos / 3;
+    twos %= 3;
+  } else {
+    fours = twos / 2;
+    twos %= 2;
+  }
+  for (int i = 0; i < eights; ++i) p.r[p.n++] = 8;
+  for (int i = 0; i < fours; ++i) p.r[p.n++] = 4;
+  for (int i = 0; i < sixes; ++i) p.r[p.n++] = 6;
+  for (int i = 0; i < twos; ++i) p.r[p.n++] = 2;
+  for (int i = 0; i < threes; ++i) p.r[p.n++] = 3;
+  for (int i = 0; i < fives; ++i) p.r[p.n++] = 5;
+  return p;
+}
 
 // ---- doubles to integers and back, on their bits -------------------------------------------------
 // high word of |x|: ordered like |x| over a line, exponent in bits 20..30

@@ -17,7 +17,7 @@ def fx(tmp_path_factory):
     cxx = shutil.which("g++") or shutil.which("c++")
     assert cxx, "no C++ compiler"
     out = tmp_path_factory.mktemp("fx") / "fx_lines.so"
-    subprocess.run([cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-x", "c++", "-I", str(CSRC),
+    subprocess.run([cxx, "-O2", "-std=c++17", "-ffp-contract=off", "-fPIC", "-shared", "-x", "c++", "-I", str(CSRC),
                     str(HERE / "fx_lines.cpp"), "-o", str(out)], check=True)
     return ctypes.CDLL(str(out))
 
@@ -62,7 +62,7 @@ def test_doubles_become_the_nearest_integer(fx):
     far below one."""
     rng = np.random.default_rng(5)
     ex = fx.exponent(ctypes.c_double(1.75))
-    q = 55 + 1022 - ex
+    q = fx.input_bits() + 1022 - ex
     x = [float(m) * 2.0 ** -k for m, k in zip(rng.uniform(1, 2, 4000), rng.integers(0, 120, 4000))]
     x += [m * 2.0 ** -q for m in (0.25, 0.499, 0.5, 0.501, 0.999, 1.0, 1.499, 1.5, 2.5, 3.5)]
     x += [np.nextafter(0.5, 0.0) * 2.0 ** -q, np.nextafter(0.25, 1.0) * 2.0 ** -q, 1.75, 1e-17, 1e-20, 1e-100, 1e-300,
@@ -73,3 +73,43 @@ def test_doubles_become_the_nearest_integer(fx):
     for a, b in zip(x.tolist(), v.tolist()):
         u = abs(Fraction(a)) * Fraction(2) ** q
         assert abs(b) == int(u + Fraction(1, 2)) and b * a >= 0, (a, b)  # (ties away from zero)
+
+
+def _kinds(n, rng):
+    j = np.arange(1, n)
+    x, g = j / n, rng.standard_normal(n - 1)
+    spike = np.zeros(n - 1)
+    spike[(n - 1) // 3] = 1.0
+    yield "normal", g
+    yield "smooth", np.exp(-(x - 0.3) ** 2 / 0.01)
+    yield "alternating", (-1.0) ** j * (1 + 0.1 * g)
+    yield "low mode", np.sin(3 * np.pi * x)
+    yield "high mode", np.sin(np.pi * (n - 2) * x)
+    yield "spike", spike
+    yield "ones", np.ones(n - 1)
+    yield "spread", g * np.exp(rng.uniform(-60, 0, n - 1))
+    yield "spread far", g * np.exp(12 * rng.standard_normal(n - 1))
+    for w in (0.3, 0.5, 1, 2, 5, 20):  # tails of one sign, as the solution beside a body or vortex has them
+        yield "tail %g" % w, np.exp(-np.abs(j - n / 4) / w)
+        yield "end %g" % w, np.exp(-j / w)
+    yield "power", 1.0 / j ** 3
+    yield "spike on 1e-17", spike + 1e-17
+    yield "spike on 1e-9", spike + 1e-9
+
+
+@pytest.mark.parametrize("n", [8, 24, 64, 100, 200, 360, 500, 1024, 1500, 2048])
+def test_line_error_is_below_an_fp64_transforms(fx, n):
+    """Errors (2-norm) of the kernels' steps on integers and of the same steps in FP64 against sums in extended
+    precision, root mean squares over lines of one kind."""
+    worse = {}
+    for seed in range(6):
+        rng = np.random.default_rng(seed)
+        for kind, y in _kinds(n, rng):
+            y = np.ascontiguousarray(y * rng.uniform(1, 2))
+            e = (ctypes.c_double * 2)()
+            fx.line_errors(n, _ptr(y), ctypes.byref(e, 0), ctypes.byref(e, 8))
+            worse.setdefault(kind, []).append((e[0] ** 2, e[1] ** 2))
+    for kind, e in worse.items():
+        a, b = np.sqrt(np.mean(e, axis=0))
+        # (a line whose sums are exact in FP64 leaves nothing to be below: half a unit of the results is)
+        assert a <= max(b, 2.0 ** -53), (kind, a, b)
