@@ -24,7 +24,7 @@ cudaError_t FxTables::build(int n) {
   auto split = [](long double w) {
     const long long v = llrintl(w * (long double)(1LL << 60));
     const int h = (int)((v + (1LL << 29)) >> 30);
-    return fx::wgt{h, (int)(v - ((long long)h << 30))};
+    return fx::wgt{h, (int)(v - h * (1LL << 30))};
   };
   auto cis = [&](long double num, long double den) {  // e^{-2 pi i num / den}
     const long double ang = -2.0L * pi * num / den;

@@ -345,16 +345,16 @@ __device__ __forceinline__ int line_transform(const Group<group_threads(M)>& G, 
     i64 s[PP], acc = 0;
 #pragma unroll
     for (int i = 0; i < PP; ++i) {
-      if (kEven || k0 + i < M) acc += G.buf[8 % PP == 0 ? cpad(k0) + i : cpad(k0 + i)];
+      if (kEven || k0 + i < M) acc = fx::add_wrap(acc, G.buf[8 % PP == 0 ? cpad(k0) + i : cpad(k0 + i)]);
       s[i] = acc;
     }
     i64 incl = acc;
 #pragma unroll
     for (int w = 1; w < 32; w <<= 1) {
       const i64 v = __shfl_up_sync(kAll, incl, w);
-      if ((t & 31) >= w) incl += v;
+      if ((t & 31) >= w) incl = fx::add_wrap(incl, v);
     }
-    i64 excl = incl - acc;
+    i64 excl = (i64)((fx::u64)incl - (fx::u64)acc);
     if (NT > 32) {
       // totals of the warps before this one (spare words after the padded differences)
       i64* tot = G.buf + M + (M >> 3) + 2;
@@ -362,11 +362,11 @@ __device__ __forceinline__ int line_transform(const Group<group_threads(M)>& G, 
       G.bar();
 #pragma unroll
       for (int w = 0; w < NT / 32 - 1; ++w)
-        if ((t >> 5) > w) excl += tot[w];
+        if ((t >> 5) > w) excl = fx::add_wrap(excl, tot[w]);
     }
 #pragma unroll
     for (int i = 0; i < PP; ++i)
-      if (kEven || k0 + i < M) G.buf[8 % PP == 0 ? cpad(k0) + i : cpad(k0 + i)] = s[i] + excl;
+      if (kEven || k0 + i < M) G.buf[8 % PP == 0 ? cpad(k0) + i : cpad(k0 + i)] = fx::add_wrap(s[i], excl);
   }
   G.bar();
   return V::kScale - ex - shifts + 2;

@@ -54,9 +54,11 @@ struct alignas(16) cwgt {
 //   sqrt(1/2) meets sums below 2^61, where the split of a product's factor ends;
 //   components of the FFT's result below 2^60 before the real split, which sums pairs of them;
 //   the odd outputs, prefix sums bounded by the sum of the line's magnitudes, below 2^63
-//   (the differences they sum may wrap, the sums do not).
+//   (sums of some of the differences may wrap, the outputs do not).
 constexpr int kInBits = 57, kStageBits = 59, kPostBits = 60, kOutBits = 63;
 
+// a + b of partial sums, which may wrap on the way to a sum that does not
+FX_HD i64 add_wrap(i64 a, i64 b) { return (i64)((u64)a + (u64)b); }
 FX_HD i64 mad(int a, int b, i64 c) { return (i64)a * b + c; }
 
 // arithmetic shift right by d < 31 (the same on every thread of a line), rounded to nearest even

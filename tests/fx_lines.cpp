@@ -47,7 +47,7 @@ struct Fixed {
   static wgt weight(long double w) {
     const long long v = llrintl(w * (long double)(1LL << 60));
     const int h = (int)((v + (1LL << 29)) >> 30);
-    return {h, (int)(v - ((long long)h << 30))};
+    return {h, (int)(v - h * (1LL << 30))};
   }
   static factor cis(long double num, long double den) {  // e^{-2 pi i num / den}
     const long double ang = -2.0L * kPi * num / den;
@@ -180,10 +180,17 @@ extern "C" void line_fixed(int n, const double* y, double* F) {
     std::memcpy(&x, &o, 8);
     return x;
   };
-  i64 s = 0;
+  // prefix sums of D: within chunks of 8, of the chunks' totals by doubling, both together
+  const int chunks = (M + 7) / 8;
+  std::vector<i64> total(chunks);
   for (int k = 0; k < M; ++k) {
-    s += D[k];
-    F[2 * k] = value(s);
+    if (k % 8) D[k] = add_wrap(D[k - 1], D[k]);
+    total[k / 8] = D[k];
+  }
+  for (int w = 1; w < chunks; w <<= 1)
+    for (int t = chunks - 1; t >= w; --t) total[t] = add_wrap(total[t], total[t - w]);
+  for (int k = 0; k < M; ++k) {
+    F[2 * k] = value(k < 8 ? D[k] : add_wrap(D[k], total[k / 8 - 1]));
     if (k) F[2 * k - 1] = value(E[k]);
   }
 }

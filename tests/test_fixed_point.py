@@ -2,6 +2,7 @@
 import ctypes
 import shutil
 import subprocess
+import sys
 from fractions import Fraction
 from pathlib import Path
 
@@ -12,14 +13,17 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE.parent / "immersedboundary.jl_gb300" / "csrc"
 
 
-@pytest.fixture(scope="module")
-def fx(tmp_path_factory):
+def _build(out, *flags):
     cxx = shutil.which("g++") or shutil.which("c++")
     assert cxx, "no C++ compiler"
-    out = tmp_path_factory.mktemp("fx") / "fx_lines.so"
     subprocess.run([cxx, "-O2", "-std=c++17", "-ffp-contract=off", "-fPIC", "-shared", "-x", "c++", "-I", str(CSRC),
-                    str(HERE / "fx_lines.cpp"), "-o", str(out)], check=True)
+                    *flags, str(HERE / "fx_lines.cpp"), "-o", str(out)], check=True)
     return ctypes.CDLL(str(out))
+
+
+@pytest.fixture(scope="module")
+def fx(tmp_path_factory):
+    return _build(tmp_path_factory.mktemp("fx") / "fx_lines.so")
 
 
 def _ptr(a):
@@ -113,3 +117,34 @@ def test_line_error_is_below_an_fp64_transforms(fx, n):
         a, b = np.sqrt(np.mean(e, axis=0))
         # (a line whose sums are exact in FP64 leaves nothing to be below: half a unit of the results is)
         assert a <= max(b, 2.0 ** -53), (kind, a, b)
+
+
+_EXTREME = """
+import ctypes, sys
+import numpy as np
+lib = ctypes.CDLL(sys.argv[1])
+ptr = lambda a: a.ctypes.data_as(ctypes.c_void_p)
+for n in (8, 12, 20, 48, 200, 360, 972, 1000, 1024, 1500, 2048):
+    j, rng = np.arange(1, n), np.random.default_rng(n)
+    k, e = np.pi * j / n, (ctypes.c_double * 2)()
+    top = np.nextafter(2.0, 0.0)  # rounds to the largest integer of a line
+    # the largest outputs, and combs whose outputs a and b are the largest of both signs
+    lines = [np.ones(n - 1), np.sign(np.sin(k)), np.sign(np.sin((n - 1) * k)), (-1.0) ** j, rng.choice([-1.0, 1.0], n - 1)]
+    lines += [(j == i) * 1.0 for i in (1, n // 4, n // 2, n - 1)] + [(j % 8 == 0) * 1.0, (j % 2 == 1) * 1.0]
+    for a, b in ((1, 3), (3, 9), (15, 47), (15, 45), (63, 189)):
+        f = np.sin(a * k) - np.sin(b * k)
+        lines += [np.where(np.abs(f) > t, np.sign(f), 0.0) for t in (0.0, 1.2, 1.8)]
+    for y in (y for y in lines if y.any()):
+        for s in (top, -top, 1.5):
+            lib.line_errors(n, ptr(np.ascontiguousarray(y * s)), ctypes.byref(e, 0), ctypes.byref(e, 8))
+            assert e[0] < 1e-14, (n, e[0])
+"""
+
+
+def test_no_signed_overflow_at_extreme_lines(tmp_path):
+    """Lines of the largest values, and of the largest outputs of both signs (whose partial sums wrap): no undefined
+    operation, and no lost high bit (errors of an FP64 transform's size)."""
+    out = tmp_path / "fx_trap.so"
+    _build(out, "-fsanitize=signed-integer-overflow,shift", "-fsanitize-undefined-trap-on-error")
+    r = subprocess.run([sys.executable, "-c", _EXTREME, str(out)], capture_output=True, text=True)
+    assert r.returncode == 0, (r.returncode, r.stderr[-400:])
