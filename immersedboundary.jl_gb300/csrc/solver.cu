@@ -2045,12 +2045,16 @@ int ib_create(const ib_problem* p, ib_handle** out) {
       const int64_t cells = (int64_t)g.nx * g.ny;
       h->v2f_auto = (L >= 4 || (L == 3 && cells <= (int64_t(1) << 17))) &&
                     v2f_ring_work(g) <= std::max<int64_t>(int64_t(1) << 22, 4 * cells);
-      if (!mixed)
-        if (const char* env = std::getenv("IBGB300_V2F")) {
-          if (std::strcmp(env, "sequential") == 0) h->v2f_auto = false;
-          if (std::strcmp(env, "levels") == 0) h->v2f_auto = L > 1;
-        }
-      if (!pin_v2f) h->v2f_levels = h->v2f_auto;
+      // a mixed handle takes the order on request where its grid has one-warp lines, whatever FP32 passes the tuner
+      // chose (else the rule's order stands)
+      if (mixed) h->v2f_ok = lv_base;
+      h->v2f_levels = h->v2f_auto;
+      if (const char* env = std::getenv("IBGB300_V2F")) {
+        // as ib_set_vort2flux_order: the reference's order of a mixed handle is that of the FP32 transforms
+        if (std::strcmp(env, "sequential") == 0) h->v2f_levels = false, h->v2f_fx = !mixed;
+        if (std::strcmp(env, "levels") == 0) h->v2f_levels = mixed ? h->v2f_ok || h->v2f_auto : L > 1;
+      }
+      if (!mixed) h->v2f_auto = h->v2f_levels;
       if (h->v2f_levels && ((!h->rplan.St && (e = h->rplan.build(g, h->mLap)) != cudaSuccess) ||
                             (e = h->rplan.build_fx(g, h->stream)) != cudaSuccess))
         return bail(fail(h, IB_ERR_CUDA, "ring transfer tables", e));

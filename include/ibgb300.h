@@ -183,10 +183,11 @@ int ib_set_cg_preconditioner(ib_handle* h, int32_t mode, int32_t refresh_steps);
  * reference's level order; IB_V2F_AUTO (the default) takes LEVELS from four levels on, and with
  * three up to 2^17 cells per level, but for long, narrow grids (solves by FP32 transforms: as the
  * autotuner measured).  The
- * orders agree to rounding.  The handle's step graphs are captured again; a handle in an ensemble
- * must not change it (the ensemble holds its own capture).  A mixed-precision handle set to
- * SEQUENTIAL runs Vort2Flux with the refined FP32 transforms.  IB_ERR_UNSUPPORTED for LEVELS on a
- * mixed-precision handle whose grid has no one-warp line passes. */
+ * orders agree to rounding (FP32 transforms: to their refinement).  The handle's step graphs are
+ * captured again; a handle in an ensemble must not change it (the ensemble holds its own capture).
+ * A mixed-precision handle set to SEQUENTIAL, here or by IBGB300_V2F, runs Vort2Flux with the refined
+ * FP32 transforms.  IB_ERR_UNSUPPORTED for LEVELS on a mixed-precision handle whose grid has no
+ * one-warp line passes. */
 #define IB_V2F_AUTO 0
 #define IB_V2F_LEVELS 1
 #define IB_V2F_SEQUENTIAL 2
