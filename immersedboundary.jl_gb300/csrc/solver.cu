@@ -1974,9 +1974,14 @@ int ib_create(const ib_problem* p, ib_handle** out) {
     h->h_q0 = nullptr;
     return bail(fail(h, IB_ERR_CUDA, "pinned staging", e));
   }
+  // The copies of the set-up go through the legacy stream, which h->stream neither waits for nor holds up: they
+  // begin when the arrays are zeroed and have landed before anything reads them.
+  auto copies_begin = [&] { return cudaStreamSynchronize(h->stream); };
+  auto copies_end = [&] { return cudaStreamSynchronize(nullptr); };
   {
     std::vector<double> lap, cn1, cn2;
     build_multipliers(h, lap, cn1, cn2);
+    if ((e = copies_begin()) != cudaSuccess) return bail(fail(h, IB_ERR_CUDA, "parameter upload", e));
     std::vector<double> fac(L), ihc(L), alpha(L);
     for (int l = 0; l < L; ++l) {
       const double hc = g.h * std::ldexp(1.0, l);
@@ -2011,6 +2016,7 @@ int ib_create(const ib_problem* p, ib_handle** out) {
           (e = cudaMemcpy(h->mCN1_32, c32.data(), sizeof(float) * c32.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
         return bail(fail(h, IB_ERR_CUDA, "parameter upload", e));
     }
+    if ((e = copies_end()) != cudaSuccess) return bail(fail(h, IB_ERR_CUDA, "parameter upload", e));
   }
   {
     const bool mixed = h->precision == IB_PREC_MIXED;
@@ -2095,6 +2101,7 @@ int ib_create(const ib_problem* p, ib_handle** out) {
       bs[b + 1] = bs[b] + p->body_npoints[b];
       for (int k = bs[b]; k < bs[b + 1]; ++k) bof[k] = b;
     }
+    if ((e = copies_begin()) != cudaSuccess) return bail(fail(h, IB_ERR_CUDA, "body upload", e));
     if ((e = cudaMemcpy(moving ? h->xb_body : h->xb, p->xb, sizeof(double) * 2 * nb, cudaMemcpyHostToDevice)) !=
             cudaSuccess ||
         (e = cudaMemcpy(h->ds, p->ds, sizeof(double) * nb, cudaMemcpyHostToDevice)) != cudaSuccess ||
@@ -2102,6 +2109,7 @@ int ib_create(const ib_problem* p, ib_handle** out) {
       return bail(fail(h, IB_ERR_CUDA, "body upload", e));
     if (moving && (e = cudaMemcpy(h->body_of, bof.data(), sizeof(int) * nb, cudaMemcpyHostToDevice)) != cudaSuccess)
       return bail(fail(h, IB_ERR_CUDA, "body upload", e));
+    if ((e = copies_end()) != cudaSuccess) return bail(fail(h, IB_ERR_CUDA, "body upload", e));
     if (!moving) {
       if ((e = reg_update(g, h->xb, nb, h->body_idx, h->weight, h->status, h->stream)) != cudaSuccess)
         return bail(fail(h, IB_ERR_CUDA, "delta weights", e));

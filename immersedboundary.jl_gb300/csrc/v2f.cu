@@ -718,7 +718,7 @@ cudaError_t RingPlan::build_fx(const Geometry& g, cudaStream_t s) {
       std::vector<double> sn(n - 1);
       for (int i = 1; i < n; ++i) sn[i - 1] = sin_pi(i, n);
       CE_V(cudaMalloc(&dst, sizeof(double) * (n - 1)));
-      return cudaMemcpy(dst, sn.data(), sizeof(double) * (n - 1), cudaMemcpyHostToDevice);
+      return cudaMemcpyAsync(dst, sn.data(), sizeof(double) * (n - 1), cudaMemcpyHostToDevice, s);  // (staged: sn may go)
     };
     CE_V(zero(qfx, (L - 1) * qls));
     CE_V(zero(side, (L - 1) * qls));
