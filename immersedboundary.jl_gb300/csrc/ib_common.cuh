@@ -408,8 +408,10 @@ struct RingPlan {
   // the harmonic part of a ring in terms of the coefficients of the ring d levels up, d = 1..L-2:
   // Aring (St-sides of Aring)^(d-1), [d-1][nK][nbc]
   double *qfx = nullptr, *side = nullptr, *sinx = nullptr, *siny = nullptr, *Apow = nullptr;
+  int64_t bytes = 0;  // device memory of all these
   cudaError_t build(const Geometry& g, const double* mult);  // mult: of the Poisson solve (device)
   cudaError_t build_fx(const Geometry& g, cudaStream_t s);  // after build()
+  template <typename T> cudaError_t get(T*& p, int64_t n);
   void release();
 };
 cudaError_t v2f_yspec(const Geometry& g, const DstAxis<float>& ax, float* w, const float* m, int batch, float* vrow,

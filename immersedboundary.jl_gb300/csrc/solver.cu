@@ -2520,7 +2520,10 @@ int ib_get_info(ib_handle* h, ib_info* info) {
   info->nlevels = h->g.nlev;
   info->nbodies = h->nbodies;
   info->npoints = h->nb;
-  info->device_bytes = h->device_bytes;
+  {
+    std::lock_guard<std::mutex> lock(h->op_mu);
+    info->device_bytes = h->device_bytes + h->rplan.bytes + (int64_t)sizeof(double) * h->op_cap;
+  }
   info->setup_ms = h->setup_ms;
   info->vort2flux_order = h->v2f_levels ? IB_V2F_LEVELS : IB_V2F_SEQUENTIAL;
   info->transform_form = h->precision == IB_PREC_FP64 ? IB_FORM_FIXED

@@ -702,22 +702,30 @@ cudaError_t v2f_fx_rings(const Geometry& g, const RingPlan& rp, S* rings, cudaSt
 template cudaError_t v2f_fx_rings<double>(const Geometry&, const RingPlan&, double*, cudaStream_t);
 template cudaError_t v2f_fx_rings<df64>(const Geometry&, const RingPlan&, df64*, cudaStream_t);
 
+template <typename T>
+cudaError_t RingPlan::get(T*& p, int64_t n) {
+  const cudaError_t e = cudaMalloc(&p, sizeof(T) * n);
+  if (e == cudaSuccess) bytes += (int64_t)sizeof(T) * n;
+  else p = nullptr;
+  return e;
+}
+
 // Everything is ordered by s, which does not wait for the legacy stream; a failed call leaves nothing
 // behind, so that the next one starts again.
 cudaError_t RingPlan::build_fx(const Geometry& g, cudaStream_t s) {
   if (Apow) return cudaSuccess;
   const int L = g.nlev;
-  const int64_t one = (int64_t)nK * g.nbc;
+  const int64_t one = (int64_t)nK * g.nbc, bytes0 = bytes;
   double* T = nullptr;
   const cudaError_t e = [&]() -> cudaError_t {
     auto zero = [&](double*& dst, int64_t n) -> cudaError_t {
-      CE_V(cudaMalloc(&dst, sizeof(double) * n));
+      CE_V(get(dst, n));
       return cudaMemsetAsync(dst, 0, sizeof(double) * n, s);
     };
     auto sines = [&](double*& dst, int n) -> cudaError_t {
       std::vector<double> sn(n - 1);
       for (int i = 1; i < n; ++i) sn[i - 1] = sin_pi(i, n);
-      CE_V(cudaMalloc(&dst, sizeof(double) * (n - 1)));
+      CE_V(get(dst, n - 1));
       return cudaMemcpyAsync(dst, sn.data(), sizeof(double) * (n - 1), cudaMemcpyHostToDevice, s);  // (staged: sn may go)
     };
     CE_V(zero(qfx, (L - 1) * qls));
@@ -741,6 +749,7 @@ cudaError_t RingPlan::build_fx(const Geometry& g, cudaStream_t s) {
       if (*p) cudaFree(*p);
       *p = nullptr;
     }
+    bytes = bytes0;
   }
   return e;
 }
@@ -787,15 +796,14 @@ cudaError_t RingPlan::build(const Geometry& g, const double* mult) {
     P[idx] = J2 < 0 ? make_int4(J1 * ncol + I1, q1, -1, -1) : make_int4(J1 * ncol + I1, q1, J2 * ncol + I2, q2);
   }
   auto up = [&](auto*& dst, const auto& src) -> cudaError_t {
-    const size_t bytes = src.size() * sizeof(src[0]);
-    cudaError_t e = cudaMalloc(&dst, bytes);
-    if (e == cudaSuccess) e = cudaMemcpy(dst, src.data(), bytes, cudaMemcpyHostToDevice);
+    cudaError_t e = get(dst, (int64_t)src.size());
+    if (e == cudaSuccess) e = cudaMemcpy(dst, src.data(), src.size() * sizeof(src[0]), cudaMemcpyHostToDevice);
     return e;
   };
   cudaError_t e;
   if ((e = up(pts, P)) != cudaSuccess) return e;
-  if ((e = cudaMalloc(&St, sizeof(double) * ((int64_t)Kx * ncol + (int64_t)Ky * nrow))) != cudaSuccess) return e;
-  if ((e = cudaMalloc(&Aring, sizeof(double) * (int64_t)nK * g.nbc)) != cudaSuccess) return e;
+  if ((e = get(St, (int64_t)Kx * ncol + (int64_t)Ky * nrow)) != cudaSuccess) return e;
+  if ((e = get(Aring, (int64_t)nK * g.nbc)) != cudaSuccess) return e;
   {
     // sines and decay tables, for the length of this block
     std::vector<double> sn(2 * (size_t)(nx + ny));
@@ -825,7 +833,7 @@ cudaError_t RingPlan::build(const Geometry& g, const double* mult) {
     if (e != cudaSuccess) return e;
   }
   auto zero = [&](auto*& dst, int64_t n) -> cudaError_t {
-    cudaError_t e2 = cudaMalloc(&dst, sizeof(*dst) * n);
+    cudaError_t e2 = get(dst, n);
     if (e2 == cudaSuccess) e2 = cudaMemset(dst, 0, sizeof(*dst) * n);
     return e2;
   };
@@ -849,6 +857,7 @@ void RingPlan::release() {
   St = nullptr; Aring = nullptr; pts = nullptr; vrow = nullptr; ucolp = nullptr; ucol = nullptr; qline = nullptr;
   sidex = nullptr; sidey = nullptr; ringd = nullptr; dring = nullptr; coef = nullptr;
   qfx = side = sinx = siny = Apow = nullptr;
+  bytes = 0;
 }
 
 }  // namespace ib
