@@ -21,11 +21,11 @@
 // pass), so that the next pass's lines lie in memory: 32 or 64 bytes at a time, written without
 // waiting, where a transposing load would stall the block.
 //
-// What bounds it: the integer pipes (ncu, 1024-cell lines: ALU 57% and FMA-heavy 45% busy, an instruction
-// issued in 58% of cycles, waits mostly for a busy pipe), and the latency of a line's chain where
+// What bounds it: the integer pipes (ncu, 1024-cell lines: ALU 60% and FMA-heavy 45% busy, an instruction
+// issued in 59% of cycles, waits mostly for a busy pipe), and the latency of a line's chain where
 // a launch has few lines.  Measured against the FP64-arithmetic passes (shared-memory Stockham, one
 // warp per line at 2048 cells), which the FP64 pipe's two lanes per SM bound: a 2048^2 Poisson call
-// on two fields 2.09 -> 0.53 ms with a quarter of the error (4.3e-15 against 1.8e-14); steps by these
+// on two fields 2.09 -> 0.54 ms with a tenth of the error (1.6e-15 against 2.2e-14); steps by these
 // passes alone: 1024^2 x 4 3.75 -> 1.16 ms, 384 x 256 x 4 RKC 0.88 -> 0.40, 200^2 x 5 0.81 -> 0.39, 128^2 x
 // 3 0.53 -> 0.28.
 #pragma once
